@@ -176,8 +176,10 @@ def _in_order(state, rows):
     k = torch.from_numpy(keys.view(np.int64)).cuda(non_blocking=True)
     c = torch.from_numpy(cov.view(np.int16)).cuda(non_blocking=True)
     m = torch.from_numpy(mask).cuda(non_blocking=True)
-    h = k[:, 0] if k.shape[1] == 1 else (k * torch.tensor([0x1E3779B97F4A7C15, 0x3F58476D1CE4E5B9, 0x14D049BB133111EB,
-                                                           0x2545F4914F6CDD1D][:k.shape[1]], device=k.device)).sum(1)
+    h = k[:, 0]
+    for j in range(1, k.shape[1]):
+        h = (h ^ (h >> 29)) * 0x1E3779B97F4A7C15 + k[:, j]
+        h = (h ^ (h >> 32)) * 0x3F58476D1CE4E5B9
     o = torch.argsort(h)
     n, cap = len(o), len(state["rows"][1])
     out = k.new_zeros((cap, k.shape[1])), c.new_zeros(cap), m.new_zeros(cap)
