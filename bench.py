@@ -317,7 +317,7 @@ def run_ours(args, rank, world, local):
         torch.cuda.synchronize()
         launches = ctx.launch_count() - launches0
         kms = {n: ctx.timing(n) for n in ("pass1", "solid", "pass2_emit", "pass2_count", "pass2_upsert", "pass2_direct",
-                                          "convert", "table_init", "est_", "clamp", "cms_clamp", "subsample", "")}
+                                          "convert", "table_init", "est_", "clamp", "cms_clamp", "subsample", "bins_", "")}
         ctx.set_timing(False)
         if world > 1:
             t = torch.tensor([ms], dtype=torch.float64, device="cuda")
@@ -339,8 +339,10 @@ def run_ours(args, rank, world, local):
         t = api.build_cdbg_ext(dbank, k, None, ge.genome_size, ctx=ctx, counter_bits=cb, cms_log2_width=LOG2W)
         t.release()
         ctx.sync()
-        per_k[str(k)] = {f: round(ctx.timing(f)[0], 3) for f in ("pass1", "pass2_emit", "pass2_count", "pass2_upsert",
-                                                                  "convert", "table_init") if ctx.timing(f)[0] > 0}
+        per_k[str(k)] = {f: round(ctx.timing(f)[0], 3) for f in ("bins_runs", "bins_scatter", "bins_sample", "bins_aggregate",
+                                                                  "bins_sketch", "bins_singles", "bins_gate", "pass1", "pass2_emit",
+                                                                  "pass2_count", "pass2_upsert", "convert", "table_init")
+                         if ctx.timing(f)[0] > 0}
     ctx.set_timing(False)
 
     # ---- the same step with the counted u16 sketch (what a caller asking for the
@@ -370,6 +372,7 @@ def run_ours(args, rank, world, local):
     key_bytes = {k: 8 * (api.key_bits_for_k(k) // 64) for k in KS}
     pushes = {r[0]: r[3] for r in res}
     fam_ms = {
+        "bins": kernel_ms["bins_"][0],  # both passes in one form (csrc/fbk_bins.cu)
         "pass1": kernel_ms["pass1"][0],
         "pass2": kernel_ms["solid"][0] + kernel_ms["pass2_emit"][0] + kernel_ms["pass2_count"][0]
                  + kernel_ms["pass2_upsert"][0] + kernel_ms["pass2_direct"][0],
@@ -378,6 +381,7 @@ def run_ours(args, rank, world, local):
         "pass1": sum(bank_bytes + kmers_pass[k][0] * 8 * c_b for k in KS),
         "pass2": sum(bank_bytes + kmers_pass[k][1] * 4 * c_b + pushes[k] * 2 * (key_bytes[k] + 2 + 16) for k in KS),
     }
+    alg["bins"] = alg["pass1"] + alg["pass2"]
     dom = max(fam_ms, key=fam_ms.get)
     per_pass_ms = fam_ms[dom] / (args.steps * len(KS))
     per_pass_bytes = alg[dom] / len(KS)
@@ -493,6 +497,8 @@ def run_ours(args, rank, world, local):
                                      "pass2": "pass 2 (k_solid_sweep + k_emit + k_upsert)"} if kernel_ms["solid"][0] > 0 else
                                     {"pass1": "pass 1 (k_ladder_pass1 / k_ladder_pass1_roll: one sweep, t_solid-level "
                                                "gate ladder)",
+                                     "bins": "passes 1 and 2 over minimizer bins (k_bin_runs, k_bin_scatter, k_bin_agg, "
+                                             "k_singles, k_bin_gate)",
                                      "pass2": "pass 2 (record emit k_emit_roll / k_emit_flat + k_count_records + "
                                               "k_upsert / k_upsert_all)"})[dom],
                          "bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
@@ -500,8 +506,8 @@ def run_ours(args, rank, world, local):
                          "traffic_source": traffic_src,
                          "alg_bytes_per_pass": per_pass_bytes, "ms_per_pass": per_pass_ms,
                          "note": "per pass = one k of one step; achieved = algorithmic bytes / event-timed kernel time"},
-            # the second figure the path is bound by: L2 atomics, counted as the edge-counter
-            # atomics of the upserts (one per transition push) over the upsert time
+            # the edge-counter atomics of the record buckets' upserts (one per transition push)
+            # over the upsert time, where that form ran
             "l2_atomics": {"kind": "edge-counter atomics of pass 2 (one per transition push)",
                            "ops_per_step": sum(pushes.values()),
                            "per_s": sum(pushes.values()) * args.steps / (kernel_ms["pass2_upsert"][0] / 1e3)

@@ -419,6 +419,7 @@ FBK_API fbk_status fbk_ctx_set_tuning(fbk_ctx* ctx, const char* name, double v) 
     else if (n == "filter_sizing" && (v == 0 || v == 1)) ctx->filter_sizing = (int)v;
     else if (n == "filter_load" && v >= 0.02 && v <= 0.9) ctx->filter_load = v;
     else if (n == "acc_filter" && (v == 0 || v == 1 || v == 2)) ctx->acc_filter = (int)v;
+    else if (n == "build_form" && (v == 0 || v == 1)) ctx->build_form = (int)v;
     else if (n == "upsert_all" && (v == 0 || v == 1 || v == 2)) ctx->upsert_all = (int)v;
     // the pass kernels are compiled for blocks of at most 256 threads
     else if (n == "block_pass1" && v >= 32 && v <= 256 && ((int)v % 32) == 0) ctx->block_pass1 = (int)v;
@@ -427,6 +428,11 @@ FBK_API fbk_status fbk_ctx_set_tuning(fbk_ctx* ctx, const char* name, double v) 
     else if (n == "block_emit" && v >= 32 && v <= 256 && ((int)v % 32) == 0) ctx->block_emit = (int)v;
     else if (n == "grid_pass2" && v >= 0) ctx->grid_pass2 = (int)v;
     else return set_err(ctx, FBK_ERR_INVALID, "unknown tuning name or value out of range: " + n);
+    // an option of the record buckets asks for that form of the build
+    for (const char* r : {"bucket_bytes", "stripes", "load_factor", "pass2_mode", "record_factor", "ladder_ilp", "emit_lookahead",
+                          "upsert_queue", "filter_sizing", "filter_load", "upsert_all", "block_pass1", "grid_pass1", "block_pass2",
+                          "block_emit", "grid_pass2"})
+        if (n == r) ctx->records_tuned = true;
     return FBK_OK;
 }
 
@@ -447,6 +453,7 @@ FBK_API fbk_status fbk_ctx_get_tuning(const fbk_ctx* ctx, const char* name, doub
     else if (n == "filter_sizing") *v = ctx->filter_sizing;
     else if (n == "filter_load") *v = ctx->filter_load;
     else if (n == "acc_filter") *v = ctx->acc_filter;
+    else if (n == "build_form") *v = ctx->build_form;
     else if (n == "upsert_all") *v = ctx->upsert_all;
     else if (n == "block_pass1") *v = ctx->block_pass1;
     else if (n == "grid_pass1") *v = ctx->grid_pass1;
@@ -561,7 +568,7 @@ void scan_arenas(const fbk_arena_view* arenas, int n_arenas, ArenaScan& sc) {
     struct Part {
         uint64_t bases = 0, max_pair = 0, long_bases = 0;
         uint32_t max_len = 0;
-        bool bad = false;
+        bool bad = false, disjoint = true;
         std::vector<uint64_t> hist;
     };
     std::vector<Part> parts(host_threads());
@@ -573,6 +580,7 @@ void scan_arenas(const fbk_arena_view* arenas, int n_arenas, ArenaScan& sc) {
         uint64_t bases = 0;
         for (uint64_t i = jobs[j].lo; i < jobs[j].hi; ++i) {
             const uint32_t L = v.lengths[i];
+            if (i) P.disjoint &= v.offsets[i] >= v.offsets[i - 1] + v.lengths[i - 1];
             // every sequence must lie inside its arena's words: the kernels read only there
             P.bad |= L && v.offsets[i] + (uint64_t)L > cap;
             bases += L;
@@ -592,6 +600,7 @@ void scan_arenas(const fbk_arena_view* arenas, int n_arenas, ArenaScan& sc) {
         sc.max_len = std::max(sc.max_len, P.max_len);
         sc.long_bases += P.long_bases;
         sc.bad |= P.bad;
+        sc.disjoint &= P.disjoint;
         for (uint64_t L = 0; L <= std::min<uint64_t>(P.max_len, ArenaScan::BINS - 1); ++L) sc.hist[L] += P.hist[L];
     }
     for (int a = 0; a < n_arenas; ++a) sc.n_reads += arenas[a].n_seqs;
@@ -632,6 +641,7 @@ fbk_status bank_upload_impl(fbk_ctx* ctx, const fbk_arena_view* arenas, int n_ar
     b->n_words = n_words;
     b->n_bases = n_bases;
     b->max_len = max_len;
+    b->disjoint = sc.disjoint;
     b->n_pairs = all_pairs && n_reads ? max_pair + 1 : 0;
     b->data = (uint64_t*)dev_alloc(ctx, (n_words + 8) * 8);
     b->off = (uint64_t*)dev_alloc(ctx, std::max<uint64_t>(n_reads, 1) * 8);
@@ -1638,6 +1648,15 @@ static fbk_status build_front_ladder(fbk_ctx* ctx, const fbk_bank* b, const fbk_
     const int nw = nw_of(p->key_bits);
     if (!nw || p->k < 1 || p->k > max_k_of(p->key_bits)) return set_err(ctx, FBK_ERR_INVALID, "k out of range for key_bits");
     if (log2w < 1 || log2w > 30) return set_err(ctx, FBK_ERR_INVALID, "cms_log2_width out of range");
+    if (bins_applicable(ctx, b, p, log2w)) {
+        uint64_t* kb = nullptr;
+        fbk_status st = make_keep_bits(ctx, b, ss, &kb);
+        bool declined = false;
+        if (st == FBK_OK) st = bins_build(ctx, b, p, kb, log2w, out, &declined);
+        cudaStreamSynchronize(ctx->stream);
+        dev_free(ctx, kb);
+        if (st || !declined) return st;
+    }
     Ladder lad;
     lad.log2w = log2w;
     const uint64_t lad_bytes = (uint64_t)p->t_solid * (4ULL << log2w) / 8 + 256;

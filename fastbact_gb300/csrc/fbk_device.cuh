@@ -168,6 +168,36 @@ __device__ __forceinline__ void window_canonical(const uint64_t* __restrict__ d,
     }
 }
 
+// Rolls both strands by one base c entering at the right end.  topb = 2k - 2 - 64 (NK - 1)
+// is the bit of the first base in the most significant word; tmask masks that word.
+template <int NK>
+__device__ __forceinline__ void roll_strands(uint64_t (&F)[NK], uint64_t (&R)[NK], uint32_t c, uint32_t topb, uint64_t tmask) {
+#pragma unroll
+    for (int i = 0; i < NK - 1; ++i) F[i] = (F[i] << 2) | (F[i + 1] >> 62);
+    F[NK - 1] = (F[NK - 1] << 2) | c;
+    F[0] &= tmask;
+#pragma unroll
+    for (int i = NK - 1; i > 0; --i) R[i] = (R[i] >> 2) | (R[i - 1] << 62);
+    R[0] = (R[0] >> 2) | ((uint64_t)(3u - c) << topb);
+}
+
+// Canonical key (NW words, the leading WS zero) and strand of the rolled window:
+// rc is taken iff rc < fwd (build.rs:102,258).
+template <int NW, int WS>
+__device__ __forceinline__ void strands_canonical(const uint64_t (&F)[NW - WS], const uint64_t (&R)[NW - WS], Key<NW>& can,
+                                                  bool& is_rc) {
+    constexpr int NK = NW - WS;
+    bool lt = false, eq = true;
+#pragma unroll
+    for (int i = 0; i < NK; ++i) {
+        lt = lt || (eq && R[i] < F[i]);
+        eq = eq && R[i] == F[i];
+    }
+    is_rc = lt;
+#pragma unroll
+    for (int i = 0; i < NW; ++i) can.w[i] = i < WS ? 0ULL : (lt ? R[i >= WS ? i - WS : 0] : F[i >= WS ? i - WS : 0]);
+}
+
 // Counter index of row r for key in a 4 x 2^log2w Count-Min Sketch (sketch.rs:193-195).
 __device__ __forceinline__ uint64_t cms_index(uint64_t key, int r, uint32_t log2w) {
     const uint64_t col = smix(key ^ cms_seed(r)) & ((1ULL << log2w) - 1);

@@ -459,6 +459,7 @@ FBK_API fbk_status fbk_ingest_fastq_device(fbk_ctx* ctx, const uint8_t* r1, uint
     bk->n_words = n_words;
     bk->n_bases = nb[0] + nb[1] + nb[2];
     bk->n_pairs = n_pairs;
+    bk->disjoint = true;
     uint32_t max_len = 0;
     for (int a = 0; a < 3; ++a) {
         bk->arena_reads.push_back(nr[a]);

@@ -99,6 +99,11 @@ struct fbk_ctx {
     // where a bucket holds more survivors than bucket 0 predicted).
     int filter_sizing = 1;
     double filter_load = 0.3;
+    // Builds that do not return their sketch: 1 (default) minimizer bins (fbk_bins.cu) where
+    // they apply, 0 record buckets.  Setting any option of the record buckets (bucket_bytes,
+    // ladder_ilp, ...) takes the context's builds there too.
+    int build_form = 1;
+    bool records_tuned = false;
     int batch_pass1 = 0;                  // batches with a ladder gate: 0 autotuned, 1 one multi-isolate launch, 2 a launch per isolate
     // Unfiltered passes: 1 upserts every bucket in one persistent launch, 2 (default) the
     // same with every lane's probe advanced a slot per step (64/128-bit keys; per 100x
@@ -125,6 +130,7 @@ struct fbk_bank {
     uint64_t max_chunk_bases() const { return max_chunk; }
     std::vector<uint64_t> len_hist;      // read-length histogram (last bin: all longer reads)
     uint64_t long_bases = 0;             // bases of reads in the last bin
+    bool disjoint = false;               // the reads lie one after another in the words, none overlapping the next
     cudaEvent_t ready = nullptr;         // an asynchronous upload's copies (null: uploaded synchronously)
     // upper bound of the windows of length k in reads with len >= min_len
     uint64_t windows(uint32_t k, uint32_t min_len) const {
@@ -200,6 +206,7 @@ struct ArenaScan {
     uint64_t n_reads = 0, n_bases = 0, max_pair = 0;
     uint32_t max_len = 0;
     bool bad = false;
+    bool disjoint = true;                     // in every arena a read starts at or after the end of the one before
     std::vector<uint64_t> hist, block_bases;  // hist over lengths < BINS - 1 (capped index)
     uint64_t long_bases = 0;                  // bases of reads of length >= BINS - 1
 };
@@ -249,6 +256,13 @@ fbk_status solid_build(fbk_ctx* ctx, const fbk_bank* b, const fbk_cms* cms, cons
 // The same with the pass-1 gate as a t_solid-level ladder (fbk_k_ladder.cu).
 fbk_status solid_build_ladder(fbk_ctx* ctx, const fbk_bank* b, uint32_t* ladder, uint32_t log2w, const fbk_build_params* p,
                               const uint64_t* keep_bits, uint64_t distinct_hint, fbk_table** out);
+
+// The build front end over minimizer bins (fbk_bins.cu); *declined is set when the reads'
+// shape does not suit it and the caller should take the record buckets.
+constexpr uint32_t BINS_MIN_K = 17;
+bool bins_applicable(const fbk_ctx* ctx, const fbk_bank* b, const fbk_build_params* p, uint32_t log2w);
+fbk_status bins_build(fbk_ctx* ctx, const fbk_bank* b, const fbk_build_params* p, const uint64_t* keep_bits, uint32_t log2w,
+                      fbk_table** out, bool* declined);
 
 // host f64 HyperLogLog::estimate from the register sum and zero count (sketch.rs:83-114)
 double hll_estimate_from_sum(double sum, uint64_t zeros, uint32_t p);

@@ -167,7 +167,10 @@ FBK_API fbk_status fbk_ctx_event_elapsed(fbk_ctx* ctx, int slot_a, int slot_b, d
  * 3 = 2 ahead over a flattened window stream, 4 = one lane per read with rolled k-mers
  * (the default), 5 = the same at two blocks per SM for every key width), "acc_filter"
  * (keys that cannot become SolidKmerNodes stay out of the table, see fbk_table_flags:
- * 0 never, 1 where it pays, 2 always), "upsert_all" (1: an unfiltered pass upserts every
+ * 0 never, 1 where it pays, 2 always), "build_form" (1, the default: builds that do not
+ * return their sketch run over minimizer bins where those apply; 0: over record buckets, as
+ * does every build of a context on which an option of the record buckets was set),
+ * "upsert_all" (1: an unfiltered pass upserts every
  * bucket in one persistent launch), "upsert_queue" (1: filtered upserts queue the
  * filter's survivors per warp before probing), "filter_sizing" (1: a filtered pass sizes
  * its table from the first bucket's survivors, at load "filter_load"), "batch_pass1"
@@ -269,8 +272,9 @@ FBK_API fbk_status fbk_table_info(const fbk_table* t, uint64_t* n_keys, uint64_t
 /* FBK_TABLE_ACC_FILTERED: the accumulator holds only the keys that may become
  * SolidKmerNodes.  A key's edge counter grows by at most one per window of the key,
  * so a key seen in fewer than min_trans_cov windows has an empty mask; with the
- * tuning acc_filter = 2 such keys are kept out of the table when the pass runs in one
- * read chunk without prior contigs; acc_filter = 1 (default) does so where the saving
+ * tuning acc_filter = 2 such keys are kept out of the table (all of them, or most: the
+ * form of the build decides) when the pass runs in one read chunk without prior
+ * contigs; acc_filter = 1 (default) does so where the saving
  * outweighs the cost of counting: 256-bit keys, and passes whose distinct k-mers
  * exceed a fifth of their windows.  The SolidKmerNode rows, their
  * digest and fbk_table_pushes are unchanged; n_keys and fbk_table_export_acc cover

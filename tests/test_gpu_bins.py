@@ -1,0 +1,118 @@
+"""The build over minimizer bins at the sizes where it can go wrong, against the oracle:
+the accumulator, the SolidKmerNode rows and the digest (integers, tolerance 0).
+
+k = 17 is the smallest it takes; 31/32/33, 63/64/65 and 95/96/97 are the word edges of the
+key; 127 the largest k.  The banks hold reads of exactly k and k + 1 bases among ordinary
+ones (windows with no neighbour, with one, with two, of the same k-mers and of their reverse
+complements), more distinct keys than a group's entries (windows put off to a later turn, and
+a group taken in parts), groups of more than 65535 windows (wide counts), reads cut into
+several runs, and reads that overlap in the packed words (left to the record buckets)."""
+import numpy as np
+import pytest
+
+from fastbact_gb300 import api
+from test_gpu_parity import compare_gate_only, rand_seqs
+
+pytestmark = pytest.mark.gpu
+
+COMP = bytes.maketrans(b"ACGT", b"TGCA")
+KS = [(17, 64), (21, 64), (31, 64), (32, 128), (33, 128), (63, 128), (64, 256), (65, 256), (95, 256), (96, 256), (97, 256),
+      (127, 256)]
+
+
+def rc(s):
+    return s[::-1].translate(COMP)
+
+
+def bank_of(seqs):
+    a, b = len(seqs) // 3, 2 * len(seqs) // 3
+    return api.ReadBank(api.BitSeqArena.from_seqs(seqs[:a]), api.BitSeqArena.from_seqs(seqs[a:b]), api.BitSeqArena.from_seqs(seqs[b:]))
+
+
+def low_minimizer():
+    """A 15-mer whose hash is below nearly every other's, so that it is the minimizer of
+    every window that holds it (the hash of k_bin_runs)."""
+    rng = np.random.default_rng(7)
+    codes = rng.integers(0, 4, (1 << 20, 15)).astype(np.uint64)
+    w = np.uint64(4) ** np.arange(15, dtype=np.uint64)
+    rev = (3 - codes) @ w                   # base i at bits 2 i: the reverse complement's integer
+    fwd = codes @ w[::-1]
+    z = ((np.minimum(fwd, rev) ^ np.uint64(0x3C6EF372)) * np.uint64(0x9E3779B1)) & np.uint64(0xFFFFFFFF)
+    z ^= z >> np.uint64(15)
+    z = (z * np.uint64(0x85EBCA77)) & np.uint64(0xFFFFFFFF)
+    return bytes(b"ACGT"[c] for c in codes[int(np.argmin(z))])
+
+
+@pytest.mark.parametrize("k,kb", KS)
+@pytest.mark.parametrize("acc_filter", [0, 1, 2])
+def test_short_reads_and_word_edges(k, kb, acc_filter):
+    rng = np.random.default_rng(k)
+    genome = rand_seqs(int(rng.integers(1 << 30)), 1, 3000, 3000)[0]
+    seqs = []
+    for i in range(0, 2700, 7):
+        seqs.append(genome[i:i + 290])
+    for i in range(0, 2700, 11):  # one window, two windows, both strands; some seen only here
+        seqs += [genome[i:i + k], rc(genome[i + 3:i + 3 + k + 1]), rc(genome[i:i + k])]
+    seqs += rand_seqs(5, 40, k, k) + rand_seqs(6, 40, k + 1, k + 2) + rand_seqs(8, 20, 1, k - 1) + [b"", b"A" * 400, b"AC" * 150]
+    lone = rand_seqs(9, 30, k + 2, k + 2)   # a window without neighbours, then the same k-mer with both
+    seqs += [s[1:-1] for s in lone] + lone
+    order = rng.permutation(len(seqs))
+    c = api.Context(0)
+    try:
+        c.set_tuning(acc_filter=acc_filter)
+        compare_gate_only(c, bank_of([seqs[i] for i in order]), k, kb, 16, None, 12)
+        compare_gate_only(c, bank_of([seqs[i] for i in order]), k, kb, 4, 2, 14)
+    finally:
+        c.close()
+
+
+@pytest.mark.parametrize("k,kb", [(21, 64), (31, 64), (45, 128), (77, 256)])
+def test_more_keys_than_a_group_holds(ctx, k, kb):
+    """All keys distinct (put off to later turns), then 20,000 windows of one minimizer (taken
+    in parts), some of them twice."""
+    seqs = rand_seqs(3, 700, 100, 400)
+    compare_gate_only(ctx, bank_of(seqs), k, kb, 16, None, 14)
+    x = low_minimizer()
+    flank = rand_seqs(4, 2400, 60, 80)
+    seqs = [flank[i] + x + flank[i + 1] for i in range(0, 2400, 2)]
+    seqs += [rc(s) for s in seqs[::9]] + [s[5:] for s in seqs[::7]]
+    compare_gate_only(ctx, bank_of(seqs), k, kb, 16, None, 16)
+
+
+@pytest.mark.parametrize("k,kb", [(21, 64), (55, 128), (99, 256)])
+def test_groups_with_wide_counts(ctx, k, kb):
+    """One k-mer 100,000 times and more (its counts pass 65535), with reads of several
+    thousand bases (runs cut every 2048 windows) and ordinary ones around it."""
+    seqs = [b"A" * 3000] * 30 + [b"T" * 2500] * 20 + [b"ACG" * 900] * 50 + rand_seqs(11, 200, 150, 300)
+    compare_gate_only(ctx, bank_of(seqs), k, kb, 16, None, 12)
+
+
+@pytest.mark.parametrize("k", [21, 33, 77])
+def test_sampled_sizes(ctx, k):
+    """Above 4 M windows a sample of the bins sizes the groups and the rows."""
+    p = api.synth_params(seed=91, genome_len=150_000, coverage=60.0, sub_rate=0.008, n_repeats=3, repeat_len=900)
+    bank = api.synth_isolate(p, threads=0, sample_pairs=0)[0]
+    assert sum(int(np.maximum(a.lengths.astype(np.int64) - k + 1, 0).sum()) for a in bank.arenas) > 4 << 20
+    compare_gate_only(ctx, bank, k, api.key_bits_for_k(k), 16, None, 18)
+
+
+def test_overlapping_reads():
+    """Reads that share packed words: adjacent windows of the bank need not be a read's.
+    (Every accumulated key is kept: which ones a filter keeps is the form's own.)"""
+    ctx = api.Context(0)
+    ctx.set_tuning(acc_filter=0)
+    a = api.BitSeqArena.from_seqs(rand_seqs(21, 1, 4000, 4000))
+    offs = np.array([0, 50, 50, 70, 100, 60, 3000, 2990], np.uint64)
+    lens = np.array([80, 100, 100, 31, 300, 40, 200, 220], np.uint32)
+    seq = a.extract_ascii(0)
+    shared = api.ReadBank(api.BitSeqArena(a.data, offs, lens), api.BitSeqArena(), api.BitSeqArena())
+    apart = api.ReadBank(api.BitSeqArena.from_seqs([seq[int(o):int(o + n)] for o, n in zip(offs, lens)]))
+    got = []
+    for bank in (shared, apart):
+        t = api.build_cdbg_ext(bank, 31, 1, 100000, ctx=ctx, counter_bits=4, cms_log2_width=12)
+        u = api.build_cdbg_ext(bank, 31, None, 100000, ctx=ctx, counter_bits=4, cms_log2_width=12)
+        got.append((t.digest(), t.pushes(), u.digest(), u.pushes(), u.acc_digest()))
+        t.release()
+        u.release()
+    ctx.close()
+    assert got[0] == got[1]
