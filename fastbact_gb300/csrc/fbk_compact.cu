@@ -7,14 +7,19 @@
 // skipped; then it walks the remaining all-1-in-1-out cycles; then it links unitigs
 // whose ends overlap by k or k-1 bases.  Here:
 //   1. a node index (open addressing over the converted rows) is built on the device;
-//   2. every (boundary node, direction, out-edge) start walks its path on the device,
-//      one thread per start, with no shared marks: a unitig reachable from both ends
-//      is kept from the end whose (row, direction, edge) is smaller — the same set of
-//      unitigs, decided without ordering;
-//   3. a second walk writes the bases of the kept paths and marks their nodes, and a
-//      per-unitig pass stores min(sequence, reverse complement) as the reference does;
-//   4. the 1-in-1-out nodes no path visited (isolated cycles, few) and the overlap
+//   2. the successor of every 1-in-1-out directed node is looked up once, and doubled: table
+//      l holds the node 2^l steps on, as long as all of them are 1-in-1-out;
+//   3. every (boundary node, direction, out-edge) start finds its path's length and end by
+//      descending those tables, one thread per start, with no shared marks: a unitig
+//      reachable from both ends is kept from the end whose (row, direction, edge) is smaller
+//      — the same set of unitigs, decided without ordering;
+//   4. the bases of the kept paths are written eight to a thread, each thread jumping to its
+//      place, already in the orientation of min(sequence, reverse complement);
+//   5. the 1-in-1-out nodes no path visited (isolated cycles, few) and the overlap
 //      edges are handled on the host, as build.rs:450-594 does.
+// A walk of one thread along a whole unitig is a chain of dependent loads, about 1 us a
+// step: 44 ms twice for the 42 k steps of the longest unitig of a 1 Mbp genome (k = 31, 1.0 M
+// rows), where the tables take 0.25 ms, the paths 0.05 and their bases 0.04.
 // A unitig's coverage is the mean node coverage of its path without the last node
 // (build.rs:379-435); which end a path starts from therefore changes its coverage
 // when the end nodes differ, exactly as the reference's map order does.
@@ -62,6 +67,44 @@ __host__ __device__ __forceinline__ uint32_t kbase(const Key<NW>& x, uint32_t i,
     // base i from the 5' end (i = 0: most significant)
     const uint32_t pos = 2 * (k - 1 - i);
     return (uint32_t)(x.w[NW - 1 - pos / 64] >> (pos % 64)) & 3u;
+}
+// Base 0 (the 5' end) and the reverse complement, on registers (no word index of its own).
+template <int NW>
+__device__ __forceinline__ uint32_t kfirst(const Key<NW>& x, uint32_t k) {
+    const uint32_t pos = 2 * (k - 1), wd = NW - 1 - pos / 64;
+    uint64_t v = 0;
+#pragma unroll
+    for (int i = 0; i < NW; ++i) v = (uint32_t)i == wd ? x.w[i] : v;
+    return (uint32_t)(v >> (pos % 64)) & 3u;
+}
+template <int NW>
+__device__ __forceinline__ Key<NW> krc_dev(const Key<NW>& x, uint32_t k) {
+    // all 32 NW groups reversed and complemented, then the 64 NW - 2k bits of padding dropped
+    const uint32_t s = 64u * NW - 2u * k, ws = s >> 6, bs = s & 63;
+    uint64_t y[NW];
+#pragma unroll
+    for (int i = 0; i < NW; ++i) y[i] = ~rev2(x.w[NW - 1 - i]);
+    Key<NW> r;
+#pragma unroll
+    for (int i = 0; i < NW; ++i) {
+        uint64_t hi = 0, lo = 0;  // words i - ws and i - ws - 1
+#pragma unroll
+        for (int j = 0; j < NW; ++j) {
+            hi = (uint32_t)(i - j) == ws ? y[j] : hi;
+            lo = (uint32_t)(i - j - 1) == ws ? y[j] : lo;
+        }
+        r.w[i] = (hi >> bs) | (bs ? lo << (64 - bs) : 0ULL);
+    }
+    return r;
+}
+template <int NW>
+__device__ __forceinline__ void kshr2_put_dev(Key<NW>& x, uint32_t c, uint32_t k) {
+#pragma unroll
+    for (int i = NW - 1; i >= 0; --i) x.w[i] = (x.w[i] >> 2) | (i > 0 ? (x.w[i - 1] << 62) : 0ULL);
+    const uint32_t pos = 2 * (k - 1), wd = NW - 1 - pos / 64;
+#pragma unroll
+    for (int i = 0; i < NW; ++i)
+        if ((uint32_t)i == wd) x.w[i] |= (uint64_t)c << (pos % 64);
 }
 template <int NW>
 __host__ __device__ __forceinline__ Key<NW> krc(const Key<NW>& x, uint32_t k) {
@@ -142,19 +185,85 @@ __global__ void k_cidx_build(const uint64_t* __restrict__ keys, uint64_t n, uint
 
 __device__ __forceinline__ uint32_t pc4(uint32_t v) { return __popc(v & 15u); }
 
-// Walk starts per row: every out-edge of both directions of a boundary row.
-__global__ void k_walk_count(const uint8_t* __restrict__ mask, uint64_t n, uint32_t* cnt) {
-    for (uint64_t r = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; r < n; r += (uint64_t)gridDim.x * blockDim.x) {
-        const uint32_t m = mask[r];
-        const bool boundary = pc4(m) != 1 || pc4(m >> 4) != 1;
-        cnt[r] = boundary ? pc4(m) + pc4(m >> 4) : 0;
+__device__ __forceinline__ bool one_in_one_out(uint32_t m) { return pc4(m) == 1 && pc4(m >> 4) == 1; }
+
+// Walk starts of a row: every out-edge of both directions of a boundary row.
+__device__ __forceinline__ uint32_t starts_of(uint32_t m) { return one_in_one_out(m) ? 0u : pc4(m) + pc4(m >> 4); }
+
+// Exclusive prefix sums of n values v(i), in tiles of 2048: the tiles' sums, then every tile's
+// prefix from the sums before it.  pre[n] is the total.
+constexpr uint32_t PRE_TILE = 2048;
+template <class Fn>
+__global__ void __launch_bounds__(256) k_tile_sums(Fn v, uint64_t n, uint64_t* __restrict__ part) {
+    __shared__ uint64_t s[8];
+    uint64_t t = 0;
+    for (uint32_t j = 0; j < PRE_TILE / 256; ++j) {
+        const uint64_t i = (uint64_t)blockIdx.x * PRE_TILE + j * 256 + threadIdx.x;
+        if (i < n) t += v(i);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
+    if ((threadIdx.x & 31) == 0) s[threadIdx.x >> 5] = t;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int j = 1; j < 8; ++j) t += s[j];
+        part[blockIdx.x] = t;
     }
 }
+template <class Fn>
+__global__ void __launch_bounds__(256) k_tile_prefix(Fn v, uint64_t n, const uint64_t* __restrict__ part, uint64_t* __restrict__ pre) {
+    __shared__ uint64_t s[8], s_base;
+    const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    uint64_t t = 0;
+    for (uint32_t j = threadIdx.x; j < blockIdx.x; j += 256) t += part[j];
+    __syncwarp();
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
+    if (lane == 0) s[w] = t;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int j = 1; j < 8; ++j) t += s[j];
+        s_base = t;
+    }
+    __syncthreads();
+    const uint64_t i0 = (uint64_t)blockIdx.x * PRE_TILE + threadIdx.x * 8;
+    uint64_t x[8], sum = 0;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        x[j] = i0 + j < n ? v(i0 + j) : 0;
+        sum += x[j];
+    }
+    uint64_t inc = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint64_t y = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= (uint32_t)o) inc += y;
+    }
+    if (lane == 31) s[w] = inc;
+    __syncthreads();
+    uint64_t p = s_base + inc - sum;
+    for (uint32_t j = 0; j < w; ++j) p += s[j];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        if (i0 + j < n) pre[i0 + j] = p;
+        p += x[j];
+        if (i0 + j + 1 == n) pre[n] = p;
+    }
+}
+struct StartCount {
+    const uint8_t* mask;
+    __device__ uint64_t operator()(uint64_t i) const { return starts_of(mask[i]); }
+};
+struct PathLength {
+    const uint32_t* len;
+    __device__ uint64_t operator()(uint64_t i) const { return len[i]; }
+};
+
 // Start list from the exclusive prefix of the counts: start = row << 4 | dir << 3 | edge.
 __global__ void k_walk_starts(const uint8_t* __restrict__ mask, uint64_t n, const uint64_t* __restrict__ pre, uint64_t* starts) {
     for (uint64_t r = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; r < n; r += (uint64_t)gridDim.x * blockDim.x) {
         const uint32_t m = mask[r];
-        if (pc4(m) == 1 && pc4(m >> 4) == 1) continue;
+        if (one_in_one_out(m)) continue;
         uint64_t o = pre[r];
         for (uint32_t dir = 0; dir < 2; ++dir) {
             const uint32_t out = dir ? (m >> 4) & 15u : m & 15u;
@@ -164,95 +273,178 @@ __global__ void k_walk_starts(const uint8_t* __restrict__ mask, uint64_t n, cons
     }
 }
 
-// One walk (build.rs:349-445 without the marks).  Returns the bases (k + steps), the
-// coverage sum and points, and whether this start keeps the unitig.  When `seq` is
-// given, writes the bases in walk orientation and marks the visited rows.
+// A directed node is row << 1 | direction (1: the reverse complement of the row's key).
+constexpr uint32_t NO_NODE = 0xFFFFFFFFu;
+
+// The k-mer of a directed node and its reverse complement, moved one base along edge b: the
+// row it leads to (-1: none) and the direction in which that is entered.
 template <int NW>
-__device__ void walk(const Rows& R, uint32_t k, uint64_t start, uint64_t max_steps, uint64_t& len, unsigned long long& cov_sum,
-                     uint64_t& points, bool& keep, uint8_t* seq, uint8_t* visited, uint32_t* status) {
-    const uint64_t r0 = start >> 4;
-    const uint32_t dir0 = (uint32_t)(start >> 3) & 1u, b0 = (uint32_t)start & 7u;
-    const Key<NW> u = row_key<NW>(R, r0);
-    Key<NW> f = dir0 ? krc<NW>(u, k) : u;
-    Key<NW> rv = dir0 ? u : krc<NW>(u, k);
-    if (seq) {
-        for (uint32_t i = 0; i < k; ++i) seq[i] = "ACGT"[kbase<NW>(f, i, k)];
-        visited[r0] = 1;
+__device__ __forceinline__ int64_t take_edge(const Rows& R, uint32_t k, uint64_t row, uint32_t dir, uint32_t b, Key<NW>& f, Key<NW>& rv,
+                                             uint32_t& rc_p, bool& c_rc) {
+    const Key<NW> u = row_key<NW>(R, row), ur = krc_dev<NW>(u, k);
+    f = dir ? ur : u;
+    rv = dir ? u : ur;
+    rc_p = 3u - kfirst<NW>(f, k);
+    kshl2_push<NW>(f, b, k);
+    kshr2_put_dev<NW>(rv, 3u - b, k);
+    c_rc = kless<NW>(rv, f);
+    return find_row<NW>(R, c_rc ? rv : f);
+}
+__device__ __forceinline__ uint32_t only_edge(uint32_t m, uint32_t dir) { return __ffs(dir ? (m >> 4) & 15u : m & 15u) - 1; }
+
+// The successor of every directed 1-in-1-out node, where it is one too.
+template <int NW>
+__global__ void __launch_bounds__(256) k_next(Rows R, uint32_t k, uint32_t* __restrict__ next) {
+    for (uint64_t s = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; s < 2 * R.n; s += (uint64_t)gridDim.x * blockDim.x) {
+        const uint32_t m = R.mask[s >> 1];
+        uint32_t to = NO_NODE;
+        if (one_in_one_out(m)) {
+            Key<NW> f, rv;
+            uint32_t rc_p;
+            bool c_rc;
+            const int64_t r = take_edge<NW>(R, k, s >> 1, (uint32_t)s & 1u, only_edge(m, (uint32_t)s & 1u), f, rv, rc_p, c_rc);
+            if (r >= 0 && one_in_one_out(R.mask[r])) to = (uint32_t)(r << 1) | (c_rc ? 1u : 0u);
+        }
+        next[s] = to;
     }
-    uint32_t rc_p = 3u - kbase<NW>(f, 0, k);
-    kshl2_push<NW>(f, b0, k);
-    kshr2_put<NW>(rv, 3u - b0, k);
-    len = k + 1;
-    if (seq) seq[k] = "ACGT"[b0];
-    cov_sum = R.cov[r0];
-    points = 1;
-    keep = true;
-    for (uint64_t step = 0;; ++step) {
-        const bool c_rc = kless<NW>(rv, f);
-        const Key<NW> can = c_rc ? rv : f;
-        const int64_t rc = find_row<NW>(R, can);
-        if (rc < 0) return;  // the path ends at a k-mer with no node: no walk comes back
-        const uint32_t m = R.mask[rc];
-        const uint32_t c_out = c_rc ? (m >> 4) & 15u : m & 15u;
-        const uint32_t c_in = c_rc ? m & 15u : (m >> 4) & 15u;
-        if (__popc(c_in) != 1 || __popc(c_out) != 1) {
-            // boundary end: the walk from (rc, !c_rc, rc_p) covers the same unitig
-            const uint32_t back = c_rc ? m & 15u : (m >> 4) & 15u;  // out-edges of the opposite direction
-            if ((back >> rc_p) & 1u) {
-                const uint64_t other = ((uint64_t)rc << 4) | ((uint64_t)(c_rc ? 0u : 1u) << 3) | rc_p;
-                keep = start <= other;
+}
+// Table l + 1 from table l; any: whether an entry is left.
+__global__ void __launch_bounds__(256) k_double(const uint32_t* __restrict__ in, uint32_t* __restrict__ out, uint64_t n, uint32_t* any) {
+    bool some = false;
+    for (uint64_t s = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; s < n; s += (uint64_t)gridDim.x * blockDim.x) {
+        const uint32_t a = in[s], b = a == NO_NODE ? NO_NODE : in[a];
+        out[s] = b;
+        some |= b != NO_NODE;
+    }
+    if (__any_sync(0xffffffffu, some) && (threadIdx.x & 31) == 0) atomicOr(any, 1u);
+}
+
+constexpr int MAX_TABLES = 33;
+struct Jumps {
+    const uint32_t* t[MAX_TABLES];  // t[l][s]: 2^l steps on from s
+    int n;
+};
+
+// A path (build.rs:349-445): its first 1-in-1-out node (NO_NODE: none), how many of them, and
+// how it is stored: 0 as walked, 1 reverse complemented, 2 decided once it is written.
+struct Path {
+    uint32_t first, nodes, flip;
+};
+template <int NW>
+__global__ void __launch_bounds__(256) k_paths(Rows R, Jumps J, uint32_t k, const uint64_t* __restrict__ starts, uint64_t n_starts,
+                                               uint32_t* __restrict__ len_out, Path* __restrict__ paths, uint32_t* status) {
+    for (uint64_t s = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; s < n_starts; s += (uint64_t)gridDim.x * blockDim.x) {
+        const uint64_t start = starts[s];
+        const uint64_t r0 = start >> 4;
+        const uint32_t dir0 = (uint32_t)(start >> 3) & 1u;
+        Key<NW> f, rv;
+        uint32_t rc_p;
+        bool c_rc;
+        Key<NW> head = row_key<NW>(R, r0);
+        if (dir0) head = krc_dev<NW>(head, k);
+        int64_t r = take_edge<NW>(R, k, r0, dir0, (uint32_t)start & 7u, f, rv, rc_p, c_rc);
+        Path p{NO_NODE, 0, 0};
+        if (r >= 0 && one_in_one_out(R.mask[r])) {
+            p.first = (uint32_t)(r << 1) | (c_rc ? 1u : 0u);
+            uint32_t at = p.first;
+            uint64_t nodes = 1;
+            for (int l = J.n - 1; l >= 0; --l) {
+                const uint32_t nx = J.t[l][at];
+                if (nx != NO_NODE) {
+                    at = nx;
+                    nodes += 1ULL << l;
+                }
             }
-            if (seq) visited[rc] = 1;
-            return;
+            if (nodes > R.n + 1) {  // a path longer than the node count: impossible for valid rows
+                atomicOr(status, ST_SPIN_TIMEOUT);
+                nodes = 1;
+            }
+            p.nodes = (uint32_t)nodes;
+            r = take_edge<NW>(R, k, at >> 1, at & 1u, only_edge(R.mask[at >> 1], at & 1u), f, rv, rc_p, c_rc);
         }
-        if (step >= max_steps) {
-            atomicOr(status, ST_SPIN_TIMEOUT);  // a path longer than the node count: impossible for valid rows
-            return;
+        bool keep = true;  // a path that ends at a k-mer with no node: no walk comes back
+        if (r >= 0) {
+            // boundary end: the walk from (r, !c_rc, rc_p) covers the same unitig
+            const uint32_t m = R.mask[r], back = c_rc ? m & 15u : (m >> 4) & 15u;
+            if ((back >> rc_p) & 1u) keep = start <= (((uint64_t)r << 4) | ((uint64_t)(c_rc ? 0u : 1u) << 3) | rc_p);
         }
-        if (seq) visited[rc] = 1;
-        const uint32_t nb = __ffs(c_out) - 1;
-        rc_p = 3u - kbase<NW>(f, 0, k);
-        kshl2_push<NW>(f, nb, k);
-        kshr2_put<NW>(rv, 3u - nb, k);
-        if (seq) seq[len] = "ACGT"[nb];
-        len++;
-        cov_sum += R.cov[rc];
-        points++;
+        // min(sequence, reverse complement) (build.rs:438-439): their first k bases decide
+        p.flip = kless<NW>(rv, head) ? 1u : keq<NW>(rv, head) ? 2u : 0u;
+        len_out[s] = keep ? k + 1 + p.nodes : 0;
+        paths[s] = p;
     }
 }
 
+// Writes the kept paths' bases, marks their nodes and sums the coverage of the start and the
+// 1-in-1-out nodes.  A thread takes 8 consecutive bases of the concatenated paths: it jumps
+// to the node of its first one and steps on from there.
 template <int NW>
-__global__ void k_walk_measure(Rows R, uint32_t k, const uint64_t* __restrict__ starts, uint64_t n_starts, uint64_t* len_out,
-                               unsigned long long* cov_out, uint64_t* pts_out, uint32_t* status) {
-    for (uint64_t s = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; s < n_starts; s += (uint64_t)gridDim.x * blockDim.x) {
-        uint64_t len, pts;
-        unsigned long long cs;
-        bool keep;
-        walk<NW>(R, k, starts[s], R.n + 1, len, cs, pts, keep, nullptr, nullptr, status);
-        len_out[s] = keep ? len : 0;
-        cov_out[s] = cs;
-        pts_out[s] = pts;
+__global__ void __launch_bounds__(256) k_path_bases(Rows R, Jumps J, uint32_t k, const uint64_t* __restrict__ starts, uint64_t n_starts,
+                                                    const uint32_t* __restrict__ len, const uint64_t* __restrict__ off,
+                                                    const Path* __restrict__ paths, uint64_t total, uint8_t* __restrict__ seqs,
+                                                    uint8_t* __restrict__ visited, unsigned long long* __restrict__ cov) {
+    for (uint64_t p0 = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) * 8; p0 < total; p0 += (uint64_t)gridDim.x * blockDim.x * 8) {
+        // the path of base p0: the last one that starts at or before it (paths not kept have
+        // no bases and start where the next one does)
+        uint64_t lo = 0, hi = n_starts;
+        while (hi - lo > 1) {
+            const uint64_t mid = (lo + hi) / 2;
+            if (off[mid] <= p0) lo = mid;
+            else hi = mid;
+        }
+        uint64_t s = lo;
+        const uint64_t p1 = min(p0 + 8, total);
+        uint64_t p = p0;
+        while (p < p1) {
+            while (!len[s] || off[s] + len[s] <= p) ++s;
+            const uint32_t L = len[s];
+            const uint64_t start = starts[s];
+            const Path path = paths[s];
+            const uint64_t end = min(p1, off[s] + L);
+            uint32_t j = (uint32_t)(p - off[s]);
+            uint32_t at = path.first;
+            if (j > k) {  // node j - k (1-based)
+                const uint32_t d = j - k - 1;
+                for (int l = 0; l < J.n; ++l)
+                    if ((d >> l) & 1u) at = J.t[l][at];
+            }
+            unsigned long long c = 0;
+            Key<NW> head;
+            if (j < k) {
+                head = row_key<NW>(R, start >> 4);
+                if ((start >> 3) & 1u) head = krc_dev<NW>(head, k);
+            }
+            for (; p < end; ++p, ++j) {
+                uint32_t b;
+                if (j < k) {
+                    const uint32_t pos = 2 * (k - 1 - j), wd = NW - 1 - pos / 64;
+                    uint64_t v = 0;
+#pragma unroll
+                    for (int i = 0; i < NW; ++i) v = (uint32_t)i == wd ? head.w[i] : v;
+                    b = (uint32_t)(v >> (pos % 64)) & 3u;
+                } else if (j == k) {
+                    b = (uint32_t)start & 7u;
+                    c += R.cov[start >> 4];
+                } else {
+                    const uint32_t row = at >> 1;
+                    b = only_edge(R.mask[row], at & 1u);
+                    c += R.cov[row];
+                    visited[row] = 1;
+                    at = J.t[0][at];
+                }
+                seqs[off[s] + (path.flip == 1 ? L - 1 - j : j)] = "ACGT"[path.flip == 1 ? 3u - b : b];
+            }
+            if (c) atomicAdd(&cov[s], c);
+        }
     }
 }
 
-template <int NW>
-__global__ void k_walk_write(Rows R, uint32_t k, const uint64_t* __restrict__ starts, uint64_t n_starts,
-                             const uint64_t* __restrict__ len, const uint64_t* __restrict__ off, uint8_t* seqs, uint8_t* visited,
-                             uint32_t* status) {
-    for (uint64_t s = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; s < n_starts; s += (uint64_t)gridDim.x * blockDim.x) {
-        if (!len[s]) continue;
-        uint64_t l, pts;
-        unsigned long long cs;
-        bool keep;
-        walk<NW>(R, k, starts[s], R.n + 1, l, cs, pts, keep, seqs + off[s], visited, status);
-    }
-}
-
-// min(sequence, reverse complement), in place (build.rs:438-439).
-__global__ void k_canon_seq(uint8_t* seqs, const uint64_t* __restrict__ off, const uint64_t* __restrict__ len, uint64_t n) {
+// min(sequence, reverse complement), in place, for the paths whose first k bases left it open.
+__global__ void k_canon_seq(uint8_t* seqs, const uint64_t* __restrict__ off, const uint32_t* __restrict__ len,
+                            const Path* __restrict__ paths, uint64_t n) {
     for (uint64_t s = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; s < n; s += (uint64_t)gridDim.x * blockDim.x) {
         const uint64_t L = len[s];
-        if (!L) continue;
+        if (!L || paths[s].flip != 2) continue;
         uint8_t* q = seqs + off[s];
         auto comp = [](uint8_t c) -> uint8_t { return c == 'A' ? 'T' : c == 'C' ? 'G' : c == 'G' ? 'C' : 'A'; };
         int cmp = 0;
@@ -271,11 +463,14 @@ __global__ void k_canon_seq(uint8_t* seqs, const uint64_t* __restrict__ off, con
     }
 }
 
-// Rows that are 1-in-1-out and on no path: candidates for isolated cycles.
-__global__ void k_cycle_candidates(const uint8_t* __restrict__ mask, const uint8_t* __restrict__ visited, uint64_t n, uint8_t* flag) {
+// Rows that are 1-in-1-out and on no path: candidates for isolated cycles, and how many.
+__global__ void k_cycle_candidates(const uint8_t* __restrict__ mask, const uint8_t* __restrict__ visited, uint64_t n, uint8_t* flag,
+                                   unsigned long long* n_flag) {
     for (uint64_t r = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; r < n; r += (uint64_t)gridDim.x * blockDim.x) {
         const uint32_t m = mask[r];
-        flag[r] = (!visited[r] && pc4(m) == 1 && pc4(m >> 4) == 1) ? 1 : 0;
+        const bool f = !visited[r] && one_in_one_out(m);
+        flag[r] = f ? 1 : 0;
+        if (f) atomicAdd(n_flag, 1ULL);
     }
 }
 
@@ -413,28 +608,30 @@ void link_unitigs(uint32_t k, fbk_unitigs* U) {
         if (U->u[id].circular) add(id, 0, id, 0, k - 1, 10);  // build.rs:546-547
     for (uint32_t ov : {k, k - 1}) {
         if (ov == 0) continue;
+        // an end of the reverse complement is the complement of the other end: the whole of it
+        // is never needed
         std::unordered_map<std::string, std::vector<std::pair<uint32_t, uint32_t>>> prefix;
-        std::vector<std::string> rcs(n);
-        for (uint32_t id = 0; id < n; ++id) {
-            const std::string& f = U->u[id].seq;
-            rcs[id] = rc_string(f);
-            if (f.size() >= ov) {
-                prefix[f.substr(0, ov)].push_back({id, 0});
-                prefix[rcs[id].substr(0, ov)].push_back({id, 1});
-            }
-        }
+        prefix.reserve(2 * (size_t)n);
+        std::vector<std::string> tail[2];  // last ov bases of both strands
+        tail[0].resize(n);
+        tail[1].resize(n);
         for (uint32_t id = 0; id < n; ++id) {
             const std::string& f = U->u[id].seq;
             if (f.size() < ov) continue;
-            auto a = prefix.find(f.substr(f.size() - ov));
-            if (a != prefix.end())
+            const std::string head = f.substr(0, ov);
+            tail[0][id] = f.substr(f.size() - ov);
+            tail[1][id] = rc_string(head);
+            prefix[head].push_back({id, 0});
+            prefix[rc_string(tail[0][id])].push_back({id, 1});
+        }
+        for (uint32_t id = 0; id < n; ++id) {
+            if (U->u[id].seq.size() < ov) continue;
+            for (int s = 0; s < 2; ++s) {
+                auto a = prefix.find(tail[s][id]);
+                if (a == prefix.end()) continue;
                 for (auto& t : a->second)
-                    if (t.first != id || U->u[id].circular) add(id, 0, t.first, t.second, ov, 10);
-            const std::string& r = rcs[id];
-            auto c = prefix.find(r.substr(r.size() - ov));
-            if (c != prefix.end())
-                for (auto& t : c->second)
-                    if (t.first != id || U->u[id].circular) add(id, 1, t.first, t.second, ov, 10);
+                    if (t.first != id || U->u[id].circular) add(id, s, t.first, t.second, ov, 10);
+            }
         }
     }
     for (uint32_t id = 0; id < n; ++id)
@@ -467,88 +664,116 @@ fbk_status compact_impl(fbk_table* t, fbk_unitigs* U) {
         }
     } B{ctx, {}};
     uint32_t* idx = (uint32_t*)B.get(cap * 4);
-    uint32_t* cnt = (uint32_t*)B.get(n * 4);
     uint8_t* visited = (uint8_t*)B.get(n);
-    if (!idx || !cnt || !visited) return set_err(ctx, FBK_ERR_OOM, "compaction index");
+    uint64_t* pre = (uint64_t*)B.get((n + 1) * 8);
+    const uint64_t tiles = (n + PRE_TILE - 1) / PRE_TILE;
+    uint64_t* part = (uint64_t*)B.get(tiles * 8);
+    uint32_t* any = (uint32_t*)B.get(4 * MAX_TABLES);
+    uint8_t* flag = (uint8_t*)B.get(n);
+    Jumps J{};
+    auto table = [&]() { return (uint32_t*)B.get(2 * n * 4); };
+    uint32_t* last = table();
+    if (!idx || !visited || !pre || !part || !any || !flag || !last) return set_err(ctx, FBK_ERR_OOM, "compaction index");
     CK(ctx, cudaMemsetAsync(idx, 0, cap * 4, ctx->stream));
     CK(ctx, cudaMemsetAsync(visited, 0, n, ctx->stream));
+    CK(ctx, cudaMemsetAsync(any, 0, 4 * MAX_TABLES, ctx->stream));
     CK(ctx, cudaMemsetAsync(ctx->d_status, 0, 4, ctx->stream));
-    TIMED(ctx, "compact_index", (k_cidx_build<NW><<<L.grid, L.block, 0, L.stream>>>(t->out_keys, n, idx, cap, ctx->d_status),
-                                 cudaGetLastError()));
-    TIMED(ctx, "compact_count", (k_walk_count<<<L.grid, L.block, 0, L.stream>>>(t->out_mask, n, cnt), cudaGetLastError()));
-    // prefix of the per-row start counts (host: one pass over n u32)
-    std::vector<uint32_t> hc(n);
-    CK(ctx, cudaMemcpyAsync(hc.data(), cnt, n * 4, cudaMemcpyDeviceToHost, ctx->stream));
-    CK(ctx, cudaStreamSynchronize(ctx->stream));
-    std::vector<uint64_t> pre(n);
-    uint64_t n_starts = 0;
-    for (uint64_t r = 0; r < n; ++r) {
-        pre[r] = n_starts;
-        n_starts += hc[r];
-    }
-    U->linear_walks = n_starts;
+    CK(ctx, cudaMemsetAsync(ctx->d_counts, 0, 8, ctx->stream));
     Rows R{t->out_keys, t->out_cov, t->out_mask, n, idx, cap};
-    std::vector<uint64_t> hlen(n_starts), hoff(n_starts);
+    TIMED(ctx, "compact_index", (k_cidx_build<NW><<<L.grid, L.block, 0, ctx->stream>>>(t->out_keys, n, idx, cap, ctx->d_status),
+                                 cudaGetLastError()));
+    TIMED(ctx, "compact_count", (k_tile_sums<<<(unsigned)tiles, 256, 0, ctx->stream>>>(StartCount{t->out_mask}, n, part), cudaGetLastError()));
+    TIMED(ctx, "compact_count", (k_tile_prefix<<<(unsigned)tiles, 256, 0, ctx->stream>>>(StartCount{t->out_mask}, n, part, pre), cudaGetLastError()));
+    TIMED(ctx, "compact_next", (k_next<NW><<<L.grid, L.block, 0, ctx->stream>>>(R, k, last), cudaGetLastError()));
+    J.t[J.n++] = last;
+    // Tables until none of their entries is left (a path of 2^l nodes needs l + 1 of them; an
+    // isolated cycle never runs out, so there are at most as many as the nodes can fill).
+    // The host looks after every four.
+    uint64_t* h = (uint64_t*)ctx->h_pinned;
+    for (bool more = true; more;) {
+        for (int q = 0; q < 4 && more; ++q) {
+            if ((1ULL << (J.n - 1)) > n) {
+                more = false;
+                break;
+            }
+            uint32_t* up = table();
+            if (!up) return set_err(ctx, FBK_ERR_OOM, "compaction tables");
+            TIMED(ctx, "compact_next", (k_double<<<L.grid, L.block, 0, ctx->stream>>>(last, up, 2 * n, any + J.n), cudaGetLastError()));
+            J.t[J.n++] = last = up;
+        }
+        if (!more) break;
+        CK(ctx, cudaMemcpyAsync(h, any + J.n - 1, 4, cudaMemcpyDeviceToHost, ctx->stream));
+        CK(ctx, cudaStreamSynchronize(ctx->stream));
+        more = *(uint32_t*)h != 0;
+    }
+    CK(ctx, cudaMemcpyAsync(h, pre + n, 8, cudaMemcpyDeviceToHost, ctx->stream));
+    CK(ctx, cudaStreamSynchronize(ctx->stream));
+    const uint64_t n_starts = h[0];
+    U->linear_walks = n_starts;
+    std::vector<uint32_t> hlen(n_starts);
+    std::vector<uint64_t> hoff(n_starts);
     std::vector<unsigned long long> hcs(n_starts);
-    std::vector<uint64_t> hpts(n_starts);
-    uint8_t* seqs = nullptr;
+    std::vector<uint8_t> hseq;
     uint64_t total = 0;
     if (n_starts) {
-        uint64_t* d_pre = (uint64_t*)B.get(n * 8);
+        const uint64_t st_tiles = (n_starts + PRE_TILE - 1) / PRE_TILE;
         uint64_t* starts = (uint64_t*)B.get(n_starts * 8);
-        uint64_t* len = (uint64_t*)B.get(n_starts * 8);
+        uint32_t* len = (uint32_t*)B.get(n_starts * 4);
+        Path* paths = (Path*)B.get(n_starts * sizeof(Path));
         unsigned long long* cs = (unsigned long long*)B.get(n_starts * 8);
-        uint64_t* pts = (uint64_t*)B.get(n_starts * 8);
-        uint64_t* off = (uint64_t*)B.get(n_starts * 8);
-        if (!d_pre || !starts || !len || !cs || !pts || !off) return set_err(ctx, FBK_ERR_OOM, "compaction walks");
-        CK(ctx, cudaMemcpyAsync(d_pre, pre.data(), n * 8, cudaMemcpyHostToDevice, ctx->stream));
-        TIMED(ctx, "compact_starts", (k_walk_starts<<<L.grid, L.block, 0, L.stream>>>(t->out_mask, n, d_pre, starts), cudaGetLastError()));
-        TIMED(ctx, "compact_walk", (k_walk_measure<NW><<<L.grid, L.block, 0, L.stream>>>(R, k, starts, n_starts, len, cs, pts,
-                                                                                          ctx->d_status),
+        uint64_t* off = (uint64_t*)B.get((n_starts + 1) * 8);
+        uint64_t* st_part = (uint64_t*)B.get(st_tiles * 8);
+        if (!starts || !len || !paths || !cs || !off || !st_part) return set_err(ctx, FBK_ERR_OOM, "compaction walks");
+        CK(ctx, cudaMemsetAsync(cs, 0, n_starts * 8, ctx->stream));
+        TIMED(ctx, "compact_starts", (k_walk_starts<<<L.grid, L.block, 0, ctx->stream>>>(t->out_mask, n, pre, starts), cudaGetLastError()));
+        TIMED(ctx, "compact_walk", (k_paths<NW><<<L.grid, L.block, 0, ctx->stream>>>(R, J, k, starts, n_starts, len, paths, ctx->d_status),
                                     cudaGetLastError()));
-        CK(ctx, cudaMemcpyAsync(hlen.data(), len, n_starts * 8, cudaMemcpyDeviceToHost, ctx->stream));
-        CK(ctx, cudaMemcpyAsync(hcs.data(), cs, n_starts * 8, cudaMemcpyDeviceToHost, ctx->stream));
-        CK(ctx, cudaMemcpyAsync(hpts.data(), pts, n_starts * 8, cudaMemcpyDeviceToHost, ctx->stream));
+        TIMED(ctx, "compact_walk", (k_tile_sums<<<(unsigned)st_tiles, 256, 0, ctx->stream>>>(PathLength{len}, n_starts, st_part), cudaGetLastError()));
+        TIMED(ctx, "compact_walk", (k_tile_prefix<<<(unsigned)st_tiles, 256, 0, ctx->stream>>>(PathLength{len}, n_starts, st_part, off),
+                                    cudaGetLastError()));
+        CK(ctx, cudaMemcpyAsync(h, off + n_starts, 8, cudaMemcpyDeviceToHost, ctx->stream));
+        CK(ctx, cudaMemcpyAsync(h + 1, ctx->d_status, 4, cudaMemcpyDeviceToHost, ctx->stream));
         CK(ctx, cudaStreamSynchronize(ctx->stream));
-        for (uint64_t s = 0; s < n_starts; ++s) {
-            hoff[s] = total;
-            total += hlen[s];
-        }
-        seqs = (uint8_t*)B.get(std::max<uint64_t>(total, 1));
+        total = h[0];
+        if ((uint32_t)h[1]) return set_err(ctx, FBK_ERR_INVALID, "compaction: node index full or a path longer than the node count");
+        uint8_t* seqs = (uint8_t*)B.get(std::max<uint64_t>(total, 1));
         if (!seqs) return set_err(ctx, FBK_ERR_OOM, "compaction sequences");
-        CK(ctx, cudaMemcpyAsync(off, hoff.data(), n_starts * 8, cudaMemcpyHostToDevice, ctx->stream));
-        TIMED(ctx, "compact_write", (k_walk_write<NW><<<L.grid, L.block, 0, L.stream>>>(R, k, starts, n_starts, len, off, seqs, visited,
-                                                                                         ctx->d_status),
-                                     cudaGetLastError()));
-        TIMED(ctx, "compact_canon", (k_canon_seq<<<L.grid, L.block, 0, L.stream>>>(seqs, off, len, n_starts), cudaGetLastError()));
+        if (total)
+            TIMED(ctx, "compact_write", (k_path_bases<NW><<<L.grid, L.block, 0, ctx->stream>>>(R, J, k, starts, n_starts, len, off, paths, total,
+                                                                                               seqs, visited, cs),
+                                         cudaGetLastError()));
+        TIMED(ctx, "compact_canon", (k_canon_seq<<<L.grid, L.block, 0, ctx->stream>>>(seqs, off, len, paths, n_starts), cudaGetLastError()));
+        hseq.resize(total);
+        CK(ctx, cudaMemcpyAsync(hlen.data(), len, n_starts * 4, cudaMemcpyDeviceToHost, ctx->stream));
+        CK(ctx, cudaMemcpyAsync(hoff.data(), off, n_starts * 8, cudaMemcpyDeviceToHost, ctx->stream));
+        CK(ctx, cudaMemcpyAsync(hcs.data(), cs, n_starts * 8, cudaMemcpyDeviceToHost, ctx->stream));
+        if (total) CK(ctx, copy_d2h(ctx, hseq.data(), seqs, total));
     }
-    uint32_t bits = 0;
-    fbk_status st = ctx_check_status(ctx, &bits);
-    if (st) return st;
-    if (bits) return set_err(ctx, FBK_ERR_INVALID, "compaction: node index full or a path longer than the node count");
-    std::vector<uint8_t> hseq(total);
-    if (total) CK(ctx, cudaMemcpyAsync(hseq.data(), seqs, total, cudaMemcpyDeviceToHost, ctx->stream));
-    // isolated cycles: candidate rows to the host
-    uint8_t* flag = (uint8_t*)B.get(n);
-    if (!flag) return set_err(ctx, FBK_ERR_OOM, "compaction cycle flags");
-    TIMED(ctx, "compact_cycles", (k_cycle_candidates<<<L.grid, L.block, 0, L.stream>>>(t->out_mask, visited, n, flag), cudaGetLastError()));
-    std::vector<uint8_t> hflag(n);
-    CK(ctx, cudaMemcpyAsync(hflag.data(), flag, n, cudaMemcpyDeviceToHost, ctx->stream));
+    // isolated cycles: candidate rows to the host, if there are any
+    TIMED(ctx, "compact_cycles", (k_cycle_candidates<<<L.grid, L.block, 0, ctx->stream>>>(t->out_mask, visited, n, flag, ctx->d_counts),
+                                  cudaGetLastError()));
+    CK(ctx, cudaMemcpyAsync(h, ctx->d_counts, 8, cudaMemcpyDeviceToHost, ctx->stream));
     CK(ctx, cudaStreamSynchronize(ctx->stream));
+    std::vector<uint8_t> hflag;
+    if (h[0]) {
+        hflag.resize(n);
+        CK(ctx, cudaMemcpyAsync(hflag.data(), flag, n, cudaMemcpyDeviceToHost, ctx->stream));
+        CK(ctx, cudaStreamSynchronize(ctx->stream));
+    }
     for (uint64_t s = 0; s < n_starts; ++s) {
         if (!hlen[s]) continue;
-        HUnitig h;
-        h.seq.assign((const char*)hseq.data() + hoff[s], hlen[s]);
-        h.cov = std::max(1.0f, (float)hcs[s] / (float)hpts[s]);
-        h.circular = false;
+        HUnitig u;
+        u.seq.assign((const char*)hseq.data() + hoff[s], hlen[s]);
+        u.cov = std::max(1.0f, (float)hcs[s] / (float)(hlen[s] - k));  // the start and the nodes: k + 1 + nodes bases
+        u.circular = false;
         U->bases += hlen[s];
-        U->u.push_back(std::move(h));
+        U->u.push_back(std::move(u));
     }
     std::vector<uint64_t> ck;
     std::vector<uint16_t> cc;
     std::vector<uint8_t> cm;
     std::vector<uint64_t> rows;
-    for (uint64_t r = 0; r < n; ++r)
+    for (uint64_t r = 0; r < hflag.size(); ++r)
         if (hflag[r]) rows.push_back(r);
     U->cycle_candidates = rows.size();
     if (!rows.empty()) {
