@@ -14,6 +14,8 @@
 // gives the registers at every checkpoint, and one thread per checkpoint sums
 // 2^-reg in register order in f64 — the exact operation sequence of
 // HyperLogLog::estimate (sketch.rs:88-96) — so the host finishes with the same bits.
+#include <algorithm>
+
 #include "fbk_device.cuh"
 #include "fbk_kernels.cuh"
 
@@ -34,7 +36,7 @@ __global__ void __launch_bounds__(256) k_est_firstpos(BankDev b, const uint64_t*
     for (uint64_t r = b.r_begin + gw; r < b.r_end; r += nwarps) {
         const uint32_t len = b.len[r];
         if (len < k) continue;
-        const uint64_t off = b.off[r], t0 = kbase[r];
+        const uint64_t off = b.off[r], t0 = kbase ? kbase[r] : off;
         // lane takes a run of consecutive windows and rolls the hash along it
         const uint32_t nk = len - k + 1, run = (nk + 31) >> 5;
         const uint32_t lo = lane * run < nk ? lane * run : nk, hi = lo + run < nk ? lo + run : nk;
@@ -60,7 +62,7 @@ __global__ void __launch_bounds__(256) k_est_hll(BankDev b, const uint64_t* __re
     for (uint64_t r = b.r_begin + gw; r < b.r_end; r += nwarps) {
         const uint32_t len = b.len[r];
         if (len < k) continue;
-        const uint64_t off = b.off[r], t0 = kbase[r];
+        const uint64_t off = b.off[r], t0 = kbase ? kbase[r] : off;
         uint32_t seg = est_segment(r >> 1);  // reads are R1,R2 interleaved per pair
         if (seg >= n_segs) seg = n_segs - 1;
         uint32_t* rt = regs_total + (uint64_t)seg * m;
@@ -74,26 +76,30 @@ __global__ void __launch_bounds__(256) k_est_hll(BankDev b, const uint64_t* __re
             for (int rr = 0; rr < 4; ++rr) solid &= __ldcg(first + cms_index(raw, rr, log2w)) < t;
             uint32_t idx, rho;
             hll_idx_rho(smix(raw), p, idx, rho);
-            // Registers only grow, so a stale read that is already >= rho is safe to skip.
-            if (*(volatile uint32_t*)&rt[idx] < rho) atomicMax(&rt[idx], rho);
-            if (solid && *(volatile uint32_t*)&rs[idx] < rho) atomicMax(&rs[idx], rho);
+            // Registers only grow, so a stale read that is already >= rho is safe to skip, and
+            // one from L1, however old, costs an atomic too many at worst.
+            if (__ldca(&rt[idx]) < rho) atomicMax(&rt[idx], rho);
+            if (solid && __ldca(&rs[idx]) < rho) atomicMax(&rs[idx], rho);
         });
     }
 }
 
-// In-place prefix max over segments, one thread per register.
-__global__ void k_est_prefix(uint32_t* regs, uint64_t m, uint32_t n_segs) {
+// In-place prefix max over the segments [s0, s1), one thread per register, on top of the
+// registers at the end of segment s0 - 1.
+__global__ void __launch_bounds__(128) k_est_prefix(uint32_t* regs_total, uint32_t* regs_solid, uint64_t m, uint32_t s0, uint32_t s1) {
+    uint32_t* regs = blockIdx.y ? regs_solid : regs_total;
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < m; i += (uint64_t)gridDim.x * blockDim.x) {
-        uint32_t v = regs[i];
-        for (uint32_t s = 1; s < n_segs; ++s) {
-            uint32_t x = regs[(uint64_t)s * m + i];
+        uint32_t v = s0 ? regs[(uint64_t)(s0 - 1) * m + i] : 0;
+#pragma unroll 8
+        for (uint32_t s = s0; s < s1; ++s) {
+            const uint32_t x = regs[(uint64_t)s * m + i];
             v = x > v ? x : v;
             regs[(uint64_t)s * m + i] = v;
         }
     }
 }
 
-// One block per (sketch, segment end): the f64 sum of 2^-reg in register order and
+// One block per (sketch, segment end of [s0, s1)): the f64 sum of 2^-reg in register order and
 // the number of zero registers (sketch.rs:88-96).  With m = 2^p registers all <= V =
 // 53 - p, every partial sum of the sequence is a multiple of 2^-V no larger than 2^p,
 // i.e. fits 53 bits: the sequential f64 sum is then exact and equals the integer sum
@@ -102,14 +108,13 @@ __global__ void k_est_prefix(uint32_t* regs, uint64_t m, uint32_t n_segs) {
 // after its index bits) is summed sequentially by one thread, in register order, with
 // 2^-v built exactly from its bits.
 __global__ void __launch_bounds__(256) k_est_sums(const uint32_t* regs_total, const uint32_t* regs_solid, uint32_t p,
-                                                  uint32_t n_segs, double* sums, unsigned long long* zeros) {
+                                                  uint32_t n_segs, uint32_t s0, double* sums, unsigned long long* zeros) {
     const uint64_t m = 1ULL << p;
     const uint32_t V = 53 - p;
     __shared__ unsigned long long s_sum[8], s_zero[8];
     __shared__ uint32_t s_big;
-    const uint32_t i = blockIdx.x;
-    if (i >= 2 * n_segs) return;
-    const uint32_t* r = (i < n_segs ? regs_total : regs_solid) + (uint64_t)(i % n_segs) * m;
+    const uint32_t seg = s0 + blockIdx.x, i = blockIdx.y * n_segs + seg;
+    const uint32_t* r = (blockIdx.y ? regs_solid : regs_total) + (uint64_t)seg * m;
     if (threadIdx.x == 0) s_big = 0;
     __syncthreads();
     unsigned long long acc = 0, z = 0;
@@ -283,13 +288,14 @@ cudaError_t launch_est_hll(const Launch& L, const BankDev& b, const uint64_t* kb
     k_est_hll<<<L.grid, L.block, 0, L.stream>>>(b, kbase, k, first, log2w, p, n_segs, regs_total, regs_solid);
     return cudaGetLastError();
 }
-cudaError_t launch_est_prefix(const Launch& L, uint32_t* regs, uint32_t p, uint32_t n_segs) {
-    k_est_prefix<<<L.grid, L.block, 0, L.stream>>>(regs, 1ULL << p, n_segs);
+cudaError_t launch_est_prefix(const Launch& L, uint32_t* regs_total, uint32_t* regs_solid, uint32_t p, uint32_t s0, uint32_t s1) {
+    const dim3 grid((unsigned)std::max<uint64_t>(1, std::min<uint64_t>((1ULL << p) / 128, L.grid)), 2);
+    k_est_prefix<<<grid, 128, 0, L.stream>>>(regs_total, regs_solid, 1ULL << p, s0, s1);
     return cudaGetLastError();
 }
 cudaError_t launch_est_sums(const Launch& L, const uint32_t* regs_total, const uint32_t* regs_solid, uint32_t p,
-                            uint32_t n_segs, double* sums, unsigned long long* zeros) {
-    k_est_sums<<<2 * n_segs, 256, 0, L.stream>>>(regs_total, regs_solid, p, n_segs, sums, zeros);
+                            uint32_t n_segs, uint32_t s0, uint32_t s1, double* sums, unsigned long long* zeros) {
+    k_est_sums<<<dim3(s1 - s0, 2), 256, 0, L.stream>>>(regs_total, regs_solid, p, n_segs, s0, sums, zeros);
     return cudaGetLastError();
 }
 cudaError_t launch_hll_add(const Launch& L, uint32_t* regs, uint32_t p, const uint64_t* hashes, uint64_t n, int mix) {

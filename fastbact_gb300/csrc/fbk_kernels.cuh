@@ -222,9 +222,9 @@ cudaError_t launch_est_firstpos(const Launch& L, const BankDev& b, const uint64_
                                 uint32_t log2w);
 cudaError_t launch_est_hll(const Launch& L, const BankDev& b, const uint64_t* kbase, uint32_t k, const uint32_t* first,
                            uint32_t log2w, uint32_t p, uint32_t n_segs, uint32_t* regs_total, uint32_t* regs_solid);
-cudaError_t launch_est_prefix(const Launch& L, uint32_t* regs, uint32_t p, uint32_t n_segs);
+cudaError_t launch_est_prefix(const Launch& L, uint32_t* regs_total, uint32_t* regs_solid, uint32_t p, uint32_t s0, uint32_t s1);
 cudaError_t launch_est_sums(const Launch& L, const uint32_t* regs_total, const uint32_t* regs_solid, uint32_t p,
-                            uint32_t n_segs, double* sums, unsigned long long* zeros);
+                            uint32_t n_segs, uint32_t s0, uint32_t s1, double* sums, unsigned long long* zeros);
 cudaError_t launch_hll_add(const Launch& L, uint32_t* regs, uint32_t p, const uint64_t* hashes, uint64_t n, int mix);
 cudaError_t launch_hll_merge(const Launch& L, uint32_t* dst, const uint32_t* src, uint64_t n);
 cudaError_t launch_subsample_mask(const Launch& L, uint64_t n_pairs, double factor, uint64_t seed, uint64_t* bits);

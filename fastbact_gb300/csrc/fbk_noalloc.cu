@@ -247,9 +247,8 @@ extern "C" FBK_API fbk_status fbk_estimate_sample_noalloc(int device, void* stre
     L.sms = sms;
     if (e == cudaSuccess) e = launch_est_firstpos(L, bv, d_kbase, k, d_first, log2w);
     if (e == cudaSuccess) e = launch_est_hll(L, bv, d_kbase, k, d_first, log2w, p, n_segs, d_rt, d_rs);
-    if (e == cudaSuccess) e = launch_est_prefix(L, d_rt, p, n_segs);
-    if (e == cudaSuccess) e = launch_est_prefix(L, d_rs, p, n_segs);
-    if (e == cudaSuccess) e = launch_est_sums(L, d_rt, d_rs, p, n_segs, d_sums, d_zeros);
+    if (e == cudaSuccess) e = launch_est_prefix(L, d_rt, d_rs, p, 0, n_segs);
+    if (e == cudaSuccess) e = launch_est_sums(L, d_rt, d_rs, p, n_segs, 0, n_segs, d_sums, d_zeros);
     double h_sums[2 * MAX_SEGS];
     unsigned long long h_zeros[2 * MAX_SEGS];
     if (e == cudaSuccess) e = cudaMemcpyAsync(h_sums, d_sums, 2ull * n_segs * 8, cudaMemcpyDeviceToHost, st);

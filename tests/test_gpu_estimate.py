@@ -1,0 +1,39 @@
+"""The estimator's sample loop where its rounds and forms can go wrong, against the oracle's
+sequential loop: registers and whole numbers, and the floats from the same operations
+(tolerance 0).
+
+The loop stops at the first checkpoint, in a later round, at no checkpoint (the sample ends
+inside a segment), or has fewer pairs than one; small sketches, whose counters are shared by
+many k-mers; every word count of k; and a sample whose reads do not lie in read order in
+its packed words."""
+import numpy as np
+import pytest
+
+from fastbact_gb300 import api
+from oracle import orc
+from test_gpu_parity import sample_reads
+
+pytestmark = pytest.mark.gpu
+
+
+def same(ctx, sample, n, stats, k, p, log2w):
+    rc, oe, ort, ors = orc.estimate_from_reads(sample_reads(sample, n), orc.count_stats(**stats.__dict__), 250000, 50.0, k=k,
+                                               cms_width=1 << log2w, hll_p=p)
+    assert rc == 0
+    ge, rt, rs = api.estimate_sample(ctx, sample, n, stats, max_pairs=250000, target_cov=50.0, k=k, hll_p=p, cms_log2_width=log2w)
+    assert np.array_equal(rt, ort) and np.array_equal(rs, ors)
+    for f in ("genome_size", "estimated_cov", "subsample_factor", "u_ge_1", "u_ge_2", "sample_kmer_depth", "pairs_sampled", "m_sample"):
+        assert getattr(ge, f) == getattr(oe, f), f
+    return ge.pairs_sampled
+
+
+@pytest.mark.parametrize("genome,cov,k,p,log2w", [
+    (20_000, 120.0, 21, 14, 23), (150_000, 30.0, 21, 14, 23), (150_000, 60.0, 31, 16, 16), (300_000, 25.0, 17, 14, 20),
+    (300_000, 25.0, 11, 12, 12), (40_000, 25.0, 33, 14, 18), (200_000, 40.0, 127, 14, 20), (100_000, 90.0, 64, 4, 14)])
+@pytest.mark.parametrize("in_order", [True, False])
+def test_sample_loop_rounds(ctx, genome, cov, k, p, log2w, in_order):
+    prm = api.synth_params(seed=genome + k, genome_len=genome, coverage=cov, gc=0.5, n_repeats=3, repeat_len=1500, sub_rate=0.005)
+    _, _, sample, n, stats = api.synth_isolate(prm, sample_pairs=150_000)
+    if not in_order:
+        sample = api.BitSeqArena(sample.data, sample.offsets[::-1].copy(), sample.lengths[::-1].copy())
+    same(ctx, sample, n, stats, k, p, log2w)
