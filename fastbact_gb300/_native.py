@@ -214,6 +214,8 @@ SIGNATURES = {
     "fbk_index_terminal_kmers": (S, [vp, u8p, u64p, C.c_uint64, C.c_uint32, C.c_uint32, u64p, u32p, u8p, u32p, C.c_uint64, u64p]),
     "fbk_ingest_fastq_device": (S, [vp, u8p, C.c_uint64, u8p, C.c_uint64, C.c_double, C.c_uint64, C.c_uint32, C.c_int, C.c_int,
                                     C.c_uint64, P(vp), P(IngestStatsC)]),
+    "fbk_ingest_fastq_fd_device": (S, [vp, C.c_int, C.c_int, C.c_double, C.c_uint64, C.c_uint32, C.c_int, C.c_int, C.c_uint64,
+                                       P(vp), P(IngestStatsC)]),
     "fbk_bank_export": (S, [vp, u64p, u64p, u32p, u32p]),
     "fbk_bank_arena_counts": (S, [vp, u64p]),
     "fbk_bank_words": (S, [vp, u64p]),

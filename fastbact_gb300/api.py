@@ -19,6 +19,8 @@ buffers and parameters across the C ABI.
 from __future__ import annotations
 
 import ctypes as C
+import os
+import stat
 import weakref
 from dataclasses import dataclass, field
 
@@ -847,13 +849,17 @@ def ingest_fastq_device(ctx: Context, r1: str, r2: str, subsample_factor: float 
                         enable_trim: bool = True, enable_merge: bool = True, seed: int = 0):
     """ingest_reads_ext_with_seed (trim_merge.rs:307-417) on the device: reads the two
     files, uploads their bytes and returns (DeviceBank, IngestStats, merged_bases)."""
-    a = np.fromfile(str(r1), dtype=np.uint8)
-    b = np.fromfile(str(r2), dtype=np.uint8)
     h = C.c_void_p()
     st = N.IngestStatsC()
-    check(N.lib().fbk_ingest_fastq_device(ctx.handle, ptr(a) if a.size else None, a.size, ptr(b) if b.size else None, b.size,
-                                          subsample_factor, min_len, min_qual, int(enable_trim), int(enable_merge), seed,
-                                          C.byref(h), C.byref(st)), ctx.handle, "device ingest")
+    args = (subsample_factor, min_len, min_qual, int(enable_trim), int(enable_merge), seed, C.byref(h), C.byref(st))
+    with open(str(r1), "rb") as f1, open(str(r2), "rb") as f2:
+        if all(stat.S_ISREG(os.fstat(f.fileno()).st_mode) for f in (f1, f2)):
+            rc = N.lib().fbk_ingest_fastq_fd_device(ctx.handle, f1.fileno(), f2.fileno(), *args)
+        else:
+            a, b = (np.fromfile(f, dtype=np.uint8) for f in (f1, f2))
+            rc = N.lib().fbk_ingest_fastq_device(ctx.handle, ptr(a) if a.size else None, a.size, ptr(b) if b.size else None,
+                                                 b.size, *args)
+    check(rc, ctx.handle, "device ingest")
     stats = IngestStats(st.input_read_pairs, st.retained_read_pairs, st.merged_pairs_count, st.unmerged_pairs_count,
                         st.bases_before_trim, st.bases_after_trim)
     return DeviceBank.from_handle(ctx, h), stats, st.merged_bases

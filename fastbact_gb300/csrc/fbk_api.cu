@@ -1,6 +1,7 @@
 // fbk_api.cu — host side of the C ABI: contexts, device pool, bank upload, and the
 // CountMinSketch / HyperLogLog / solid-table objects with their build passes.
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -507,28 +508,56 @@ static cudaError_t stage_ready(fbk_ctx* ctx) {
     return e;
 }
 
-static void pool_copy(void* dst, const void* src, size_t n) {
+template <class Fn>
+static void pool_pieces(size_t n, Fn&& piece) {
     host_parallel_for((n + STAGE_PIECE - 1) / STAGE_PIECE, [&](uint64_t i, unsigned) {
         const size_t o = i * STAGE_PIECE;
-        std::memcpy((char*)dst + o, (const char*)src + o, std::min(STAGE_PIECE, n - o));
+        piece(o, std::min(STAGE_PIECE, n - o));
     });
 }
+static void pool_copy(void* dst, const void* src, size_t n) {
+    pool_pieces(n, [&](size_t o, size_t m) { std::memcpy((char*)dst + o, (const char*)src + o, m); });
+}
 
-cudaError_t copy_h2d(fbk_ctx* ctx, void* dst, const void* src, size_t bytes) {
-    if (bytes == 0) return cudaSuccess;
-    if (bytes < STAGE_MIN || host_page_locked(src))
-        return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, ctx->stream);
+// fill(slot, first byte, bytes): the next bytes of the source in a staging slot
+template <class Fn>
+static cudaError_t staged_h2d(fbk_ctx* ctx, void* dst, size_t bytes, Fn&& fill) {
     cudaError_t e = stage_ready(ctx);
     for (size_t done = 0; e == cudaSuccess && done < bytes;) {
         const int slot = (int)((done / STAGE_BYTES) & 1);
         const size_t n = std::min(STAGE_BYTES, bytes - done);
         e = cudaEventSynchronize(ctx->stage_ev[slot]);  // the slot's previous DMA has finished
         if (e != cudaSuccess) break;
-        pool_copy(ctx->h_stage[slot], (const char*)src + done, n);
+        fill(ctx->h_stage[slot], done, n);
         e = cudaMemcpyAsync((char*)dst + done, ctx->h_stage[slot], n, cudaMemcpyHostToDevice, ctx->stream);
         if (e == cudaSuccess) e = cudaEventRecord(ctx->stage_ev[slot], ctx->stream);
         done += n;
     }
+    return e;
+}
+
+cudaError_t copy_h2d(fbk_ctx* ctx, void* dst, const void* src, size_t bytes) {
+    if (bytes == 0) return cudaSuccess;
+    if (bytes < STAGE_MIN || host_page_locked(src))
+        return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, ctx->stream);
+    return staged_h2d(ctx, dst, bytes, [&](void* slot, size_t o, size_t n) { pool_copy(slot, (const char*)src + o, n); });
+}
+
+cudaError_t copy_h2d_from(fbk_ctx* ctx, void* dst, size_t bytes, const std::function<bool(void*, size_t, size_t)>& read, bool* ok) {
+    *ok = true;
+    if (bytes == 0) return cudaSuccess;
+    if (bytes < STAGE_MIN) {
+        std::vector<char> all(bytes);
+        *ok = read(all.data(), 0, bytes);
+        return *ok ? cudaMemcpyAsync(dst, all.data(), bytes, cudaMemcpyHostToDevice, ctx->stream) : cudaSuccess;
+    }
+    std::atomic<bool> good{true};
+    const cudaError_t e = staged_h2d(ctx, dst, bytes, [&](void* slot, size_t o, size_t n) {
+        pool_pieces(n, [&](size_t p, size_t m) {
+            if (good && !read((char*)slot + p, o + p, m)) good = false;
+        });
+    });
+    *ok = good;
     return e;
 }
 

@@ -3,6 +3,7 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <functional>
 #include <map>
 #include <memory>
 #include <mutex>
@@ -220,6 +221,9 @@ void scan_arenas(const fbk_arena_view* arenas, int n_arenas, ArenaScan& sc);
 // runs far below the copy engines' rate).  copy_h2d returns with the last DMA in
 // flight (src may be reused at once); copy_d2h returns when dst holds the data.
 cudaError_t copy_h2d(fbk_ctx* ctx, void* dst, const void* src, size_t bytes);
+// The same from a source that read(dst, first byte, bytes) copies out, in several threads at
+// once; ok is cleared if one of the reads fails.
+cudaError_t copy_h2d_from(fbk_ctx* ctx, void* dst, size_t bytes, const std::function<bool(void*, size_t, size_t)>& read, bool* ok);
 cudaError_t copy_d2h(fbk_ctx* ctx, void* dst, const void* src, size_t bytes);
 
 // Upload of a packed arena set into a device bank (used by the estimator for its

@@ -596,6 +596,11 @@ typedef struct {
 FBK_API fbk_status fbk_ingest_fastq_device(fbk_ctx* ctx, const uint8_t* r1, uint64_t r1_len, const uint8_t* r2, uint64_t r2_len,
                                            double subsample_factor, uint64_t min_len, uint32_t min_qual, int enable_trim,
                                            int enable_merge, uint64_t seed, fbk_bank** out, fbk_ingest_stats* stats);
+/* The same from two open regular files, read from their start in pieces by several threads
+ * (FBK_ERR_IO if one cannot be read or is no regular file).  Their file positions stay. */
+FBK_API fbk_status fbk_ingest_fastq_fd_device(fbk_ctx* ctx, int fd1, int fd2, double subsample_factor, uint64_t min_len,
+                                              uint32_t min_qual, int enable_trim, int enable_merge, uint64_t seed, fbk_bank** out,
+                                              fbk_ingest_stats* stats);
 /* A device bank back on the host: words (fbk_bank_words of them), bank-global base offsets, lengths, pair indices (n_reads each; any pointer may be NULL). */
 FBK_API fbk_status fbk_bank_export(const fbk_bank* b, uint64_t* words, uint64_t* offsets, uint32_t* lengths, uint32_t* pair_idx);
 /* Reads per arena (merged, pe_forward, pe_reverse) and words of a bank. */
