@@ -807,7 +807,7 @@ def filter_active_reads(ctx: Context, bank, seqs: list, circular, edges, graph_k
     circular and edges are compact()'s unitigs."""
     dbank = bank if isinstance(bank, DeviceBank) else DeviceBank(ctx, bank)
     n = len(seqs)
-    useq = np.frombuffer(b"".join(seqs), np.uint8).copy() if n else np.zeros(1, np.uint8)
+    useq = np.frombuffer(b"".join(seqs), np.uint8) if n else np.zeros(1, np.uint8)
     uoff = np.zeros(n + 1, np.uint64)
     if n:
         uoff[1:] = np.cumsum([len(x) for x in seqs])
@@ -830,7 +830,7 @@ def index_terminal_kmers(ctx: Context, seqs: list, k: int, key_bits: int | None 
     k-mers (folded to u64) of the unitigs with (unitig, is_rc, position), sorted by key."""
     key_bits = key_bits or key_bits_for_k(k)
     n = len(seqs)
-    useq = np.frombuffer(b"".join(seqs), np.uint8).copy() if n else np.zeros(1, np.uint8)
+    useq = np.frombuffer(b"".join(seqs), np.uint8) if n else np.zeros(1, np.uint8)
     uoff = np.zeros(n + 1, np.uint64)
     if n:
         uoff[1:] = np.cumsum([len(x) for x in seqs])

@@ -6,10 +6,10 @@
 // k'-mer of short (< 2000 bp), circular or branching unitigs and of the first and
 // last 350 k'-mers of the other unitigs, then keeps a read when the ntHash at offset
 // 0, (len - k') / 2 or len - k' is indexed; a pair is kept when either read is.
-// Here the index is an open-addressing set of u64 hashes built on the device from the
-// packed unitigs, and one thread tests each read of the device bank.
+// Here the unitigs are packed on the device, the index is an open-addressing set of u64
+// hashes that the windows of the packed unitigs are entered into, and one thread tests a
+// merged read or a pair of the device bank and writes its keep bytes.
 #include <algorithm>
-#include <cstring>
 #include <vector>
 
 #include "fbk_device.cuh"
@@ -21,19 +21,78 @@ namespace {
 
 constexpr uint64_t HSET_EMPTY = ~0ULL;
 
-__global__ void k_hset_insert(const uint64_t* __restrict__ data, const uint64_t* __restrict__ win, uint64_t n_win, uint32_t k,
-                              unsigned long long* set, uint64_t cap, uint32_t* flags) {
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n_win; i += (uint64_t)gridDim.x * blockDim.x) {
-        const uint64_t h = nthash_canonical_at(data, win[i], k);
-        if (h == HSET_EMPTY) {  // the one value the set cannot hold is kept as a flag
-            atomicOr(flags, 1u);
-            continue;
+// ASCII to packed words (ASCII_TO_2BIT: A0 C1 G2 T3, anything else 0), one word a thread; words
+// past the bases are zero.
+__global__ void __launch_bounds__(256) k_pack_ascii(const uint8_t* __restrict__ t, uint64_t n, uint64_t* __restrict__ words, uint64_t n_words) {
+    const uint64_t w = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (w >= n_words) return;
+    uint64_t x = 0;
+    for (uint32_t j = 0; j < 32 && w * 32 + j < n; ++j) {
+        const uint8_t c = t[w * 32 + j] & 0xDF;
+        x |= (uint64_t)(c == 'C' ? 1 : c == 'G' ? 2 : c == 'T' ? 3 : 0) << (2 * j);
+    }
+    words[w] = x;
+}
+
+constexpr uint64_t FILTER_WINDOW = 350, FILTER_LONG = 2000;
+// The indexed windows of a unitig of len bases: [0, left) and [right, len - k + 1).
+struct FilterSpan {
+    uint64_t left, right, n;
+};
+__host__ __device__ __forceinline__ FilterSpan filter_span(uint64_t len, uint32_t k, bool circular, uint32_t fwd, uint32_t rev) {
+    FilterSpan f{0, 0, 0};
+    if (len < k) return f;
+    const uint64_t nk = len - k + 1;
+    f.n = nk;
+    if (len < FILTER_LONG || circular || fwd > 1 || rev > 1) return f;
+    f.left = nk < FILTER_WINDOW ? nk : FILTER_WINDOW;
+    f.right = len - FILTER_WINDOW < len - k ? len - FILTER_WINDOW : len - k;
+    return f;
+}
+
+// A thread takes FILTER_RUN places of the packed unitigs, finds the unitig of the first one by
+// bisection and rolls the hash along the windows there that are indexed.  Bound by the set's
+// CAS (random 8-byte accesses in L2).  The host packed base by base and listed the windows
+// (8 bytes each, copied over) before: the whole call took 6.5 ms for a 1 Mbp graph at 50x and
+// takes 0.39.
+constexpr uint32_t FILTER_RUN = 8;
+__global__ void __launch_bounds__(256) k_hset_insert(const uint64_t* __restrict__ data, uint64_t n_bases, const uint64_t* __restrict__ uoff,
+                                                     const uint8_t* __restrict__ circular, const uint32_t* __restrict__ fwd,
+                                                     const uint32_t* __restrict__ rev, uint64_t n_unitigs, uint32_t k,
+                                                     unsigned long long* set, uint64_t cap, uint32_t* flags) {
+    for (uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; t * FILTER_RUN < n_bases; t += (uint64_t)gridDim.x * blockDim.x) {
+        uint64_t g = t * FILTER_RUN;
+        const uint64_t end = min(g + FILTER_RUN, n_bases);
+        uint64_t lo = 0, hi = n_unitigs;  // the last unitig that begins at g or before
+        while (hi - lo > 1) {
+            const uint64_t mid = (lo + hi) / 2;
+            if (uoff[mid] - uoff[0] <= g) lo = mid;
+            else hi = mid;
         }
-        uint64_t s = smix(h) & (cap - 1);
-        for (uint64_t probe = 0; probe < cap; ++probe) {
-            const unsigned long long old = atomicCAS(&set[s], HSET_EMPTY, (unsigned long long)h);
-            if (old == HSET_EMPTY || old == h) break;
-            s = (s + 1) & (cap - 1);
+        for (uint64_t u = lo; u < n_unitigs && g < end; ++u) {
+            const uint64_t a = uoff[u] - uoff[0], e = uoff[u + 1] - uoff[0];
+            const FilterSpan f = filter_span(e - a, k, circular[u], fwd[u], rev[u]);
+            const uint64_t stop = min(end, e);
+            auto enter = [&](uint64_t from, uint64_t to) {  // windows of the unitig
+                from = max(from, g - a);
+                to = min(to, stop - a);
+                if (from >= to) return;
+                nthash_run(data, a + from, k, 0, (uint32_t)(to - from), [&](uint32_t, uint64_t h) {
+                    if (h == HSET_EMPTY) {  // the one value the set cannot hold is kept as a flag
+                        atomicOr(flags, 1u);
+                        return;
+                    }
+                    uint64_t s = smix(h) & (cap - 1);
+                    for (uint64_t probe = 0; probe < cap; ++probe) {
+                        const unsigned long long old = atomicCAS(&set[s], HSET_EMPTY, (unsigned long long)h);
+                        if (old == HSET_EMPTY || old == h) break;
+                        s = (s + 1) & (cap - 1);
+                    }
+                });
+            };
+            enter(0, f.left);
+            enter(max(f.left, f.right), f.n);
+            g = max(g, stop);
         }
     }
 }
@@ -51,19 +110,66 @@ __device__ __forceinline__ bool hset_has(const unsigned long long* set, uint64_t
 }
 
 // local_multik.rs:296-307: ntHash at offsets 0, (len - k) / 2 and len - k.
-__global__ void k_active_reads(BankDev b, uint32_t k, const unsigned long long* __restrict__ set, uint64_t cap,
-                               const uint32_t* __restrict__ flags, uint8_t* active) {
-    const uint32_t fl = *flags;
-    for (uint64_t r = b.r_begin + (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; r < b.r_end; r += (uint64_t)gridDim.x * blockDim.x) {
-        const uint32_t len = b.len[r];
-        bool a = false;
-        if (len >= k) {
-            const uint64_t off = b.off[r];
-            const uint32_t offs[3] = {0u, (len - k) / 2, len - k};
-            for (int j = 0; j < 3 && !a; ++j) a = hset_has(set, cap, fl, nthash_canonical_at(b.data, off + offs[j], k));
-        }
-        active[r] = a ? 1 : 0;
+__device__ __forceinline__ bool read_active(const BankDev& b, uint64_t r, uint32_t k, const unsigned long long* set, uint64_t cap, uint32_t fl) {
+    const uint32_t len = b.len[r];
+    bool a = false;
+    if (len >= k) {
+        const uint64_t off = b.off[r];
+        const uint32_t offs[3] = {0u, (len - k) / 2, len - k};
+        for (int j = 0; j < 3 && !a; ++j) a = hset_has(set, cap, fl, nthash_canonical_at(b.data, off + offs[j], k));
     }
+    return a;
+}
+// local_multik.rs:309-329: merged reads (M) on their own, the pairs of the other two arenas (F
+// and R reads) together; a read without a mate is not kept.
+__global__ void __launch_bounds__(256) k_active_reads(BankDev b, uint64_t M, uint64_t F, uint64_t R, uint32_t k,
+                                                      const unsigned long long* __restrict__ set, uint64_t cap,
+                                                      const uint32_t* __restrict__ flags, uint8_t* __restrict__ keep,
+                                                      unsigned long long* __restrict__ n_kept) {
+    const uint32_t fl = *flags;
+    uint32_t kept = 0;
+    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < M + max(F, R); i += (uint64_t)gridDim.x * blockDim.x) {
+        if (i < M) {
+            kept += keep[i] = read_active(b, i, k, set, cap, fl);
+            continue;
+        }
+        const uint64_t j = i - M;
+        const bool a = j < min(F, R) && (read_active(b, i, k, set, cap, fl) || read_active(b, i + F, k, set, cap, fl));
+        if (j < F) keep[i] = a;
+        if (j < R) keep[i + F] = a;
+        kept += 2 * a;
+    }
+    kept = __reduce_add_sync(0xffffffffu, kept);
+    if ((threadIdx.x & 31) == 0 && kept) atomicAdd(n_kept, (unsigned long long)kept);
+}
+
+struct Bufs {
+    fbk_ctx* c;
+    std::vector<void*> p;
+    void* get(uint64_t b) {
+        void* q = dev_alloc(c, std::max<uint64_t>(b, 8));
+        if (q) p.push_back(q);
+        return q;
+    }
+    ~Bufs() {
+        cudaStreamSynchronize(c->stream);
+        for (void* q : p) dev_free(c, q);
+    }
+};
+
+// The bases of the unitigs back to back in packed words on the device (8 words of zeros after
+// them).
+fbk_status pack_unitigs(fbk_ctx* ctx, Bufs& B, const uint8_t* ascii, const uint64_t* offsets, uint64_t n_unitigs, uint64_t** words) {
+    for (uint64_t u = 0; u < n_unitigs; ++u)
+        if (offsets[u + 1] < offsets[u]) return set_err(ctx, FBK_ERR_INVALID, "unitig offsets must not fall");
+    const uint64_t n = n_unitigs ? offsets[n_unitigs] - offsets[0] : 0, n_words = (n + 31) / 32 + 8;
+    uint8_t* text = (uint8_t*)B.get(n);
+    *words = (uint64_t*)B.get(n_words * 8);
+    if (!text || !*words) return set_err(ctx, FBK_ERR_OOM, "packed unitigs");
+    if (n) CK(ctx, copy_h2d(ctx, text, ascii + offsets[0], n));
+    TIMED(ctx, "unitig_pack", (k_pack_ascii<<<(unsigned)((n_words + 255) / 256), 256, 0, ctx->stream>>>(text, n, *words, n_words),
+                               cudaGetLastError()));
+    return FBK_OK;
 }
 
 }  // namespace
@@ -81,80 +187,48 @@ FBK_API fbk_status fbk_filter_active_reads(fbk_ctx* ctx, const fbk_bank* bank, c
     CK(ctx, cudaSetDevice(ctx->device));
     CK(ctx, bank_wait(ctx, bank));
     const uint32_t k = std::min<uint32_t>(graph_k, 31);
-    const uint64_t WINDOW = 350;
-    // pack the unitigs (ASCII_TO_2BIT: A0 C1 G2 T3, anything else 0) and list the windows
-    std::vector<uint64_t> words(8, 0), win;
-    uint64_t pos = 0;
-    auto push_base = [&](uint8_t c) {
-        const uint64_t code = c == 'C' || c == 'c' ? 1 : c == 'G' || c == 'g' ? 2 : c == 'T' || c == 't' ? 3 : 0;
-        if ((pos >> 5) + 8 >= words.size()) words.resize(words.size() * 2 + 16, 0);
-        words[pos >> 5] |= code << ((pos & 31) * 2);
-        ++pos;
-    };
+    const uint64_t M = bank->arena_reads[0], F = bank->arena_reads[1], R = bank->arena_reads[2], n_reads = M + F + R;
+    Bufs B{ctx, {}};
+    uint64_t* d_words = nullptr;
+    fbk_status st = pack_unitigs(ctx, B, unitig_ascii, unitig_offsets, n_unitigs, &d_words);
+    if (st) return st;
+    uint64_t n_win = 0;
     for (uint64_t u = 0; u < n_unitigs; ++u) {
-        const uint64_t a = unitig_offsets[u], e = unitig_offsets[u + 1], len = e - a;
-        const uint64_t base = pos;
-        for (uint64_t i = a; i < e; ++i) push_base(unitig_ascii[i]);
-        if (len < k) continue;
-        const uint64_t nk = len - k + 1;
-        if (len < 2000 || circular[u] || edges_fwd[u] > 1 || edges_rev[u] > 1) {
-            for (uint64_t i = 0; i < nk; ++i) win.push_back(base + i);
-        } else {
-            const uint64_t left = std::min<uint64_t>(WINDOW, nk);
-            for (uint64_t i = 0; i < left; ++i) win.push_back(base + i);
-            const uint64_t right = std::min<uint64_t>(len > WINDOW ? len - WINDOW : 0, len - k);
-            for (uint64_t i = right; i < nk; ++i) win.push_back(base + i);
-        }
+        const FilterSpan f = filter_span(unitig_offsets[u + 1] - unitig_offsets[u], k, circular[u], edges_fwd[u], edges_rev[u]);
+        n_win += f.left + f.n - std::max(f.left, f.right);
     }
-    const uint64_t n_words = (pos + 31) / 32 + 8;
     uint64_t cap = 1024;
-    while (cap < 2 * win.size()) cap <<= 1;
-    struct Bufs {
-        fbk_ctx* c;
-        std::vector<void*> p;
-        void* get(uint64_t b) {
-            void* q = dev_alloc(c, b);
-            if (q) p.push_back(q);
-            return q;
-        }
-        ~Bufs() {
-            cudaStreamSynchronize(c->stream);
-            for (void* q : p) dev_free(c, q);
-        }
-    } B{ctx, {}};
-    uint64_t* d_words = (uint64_t*)B.get(n_words * 8);
-    uint64_t* d_win = (uint64_t*)B.get(std::max<uint64_t>(win.size(), 1) * 8);
+    while (cap < 2 * n_win) cap <<= 1;
+    uint64_t* d_off = (uint64_t*)B.get((n_unitigs + 1) * 8);
+    uint8_t* d_circ = (uint8_t*)B.get(n_unitigs);
+    uint32_t* d_fwd = (uint32_t*)B.get(n_unitigs * 4);
+    uint32_t* d_rev = (uint32_t*)B.get(n_unitigs * 4);
     unsigned long long* set = (unsigned long long*)B.get(cap * 8);
-    uint32_t* flags = (uint32_t*)B.get(256);
-    uint8_t* active = (uint8_t*)B.get(std::max<uint64_t>(bank->n_reads, 1));
-    if (!d_words || !d_win || !set || !flags || !active) return set_err(ctx, FBK_ERR_OOM, "filter_active_reads buffers");
-    words.resize(n_words, 0);
-    CK(ctx, cudaMemcpyAsync(d_words, words.data(), n_words * 8, cudaMemcpyHostToDevice, ctx->stream));
-    if (!win.empty()) CK(ctx, cudaMemcpyAsync(d_win, win.data(), win.size() * 8, cudaMemcpyHostToDevice, ctx->stream));
-    CK(ctx, cudaMemsetAsync(set, 0xFF, cap * 8, ctx->stream));
-    CK(ctx, cudaMemsetAsync(flags, 0, 4, ctx->stream));
+    unsigned long long* d_kept = (unsigned long long*)B.get(16);
+    uint8_t* keep = (uint8_t*)B.get(n_reads);
+    if (!d_off || !d_circ || !d_fwd || !d_rev || !set || !d_kept || !keep) return set_err(ctx, FBK_ERR_OOM, "filter_active_reads buffers");
+    uint32_t* flags = (uint32_t*)(d_kept + 1);
+    CK(ctx, cudaMemsetAsync(d_kept, 0, 16, ctx->stream));
     Launch L = launch_cfg(ctx, 256, 0);
-    if (!win.empty())
-        TIMED(ctx, "filter_index", (k_hset_insert<<<L.grid, L.block, 0, L.stream>>>(d_words, d_win, win.size(), k, set, cap, flags),
+    CK(ctx, cudaMemsetAsync(set, 0xFF, cap * 8, ctx->stream));
+    if (n_win) {
+        CK(ctx, copy_h2d(ctx, d_off, unitig_offsets, (n_unitigs + 1) * 8));
+        CK(ctx, copy_h2d(ctx, d_circ, circular, n_unitigs));
+        CK(ctx, copy_h2d(ctx, d_fwd, edges_fwd, n_unitigs * 4));
+        CK(ctx, copy_h2d(ctx, d_rev, edges_rev, n_unitigs * 4));
+        TIMED(ctx, "filter_index", (k_hset_insert<<<L.grid, L.block, 0, L.stream>>>(d_words, unitig_offsets[n_unitigs] - unitig_offsets[0],
+                                                                                   d_off, d_circ, d_fwd, d_rev, n_unitigs, k, set, cap, flags),
                                     cudaGetLastError()));
-    if (bank->n_reads)
-        TIMED(ctx, "filter_reads", (k_active_reads<<<L.grid, L.block, 0, L.stream>>>(bank_view(bank, 0, bank->n_reads, nullptr), k, set,
-                                                                                    cap, flags, active),
-                                    cudaGetLastError()));
-    std::vector<uint8_t> act(bank->n_reads);
-    if (bank->n_reads) CK(ctx, cudaMemcpyAsync(act.data(), active, bank->n_reads, cudaMemcpyDeviceToHost, ctx->stream));
-    CK(ctx, cudaStreamSynchronize(ctx->stream));
-    // local_multik.rs:309-329: merged reads on their own, pairs together
-    const uint64_t M = bank->arena_reads[0], F = bank->arena_reads[1], R = bank->arena_reads[2];
+    }
     uint64_t kept = 0;
-    for (uint64_t i = 0; i < M; ++i) kept += keep_out[i] = act[i];
-    const uint64_t pe = std::min(F, R);
-    for (uint64_t i = 0; i < F; ++i) keep_out[M + i] = 0;
-    for (uint64_t i = 0; i < R; ++i) keep_out[M + F + i] = 0;
-    for (uint64_t i = 0; i < pe; ++i) {
-        const uint8_t kp = act[M + i] | act[M + F + i];
-        keep_out[M + i] = keep_out[M + F + i] = kp;
-        kept += 2 * kp;
+    if (n_reads) {
+        TIMED(ctx, "filter_reads", (k_active_reads<<<L.grid, L.block, 0, L.stream>>>(bank_view(bank, 0, bank->n_reads, nullptr), M, F, R, k,
+                                                                                    set, cap, flags, keep, d_kept),
+                                    cudaGetLastError()));
+        CK(ctx, cudaMemcpyAsync(ctx->h_pinned, d_kept, 8, cudaMemcpyDeviceToHost, ctx->stream));
+        CK(ctx, copy_d2h(ctx, keep_out, keep, n_reads));
+        CK(ctx, cudaStreamSynchronize(ctx->stream));
+        kept = *(const unsigned long long*)ctx->h_pinned;
     }
     if (n_kept) *n_kept = kept;
     return FBK_OK;
@@ -216,18 +290,13 @@ FBK_API fbk_status fbk_index_terminal_kmers(fbk_ctx* ctx, const uint8_t* unitig_
     const int nw = key_bits == 64 ? 1 : key_bits == 128 ? 2 : key_bits == 256 ? 4 : 0;
     if (!nw || k < 1 || k > (uint32_t)(32 * nw - 1)) return set_err(ctx, FBK_ERR_INVALID, "k out of range for key_bits");
     CK(ctx, cudaSetDevice(ctx->device));
-    std::vector<uint64_t> words(8, 0);
+    Bufs B{ctx, {}};
+    uint64_t* d_words = nullptr;
+    fbk_status st = pack_unitigs(ctx, B, unitig_ascii, unitig_offsets, n_unitigs, &d_words);
+    if (st) return st;
     std::vector<TermWindow> win;
-    uint64_t pos = 0;
     for (uint64_t u = 0; u < n_unitigs; ++u) {
-        const uint64_t a = unitig_offsets[u], e = unitig_offsets[u + 1], len = e - a, base = pos;
-        for (uint64_t i = a; i < e; ++i) {
-            const uint8_t c = unitig_ascii[i];
-            const uint64_t code = c == 'C' || c == 'c' ? 1 : c == 'G' || c == 'g' ? 2 : c == 'T' || c == 't' ? 3 : 0;
-            if ((pos >> 5) + 8 >= words.size()) words.resize(words.size() * 2 + 16, 0);
-            words[pos >> 5] |= code << ((pos & 31) * 2);
-            ++pos;
-        }
+        const uint64_t base = unitig_offsets[u] - unitig_offsets[0], len = unitig_offsets[u + 1] - unitig_offsets[u];
         if (len < k) continue;
         const uint64_t total = len - k + 1;
         if (total <= 2000) {
@@ -237,31 +306,14 @@ FBK_API fbk_status fbk_index_terminal_kmers(fbk_ctx* ctx, const uint8_t* unitig_
             for (uint64_t i = total - 1000; i < total; ++i) win.push_back({base + i, (uint32_t)u, (uint32_t)i});
         }
     }
-    const uint64_t n_words = (pos + 31) / 32 + 8;
-    words.resize(n_words, 0);
     uint64_t cap = 1024;
     while (cap < 2 * win.size()) cap <<= 1;
-    struct Bufs {
-        fbk_ctx* c;
-        std::vector<void*> p;
-        void* get(uint64_t b) {
-            void* q = dev_alloc(c, b);
-            if (q) p.push_back(q);
-            return q;
-        }
-        ~Bufs() {
-            cudaStreamSynchronize(c->stream);
-            for (void* q : p) dev_free(c, q);
-        }
-    } B{ctx, {}};
-    uint64_t* d_words = (uint64_t*)B.get(n_words * 8);
     TermWindow* d_win = (TermWindow*)B.get(std::max<uint64_t>(win.size(), 1) * sizeof(TermWindow));
     unsigned long long* keys = (unsigned long long*)B.get(cap * 8);
     uint32_t* cnt = (uint32_t*)B.get(cap * 4);
     uint64_t* vals = (uint64_t*)B.get(cap * 8);
     unsigned long long* ff = (unsigned long long*)B.get(64);
-    if (!d_words || !d_win || !keys || !cnt || !vals || !ff) return set_err(ctx, FBK_ERR_OOM, "terminal k-mer index buffers");
-    CK(ctx, cudaMemcpyAsync(d_words, words.data(), n_words * 8, cudaMemcpyHostToDevice, ctx->stream));
+    if (!d_win || !keys || !cnt || !vals || !ff) return set_err(ctx, FBK_ERR_OOM, "terminal k-mer index buffers");
     if (!win.empty()) CK(ctx, cudaMemcpyAsync(d_win, win.data(), win.size() * sizeof(TermWindow), cudaMemcpyHostToDevice, ctx->stream));
     CK(ctx, cudaMemsetAsync(keys, 0xFF, cap * 8, ctx->stream));
     CK(ctx, cudaMemsetAsync(cnt, 0, cap * 4, ctx->stream));
