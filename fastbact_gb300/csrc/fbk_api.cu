@@ -1684,7 +1684,7 @@ static fbk_status build_front_ladder(fbk_ctx* ctx, const fbk_bank* b, const fbk_
         if (st == FBK_OK) st = bins_build(ctx, b, p, kb, log2w, out, &declined);
         cudaStreamSynchronize(ctx->stream);
         dev_free(ctx, kb);
-        if (st || !declined) return st;
+        if (st != FBK_ERR_OOM && (st || !declined)) return st;  // short of memory: the buckets may need less
     }
     Ladder lad;
     lad.log2w = log2w;

@@ -331,6 +331,10 @@ __device__ __forceinline__ uint64_t fold_of(const uint64_t (&w)[NK]) {
 // warp needed; groups handed out (aggregate, sample).
 enum { BC_ROWS, BC_LOW, BC_SINGLES, BC_PAIRS, BC_DISTINCT, BC_MULTI, BC_KEPT, BC_WINDOWS, BC_NEED, BC_WORK, BC_WORK_S, BC_N };
 
+struct FirstKey {
+    uint64_t raw;        // canonical ntHash
+    uint32_t at, again;  // the first two places in the bank (0xFFFFFFFF: none)
+};
 struct AggArgs {
     const uint64_t* data;
     const uint64_t* runs;
@@ -351,7 +355,14 @@ struct AggArgs {
     uint32_t later_cap;
     unsigned long long* counters;
     uint32_t* status;
+    FirstKey* firsts;            // AGG_FIRST: the keys (cap_rows of them)
+    uint32_t* first;             // and the estimator's first touches, 4 rows of 2^log2w
+    uint32_t log2w;
 };
+
+// What a launch of k_bin_agg is for: the accumulator rows; the same counts of a part of the
+// bins, for the sizes; or the first two places of every key (the estimator's).
+enum { AGG_BUILD, AGG_SAMPLE, AGG_FIRST };
 
 constexpr int AGG_THREADS = 512;
 constexpr uint32_t AGG_SMEM = 113000;  // two blocks an SM (228 KB, 1 KB reserved a block)
@@ -359,6 +370,7 @@ constexpr uint32_t AGG_NARROW_MAX = 65535;  // windows of a group whose u16 coun
 constexpr uint32_t AGG_QUEUE = 64 * 8;      // bytes of a warp's queue
 constexpr uint32_t AGG_LATER = 16384;       // windows a block can put off, at most
 constexpr uint32_t AGG_TURNS = 1u << 16;    // a turn is repeated only when another lane has entered a key
+constexpr uint32_t NO_PLACE = 0xFFFFFFFFu;  // AGG_FIRST; the bank holds fewer than 2^32 - 1 bases
 constexpr uint32_t POS_TWICE = 0xFFFFFFFFu; // place + 1 of the key's first window otherwise, 0: no key
 
 // A group's keys in shared memory: entries, filled one after another, of NK key words, the
@@ -368,6 +380,11 @@ constexpr uint32_t POS_TWICE = 0xFFFFFFFFu; // place + 1 of the key's first wind
 // entries can be read without gaps.
 __host__ __device__ constexpr uint32_t agg_entries(int nk, bool wide) {
     return (AGG_SMEM - AGG_QUEUE * (AGG_THREADS / 32)) / (8u * nk + (wide ? 36u : 20u) + 8u) & ~127u;
+}
+
+// AGG_FIRST: the key words, its two places and the two slots.
+__host__ __device__ constexpr uint32_t first_entries(int nk) {
+    return (AGG_SMEM - AGG_QUEUE * (AGG_THREADS / 32)) / (8u * nk + 16u) & ~127u;
 }
 
 // Shared memory by its 32-bit address: the parts of the table start at offsets that depend on
@@ -412,6 +429,11 @@ __device__ __forceinline__ uint32_t slot_publish(uint32_t a, uint32_t v) {
     asm volatile("atom.release.cta.shared.cas.b32 %0, [%1], 0, %2;" : "=r"(old) : "r"(a), "r"(v) : "memory");
     return old;
 }
+__device__ __forceinline__ uint32_t sh_min(uint32_t a, uint32_t v) {
+    uint32_t old;
+    asm volatile("atom.shared.min.u32 %0, [%1], %2;" : "=r"(old) : "r"(a), "r"(v) : "memory");
+    return old;
+}
 __device__ __forceinline__ uint32_t first_of(bool a, bool b, bool c, bool d) { return a ? 0u : b ? 1u : c ? 2u : d ? 3u : 4u; }
 
 // A block barrier that every lane of a warp reaches together (loops whose lanes leave at
@@ -439,9 +461,10 @@ __device__ __forceinline__ void block_sync() {
 // queue of the warp and are resolved 32 at a time, so that the longer searches and the
 // entering of new keys run on full warps.  No lane waits for another: a new key's entry is
 // complete before its slot is.
-template <int NW, int WS, bool SAMPLE>
+template <int NW, int WS, int MODE>
 __global__ void __launch_bounds__(AGG_THREADS, 2) k_bin_agg(AggArgs A) {
     constexpr int NK = NW - WS;
+    constexpr bool SAMPLE = MODE == AGG_SAMPLE, FIRST = MODE == AGG_FIRST;
     extern __shared__ __align__(16) uint64_t agg_smem[];
     __shared__ uint32_t s_full, s_runs, s_entries, s_later, s_warp[AGG_THREADS / 32], s_alone[agg_entries(1, false) / 32];
     __shared__ unsigned long long s_base, s_low_base, s_next[3];  // next group, its bounds
@@ -464,7 +487,7 @@ __global__ void __launch_bounds__(AGG_THREADS, 2) k_bin_agg(AggArgs A) {
         const unsigned long long p0 = s_next[1], p1 = s_next[2];
         const uint32_t e0 = (uint32_t)(p0 >> 32), n_runs = (uint32_t)(p1 >> 32) - e0;
         const uint32_t windows = (uint32_t)p1 - (uint32_t)p0;
-        const bool wide = windows > AGG_NARROW_MAX;
+        const bool wide = !FIRST && windows > AGG_NARROW_MAX;
         block_sync();  // everyone has read s_next
         if (n_runs == 0 || (SAMPLE && wide)) {
             if (threadIdx.x == 0) fetch();
@@ -472,8 +495,8 @@ __global__ void __launch_bounds__(AGG_THREADS, 2) k_bin_agg(AggArgs A) {
             continue;
         }
         if (SAMPLE && threadIdx.x == 0) atomicAdd(&A.counters[BC_WINDOWS], (unsigned long long)windows);
-        const uint32_t cap = wide ? agg_entries(NK, true) : agg_entries(NK, false);
-        const uint32_t cl = wide ? 3u : 2u;  // log2(words of counts per entry)
+        const uint32_t cap = FIRST ? first_entries(NK) : wide ? agg_entries(NK, true) : agg_entries(NK, false);
+        const uint32_t cl = FIRST ? 0u : wide ? 3u : 2u;  // log2(words of counts per entry)
         const uint32_t n_buckets = cap / 2;
         const uint32_t ekey = sh_addr(agg_smem) + AGG_QUEUE * (AGG_THREADS / 32), ecnt = ekey + 8 * NK * cap, epos = ecnt + ((4 * cap) << cl), slots = epos + 4 * cap;
         auto window_hash = [&](Window<NK>& w, uint32_t g) {
@@ -484,7 +507,16 @@ __global__ void __launch_bounds__(AGG_THREADS, 2) k_bin_agg(AggArgs A) {
             w.tag = (uint32_t)hx & 0xFFFF0000u;
         };
         const uint32_t nr = wide ? 0u : 1u;
-        auto count_window = [&](const Window<NK>& w, uint32_t entry, bool on, bool has_l, bool has_r, bool again) {
+        auto count_window = [&](const Window<NK>& w, uint32_t g, uint32_t entry, bool on, bool has_l, bool has_r, bool again) {
+            if constexpr (FIRST) {
+                // the smaller of two places that meet stays the first, the other one is a
+                // candidate for the second; one beyond the second so far is neither
+                if (on && g < sh_ld(ecnt + 4 * entry)) {
+                    const uint32_t other = max(g, sh_min(epos + 4 * entry, g));
+                    if (other != NO_PLACE) sh_min(ecnt + 4 * entry, other);
+                }
+                return;
+            }
             sh_st_if(on && again && !(has_l && has_r), epos + 4 * entry, POS_TWICE);
             // pushes as u (base after the window) and as v (base before it)
             const uint32_t c = ecnt + ((4 * entry) << cl);
@@ -499,7 +531,7 @@ __global__ void __launch_bounds__(AGG_THREADS, 2) k_bin_agg(AggArgs A) {
         bool fetched = false;
         while (lo < (1ULL << 32)) {
             for (uint32_t i = threadIdx.x; i < n_buckets; i += blockDim.x) sh_zero128(slots + 16 * i);
-            if (threadIdx.x < cap / 32) s_alone[threadIdx.x] = 0;
+            if (!FIRST && threadIdx.x < cap / 32) s_alone[threadIdx.x] = 0;
             if (threadIdx.x == 0) s_full = s_runs = s_entries = s_later = 0;
             block_sync();
             if (threadIdx.x == 0 && !fetched) fetch();  // in flight while the group is counted
@@ -577,7 +609,7 @@ __global__ void __launch_bounds__(AGG_THREADS, 2) k_bin_agg(AggArgs A) {
                     for (int i = 0; i < NK; ++i) eq &= sh_ld64(ekey + 8 * (e * NK + i)) == w.key[i];
                     bool mine = live;
                     if (part) mine &= (smix(w.fold) >> 32) - lo < width;
-                    count_window(w, e, mine && eq, has_l, has_r, true);
+                    count_window(w, g, e, mine && eq, has_l, has_r, true);
                     const bool miss = mine && !eq;
                     const uint32_t m = __ballot_sync(0xffffffffu, miss);
                     sh_st64_if(miss, queue + 8 * (qn + __popc(m & ((1u << lane) - 1))), run_pack(g, 1, has_l, has_r, 0));
@@ -624,7 +656,7 @@ __global__ void __launch_bounds__(AGG_THREADS, 2) k_bin_agg(AggArgs A) {
 #pragma unroll
                             for (int i = 0; i < NK; ++i) eq &= sh_ld64(ekey + 8 * (e * NK + i)) == w.key[i];
                             if (eq) {
-                                if (entry != 0xFFFFFFFFu) sh_st(epos + 4 * entry, 0);  // an entry made for nothing
+                                if (!FIRST && entry != 0xFFFFFFFFu) sh_st(epos + 4 * entry, 0);  // an entry made for nothing
                                 entry = e;
                                 open = false;
                             }
@@ -644,9 +676,14 @@ __global__ void __launch_bounds__(AGG_THREADS, 2) k_bin_agg(AggArgs A) {
                                     entry = at;
 #pragma unroll
                                     for (int i = 0; i < NK; ++i) sh_st64(ekey + 8 * (at * NK + i), w.key[i]);
-                                    sh_zero128(ecnt + ((4 * at) << cl));
-                                    if (wide) sh_zero128(ecnt + 32 * at + 16);
-                                    sh_st(epos + 4 * at, g + 1);
+                                    if constexpr (FIRST) {
+                                        sh_st(ecnt + 4 * at, NO_PLACE);
+                                        sh_st(epos + 4 * at, NO_PLACE);
+                                    } else {
+                                        sh_zero128(ecnt + ((4 * at) << cl));
+                                        if (wide) sh_zero128(ecnt + 32 * at + 16);
+                                        sh_st(epos + 4 * at, g + 1);
+                                    }
                                 } else {
                                     put_off = true;
                                     open = live = false;
@@ -656,7 +693,7 @@ __global__ void __launch_bounds__(AGG_THREADS, 2) k_bin_agg(AggArgs A) {
                         if (open && !match) {
                             claimed = slot_publish(slots + 4 * slot, w.tag | (entry + 1)) == 0;
                             open = !claimed;  // taken meanwhile: the bucket is looked at again
-                            if (claimed && !has_l && !has_r) atomicOr(&s_alone[entry >> 5], 1u << (entry & 31));
+                            if (!FIRST && claimed && !has_l && !has_r) atomicOr(&s_alone[entry >> 5], 1u << (entry & 31));
                             from = 0;
                         }
                         if (++turns >= AGG_TURNS && open) {
@@ -675,7 +712,7 @@ __global__ void __launch_bounds__(AGG_THREADS, 2) k_bin_agg(AggArgs A) {
                             else s_full = 1;
                         }
                     }
-                    count_window(w, entry, live, has_l, has_r, !claimed);
+                    count_window(w, g, entry, live, has_l, has_r, !claimed);
                     __syncwarp();
                 }
             }
@@ -724,7 +761,21 @@ __global__ void __launch_bounds__(AGG_THREADS, 2) k_bin_agg(AggArgs A) {
             uint32_t n_row = 0, n_low = 0, codes = 0;  // 2 bits per entry of this thread
             static_assert(agg_entries(1, false) <= 16 * AGG_THREADS, "codes hold 16 entries a thread");
             uint32_t turn = 0;
-            for (uint32_t i = threadIdx.x; i < n_entries; i += blockDim.x, turn += 2) {
+            if constexpr (FIRST) {
+                if (threadIdx.x == 0) s_base = atomicAdd(&A.counters[BC_ROWS], (unsigned long long)n_entries);
+                block_sync();
+                for (uint32_t i = threadIdx.x; i < n_entries; i += blockDim.x) {
+                    FirstKey f{0, sh_ld(epos + 4 * i), sh_ld(ecnt + 4 * i)};
+                    if (f.at != NO_PLACE) {
+                        f.raw = nthash_canonical_at(A.data, f.at, k);
+#pragma unroll
+                        for (int row = 0; row < 4; ++row) atomicMin(A.first + cms_index(f.raw, row, A.log2w), f.at);
+                    }
+                    if (s_base + i < A.cap_rows) A.firsts[s_base + i] = f;
+                }
+                block_sync();
+            }
+            for (uint32_t i = threadIdx.x; !FIRST && i < n_entries; i += blockDim.x, turn += 2) {
                 const uint32_t pos = sh_ld(epos + 4 * i);
                 if (!pos) continue;
                 uint32_t e[8];
@@ -747,7 +798,7 @@ __global__ void __launch_bounds__(AGG_THREADS, 2) k_bin_agg(AggArgs A) {
                 tot_multi += n_row + n_low;
                 tot_kept += n_row;
                 block_sync();
-            } else {
+            } else if constexpr (!FIRST) {
                 // rows and low rows are counted, reserved once, then written
                 n_row = __reduce_add_sync(0xffffffffu, n_row);
                 n_low = __reduce_add_sync(0xffffffffu, n_low);
@@ -1098,6 +1149,38 @@ __global__ void __launch_bounds__(256) k_bin_gate(LadderDev L, uint32_t k, Table
     }
 }
 
+// The estimator's registers from its distinct keys (see bins_first).  The segment of a place:
+// the last one whose first read begins there or before.
+__global__ void __launch_bounds__(256) k_first_regs(const FirstKey* __restrict__ keys, uint64_t n, const uint64_t* __restrict__ off,
+                                                    const uint32_t* __restrict__ first, uint32_t log2w, uint32_t p, uint32_t n_segs,
+                                                    uint32_t* regs_total, uint32_t* regs_solid) {
+    const uint64_t m = 1ULL << p;
+    auto segment = [&](uint32_t place) {
+        uint32_t lo = 0, hi = n_segs;
+        while (hi - lo > 1) {
+            const uint32_t mid = (lo + hi) / 2;
+            if (off[2 * (6000 + 2000 * (uint64_t)(mid - 1))] <= place) lo = mid;
+            else hi = mid;
+        }
+        return lo;
+    };
+    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
+        const FirstKey f = keys[i];
+        if (f.at == NO_PLACE) continue;
+        bool solid = true;
+#pragma unroll
+        for (int row = 0; row < 4; ++row) solid &= __ldcg(first + cms_index(f.raw, row, log2w)) < f.at;
+        uint32_t idx, rho;
+        hll_idx_rho(smix(f.raw), p, idx, rho);
+        const uint32_t s1 = segment(f.at);
+        uint32_t* rt = regs_total + s1 * m + idx;
+        if (__ldca(rt) < rho) atomicMax(rt, rho);
+        if (!solid && f.again == NO_PLACE) continue;
+        uint32_t* rs = regs_solid + (solid ? s1 : segment(f.again)) * m + idx;
+        if (__ldca(rs) < rho) atomicMax(rs, rho);
+    }
+}
+
 // ---------------------------------------------------------------------------
 // launchers
 // ---------------------------------------------------------------------------
@@ -1108,16 +1191,20 @@ int resident_grid(K kernel, int block, size_t smem, int sms) {
     return per_sm * sms;
 }
 
-template <int NW, int WS>
-cudaError_t agg_launch(cudaStream_t st, int sms, const AggArgs& A, bool sample) {
-    auto go = [&](auto kern) -> cudaError_t {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)AGG_SMEM);
-        if (e != cudaSuccess) return e;
-        const int grid = std::min<int>(2 * sms, (int)std::max<uint32_t>(1, A.n_groups));  // later holds that many
-        kern<<<grid, AGG_THREADS, AGG_SMEM, st>>>(A);
-        return cudaGetLastError();
-    };
-    return sample ? go(k_bin_agg<NW, WS, true>) : go(k_bin_agg<NW, WS, false>);
+template <int NW, int WS, int MODE>
+cudaError_t agg_launch(cudaStream_t st, int sms, const AggArgs& A) {
+    auto kern = k_bin_agg<NW, WS, MODE>;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)AGG_SMEM);
+    if (e != cudaSuccess) return e;
+    const int grid = std::min<int>(2 * sms, (int)std::max<uint32_t>(1, A.n_groups));  // later holds that many
+    kern<<<grid, AGG_THREADS, AGG_SMEM, st>>>(A);
+    return cudaGetLastError();
+}
+// The modes that write no rows know a key by its significant words alone.
+template <int MODE>
+cudaError_t agg_launch_nk(int nk, cudaStream_t st, int sms, const AggArgs& A) {
+    return nk == 1 ? agg_launch<1, 0, MODE>(st, sms, A) : nk == 2 ? agg_launch<2, 0, MODE>(st, sms, A)
+           : nk == 3 ? agg_launch<3, 0, MODE>(st, sms, A) : agg_launch<4, 0, MODE>(st, sms, A);
 }
 template <class Kern, class... Args>
 cudaError_t stream_launch(cudaStream_t st, int sms, uint64_t n_threads, Kern kern, Args... args) {
@@ -1178,6 +1265,92 @@ bool bins_applicable(const fbk_ctx* ctx, const fbk_bank* b, const fbk_build_para
 constexpr uint64_t BINS_SAMPLE_FROM = 4u << 20;
 constexpr uint64_t BINS_SMALL_GROUP = 6000;  // windows of a group then
 
+namespace {
+
+// The reads' runs by bin.
+struct BinRuns {
+    MinPlan mp;
+    uint32_t F = 64;                              // bins, about 1500 windows each
+    unsigned long long *hist = nullptr, *counters = nullptr;  // the caller's, cleared with it
+    unsigned long long* pre = nullptr;            // (runs << 32 | windows) before each bin
+    uint64_t* runs = nullptr;
+    uint64_t n_windows = 0;
+    BinRuns(const MinPlan& m, uint64_t windows) : mp(m) {
+        while (F < RUN_MAX_BINS && (uint64_t)F * 1500 < windows) F <<= 1;
+    }
+};
+
+// Cuts the reads of bv into runs (windows: no fewer than they hold) and scatters them by bin;
+// with a sample, counts the keys of some bins.  The counters and n_windows are on the host
+// then, in ctx->h_pinned.  Clears the caller's block first.
+fbk_status bin_runs(fbk_ctx* ctx, Scratch& B, BinRuns& R, const BankDev& bv, uint32_t max_len, uint32_t k, uint64_t windows, char* cleared,
+                    uint64_t clear_bytes, AggArgs* sample, bool* declined) {
+    const MinPlan mp = R.mp;
+    const uint32_t F = R.F;
+    const int sms = ctx->num_sms;
+    const cudaStream_t stream = ctx->stream;
+    const uint64_t n_reads = bv.r_end - bv.r_begin;
+    R.pre = (unsigned long long*)B.get(8ULL * (F + 1 + (F + SCAN_TILE - 1) / SCAN_TILE));
+    uint32_t* cursor = (uint32_t*)B.get(4ULL * F);
+    if (!R.pre || !cursor) return set_err(ctx, FBK_ERR_OOM, "minimizer bins");
+    unsigned long long* part = R.pre + F + 1;
+    const uint64_t max_warps = (uint64_t)resident_grid(k_bin_runs, 256, 0, sms) * 8;
+    const uint64_t n_blocks = std::max<uint64_t>(1, std::min<uint64_t>(max_warps, n_reads) / 8);
+    const uint64_t n_warps = n_blocks * 8;
+    // a run holds about (w + 1) / 2 windows, and one more ends with every read
+    uint64_t cap_w = (uint64_t)(1.3 * ((2.0 * windows) / (mp.w + 1) + n_reads) / n_warps) + 128 + std::min<uint64_t>(max_len / 4, 2048);
+    uint32_t* log_n = (uint32_t*)B.get(4 * n_warps);
+    if (!log_n) return set_err(ctx, FBK_ERR_OOM, "minimizer bins");
+    unsigned long long* h = (unsigned long long*)ctx->h_pinned;
+    uint64_t* log = nullptr;
+    for (int attempt = 0;; ++attempt) {
+        log = (uint64_t*)B.get(8 * n_warps * cap_w);
+        R.runs = (uint64_t*)B.get(8 * n_warps * cap_w);
+        if (!log || !R.runs) return set_err(ctx, FBK_ERR_OOM, "minimizer bins: runs");
+        CK(ctx, cudaMemsetAsync(cleared, 0, clear_bytes, stream));
+        TIMED(ctx, "bins_runs", (k_bin_runs<<<(unsigned)n_blocks, 256, 0, stream>>>(bv, k, mp, F, log, log_n, (uint32_t)cap_w, R.hist,
+                                                                                    R.counters + BC_NEED),
+                                 cudaGetLastError()));
+        const unsigned tiles = (F + SCAN_TILE - 1) / SCAN_TILE;
+        TIMED(ctx, "bins_scan", (k_bin_scan_sums<<<tiles, 256, 0, stream>>>(R.hist, F, part), cudaGetLastError()));
+        TIMED(ctx, "bins_scan", (k_bin_scan<<<tiles, 256, 0, stream>>>(R.hist, F, part, R.pre, cursor), cudaGetLastError()));
+        TIMED(ctx, "bins_scatter", (k_bin_scatter<<<(unsigned)n_blocks, 256, 0, stream>>>(log, log_n, (uint32_t)cap_w, cursor, R.runs,
+                                                                                          n_warps * cap_w),
+                                    cudaGetLastError()));
+        if (sample) {
+            sample->runs = R.runs;
+            sample->n_groups = std::min<uint32_t>(F, 1024);
+            sample->stride = F / sample->n_groups;
+            sample->start = R.pre;
+            TIMED(ctx, "bins_sample", agg_launch_nk<AGG_SAMPLE>((int)((k + 31) / 32), stream, sms, *sample));
+        }
+        CK(ctx, cudaMemcpyAsync(h, R.counters, 8 * BC_N, cudaMemcpyDeviceToHost, stream));
+        CK(ctx, cudaMemcpyAsync(h + BC_N, R.pre + F, 8, cudaMemcpyDeviceToHost, stream));
+        CK(ctx, cudaStreamSynchronize(stream));
+        R.n_windows = h[BC_N] & 0xFFFFFFFFull;
+        if (!h[BC_NEED]) break;
+        // a warp's log was too short: once more with room for the longest, unless a few reads
+        // are so much longer than the rest that the logs of all warps would take gigabytes
+        if (attempt == 1 || h[BC_NEED] * n_warps > 4 * windows + (64ULL << 20)) {
+            *declined = true;
+            return FBK_OK;
+        }
+        cap_w = h[BC_NEED];
+        B.drop(log);
+        B.drop(R.runs);
+    }
+    B.drop(log);
+    return FBK_OK;
+}
+
+// Windows of a group of bins whose keys about fill 0.7 of the entries.
+uint64_t group_windows(uint32_t entries, uint64_t n_windows, uint64_t distinct) {
+    const uint64_t t = (uint64_t)(0.7 * (double)entries * (double)std::max<uint64_t>(n_windows, 1) / (double)std::max<uint64_t>(distinct, 1));
+    return std::max<uint64_t>(512, std::min<uint64_t>(t, 60000));
+}
+
+}  // namespace
+
 fbk_status bins_build(fbk_ctx* ctx, const fbk_bank* b, const fbk_build_params* p, const uint64_t* keep_bits, uint32_t log2w,
                       fbk_table** out, bool* declined) {
     *declined = false;
@@ -1191,34 +1364,22 @@ fbk_status bins_build(fbk_ctx* ctx, const fbk_bank* b, const fbk_build_params* p
     const int sms = ctx->num_sms;
     const cudaStream_t stream = ctx->stream;
     Scratch B{ctx, {}};
-    uint32_t F = 64;
-    while (F < RUN_MAX_BINS && (uint64_t)F * 1500 < windows) F <<= 1;
+    BinRuns R(mp, windows);
+    const uint32_t F = R.F;
     // one cleared block: the ladder, the bin and build counters, the windows' bitmaps
     const uint64_t bm_words = (b->n_words + 63) & ~63ULL;
     const uint64_t lad_bytes = (2 * (4ULL << log2w) / 8 + 255) & ~255ULL;
     const uint64_t clear_bytes = lad_bytes + 8ULL * F + 8 * 16 + 2 * 4 * bm_words;
     static_assert(BC_N <= 16, "build counters");
     char* cleared = (char*)B.get(clear_bytes);
-    unsigned long long* pre = (unsigned long long*)B.get(8ULL * (F + 1 + (F + SCAN_TILE - 1) / SCAN_TILE));
-    uint32_t* cursor = (uint32_t*)B.get(4ULL * F);
     uint32_t* pass = (uint32_t*)B.get(4 * bm_words);
-    if (!cleared || !pre || !cursor || !pass) return set_err(ctx, FBK_ERR_OOM, "minimizer bins");
+    if (!cleared || !pass) return set_err(ctx, FBK_ERR_OOM, "minimizer bins");
     uint32_t* lad = (uint32_t*)cleared;
-    unsigned long long* hist = (unsigned long long*)(cleared + lad_bytes);
-    unsigned long long* counters = hist + F;
+    R.hist = (unsigned long long*)(cleared + lad_bytes);
+    unsigned long long* counters = R.counters = R.hist + F;
     uint32_t* single = (uint32_t*)(counters + 16);
     uint32_t* valid = single + bm_words;
-    unsigned long long* part = pre + F + 1;
     const BankDev bv = bank_view(b, 0, b->n_reads, keep_bits);
-    const uint64_t max_warps = (uint64_t)resident_grid(k_bin_runs, 256, 0, sms) * 8;
-    const uint64_t n_blocks = std::max<uint64_t>(1, std::min<uint64_t>(max_warps, b->n_reads) / 8);
-    const uint64_t n_warps = n_blocks * 8;
-    // a run holds about (w + 1) / 2 windows, and one more ends with every read
-    uint64_t cap_w = (uint64_t)(1.3 * ((2.0 * windows) / (mp.w + 1) + b->n_reads) / n_warps) + 128 +
-                     std::min<uint64_t>(b->max_len / 4, 2048);
-    uint32_t* log_n = (uint32_t*)B.get(4 * n_warps);
-    if (!log_n) return set_err(ctx, FBK_ERR_OOM, "minimizer bins");
-    uint64_t *log = nullptr, *runs = nullptr;
     AggArgs A{};
     A.data = b->data;
     A.k = k;
@@ -1228,51 +1389,15 @@ fbk_status bins_build(fbk_ctx* ctx, const fbk_bank* b, const fbk_build_params* p
     A.later_cap = sampled ? AGG_LATER : 4096;
     A.later = (uint64_t*)B.get(16ULL * A.later_cap * (sampled ? 2 * sms : std::min<uint64_t>(2 * sms, windows / BINS_SMALL_GROUP + 1)));
     if (!A.later) return set_err(ctx, FBK_ERR_OOM, "minimizer bins");
-    auto agg = [&](bool sample) {
-        return by_width(nw, k, [&](auto a, auto w) { return agg_launch<decltype(a)::value, decltype(w)::value>(stream, sms, A, sample); });
-    };
     unsigned long long* h = (unsigned long long*)ctx->h_pinned;
     const bool may_filter = p->min_trans_cov >= 2 && ctx->acc_filter != 0;
-    uint64_t n_windows = 0;
     CK(ctx, cudaMemsetAsync(ctx->d_status, 0, 4, stream));
-    for (int attempt = 0;; ++attempt) {
-        log = (uint64_t*)B.get(8 * n_warps * cap_w);
-        runs = (uint64_t*)B.get(8 * n_warps * cap_w);
-        if (!log || !runs) return set_err(ctx, FBK_ERR_OOM, "minimizer bins: runs");
-        CK(ctx, cudaMemsetAsync(cleared, 0, clear_bytes, stream));
-        TIMED(ctx, "bins_runs", (k_bin_runs<<<(unsigned)n_blocks, 256, 0, stream>>>(bv, k, mp, F, log, log_n, (uint32_t)cap_w, hist,
-                                                                                    counters + BC_NEED),
-                                 cudaGetLastError()));
-        const unsigned tiles = (F + SCAN_TILE - 1) / SCAN_TILE;
-        TIMED(ctx, "bins_scan", (k_bin_scan_sums<<<tiles, 256, 0, stream>>>(hist, F, part), cudaGetLastError()));
-        TIMED(ctx, "bins_scan", (k_bin_scan<<<tiles, 256, 0, stream>>>(hist, F, part, pre, cursor), cudaGetLastError()));
-        TIMED(ctx, "bins_scatter", (k_bin_scatter<<<(unsigned)n_blocks, 256, 0, stream>>>(log, log_n, (uint32_t)cap_w, cursor, runs,
-                                                                                          n_warps * cap_w),
-                                    cudaGetLastError()));
-        if (sampled) {
-            A.runs = runs;
-            A.n_groups = std::min<uint32_t>(F, 1024);
-            A.stride = F / A.n_groups;
-            A.start = pre;
-            A.mtc = may_filter ? p->min_trans_cov : 0;
-            TIMED(ctx, "bins_sample", agg(true));
-        }
-        CK(ctx, cudaMemcpyAsync(h, counters, 8 * BC_N, cudaMemcpyDeviceToHost, stream));
-        CK(ctx, cudaMemcpyAsync(h + BC_N, pre + F, 8, cudaMemcpyDeviceToHost, stream));
-        CK(ctx, cudaStreamSynchronize(stream));
-        n_windows = h[BC_N] & 0xFFFFFFFFull;
-        if (!h[BC_NEED]) break;
-        // a warp's log was too short: once more with room for the longest, unless a few reads
-        // are so much longer than the rest that the logs of all warps would take gigabytes
-        if (attempt == 1 || h[BC_NEED] * n_warps > 4 * windows + (64ULL << 20)) {
-            *declined = true;
-            return FBK_OK;
-        }
-        cap_w = h[BC_NEED];
-        B.drop(log);
-        B.drop(runs);
-    }
-    B.drop(log);
+    A.mtc = may_filter ? p->min_trans_cov : 0;
+    fbk_status rs = bin_runs(ctx, B, R, bv, b->max_len, k, windows, cleared, clear_bytes, sampled ? &A : nullptr, declined);
+    if (rs || *declined) return rs;
+    const uint64_t n_windows = R.n_windows;
+    uint64_t* runs = R.runs;
+    unsigned long long* pre = R.pre;
     uint64_t distinct = n_windows, multi = n_windows, kept = n_windows;  // upper bounds without a sample
     bool filter = may_filter && (ctx->acc_filter == 2 || nw == 4);
     if (sampled && h[BC_WINDOWS]) {
@@ -1284,11 +1409,7 @@ fbk_status bins_build(fbk_ctx* ctx, const fbk_bank* b, const fbk_build_params* p
         filter = may_filter && acc_filter_on(ctx->acc_filter, nw, distinct, n_windows);
     }
     // groups that about fill 0.7 of the entries, with few enough windows for 16-bit counts
-    uint64_t target = BINS_SMALL_GROUP;
-    if (sampled)
-        target = (uint64_t)(0.7 * (double)agg_entries(nk, false) * (double)std::max<uint64_t>(n_windows, 1) /
-                            (double)std::max<uint64_t>(distinct, 1));
-    target = std::max<uint64_t>(512, std::min<uint64_t>(target, 60000));
+    const uint64_t target = sampled ? group_windows(agg_entries(nk, false), n_windows, distinct) : BINS_SMALL_GROUP;
     const uint32_t n_groups = (uint32_t)(n_windows / target + 1);
     unsigned long long* start = (unsigned long long*)B.get(8ULL * (n_groups + 1));
     if (!start) return set_err(ctx, FBK_ERR_OOM, "minimizer bins: groups");
@@ -1334,7 +1455,9 @@ fbk_status bins_build(fbk_ctx* ctx, const fbk_bank* b, const fbk_build_params* p
         TIMED(ctx, "bins_groups",
               (k_bin_groups<<<std::min<unsigned>(1024, (F + 256) / 256), 256, 0, stream>>>(pre, F, (uint32_t)target, n_groups, start),
                cudaGetLastError()));
-        TIMED(ctx, "bins_aggregate", agg(false));
+        TIMED(ctx, "bins_aggregate", by_width(nw, k, [&](auto a, auto w) {
+                  return agg_launch<decltype(a)::value, decltype(w)::value, AGG_BUILD>(stream, sms, A);
+              }));
         CK(ctx, cudaMemcpyAsync(h, counters, 8 * BC_N, cudaMemcpyDeviceToHost, stream));
         CK(ctx, cudaMemcpyAsync(h + BC_N, ctx->d_status, 4, cudaMemcpyDeviceToHost, stream));
         CK(ctx, cudaStreamSynchronize(stream));
@@ -1398,6 +1521,73 @@ fbk_status bins_build(fbk_ctx* ctx, const fbk_bank* b, const fbk_build_params* p
     tb->pushes = pushes;
     guard.t = nullptr;
     *out = tb;
+    return FBK_OK;
+}
+
+// The estimator's sample loop over distinct k-mers.  Of a k-mer's occurrences only the first
+// two say anything: the first touches its four counters earliest and is solid iff each was
+// touched before (by another k-mer), and every later one is solid, as the first has touched
+// them; a register takes the k-mer's hash from its first occurrence and its solid one from the
+// first that is solid.  So the bins give each key's first two places, the first touches are
+// the minimum over the keys, and the registers follow from the keys.
+//
+// Adds the reads [0, n_reads) to first and to the segments' registers (not yet prefixed),
+// which may hold what earlier rounds put there: minima and maxima of a part of the same
+// values.  Declined, with nothing spoilt, where memory is short or more than 0.4 of the windows
+// (0.3 for keys of several words) are distinct: a distinct key costs four random atomics and four random loads here and a
+// window about as much in the loop over occurrences (39 M windows of a 5 Mbp genome, k = 21,
+// 0.23 distinct: 2.0 ms here, 3.15 there; 36 M, k = 31, 0.41: 2.7 and 2.9; 30 M, k = 51, 0.39:
+// 2.8 and 2.4).
+fbk_status bins_first(fbk_ctx* ctx, const fbk_bank* b, uint64_t n_reads, uint64_t windows, uint32_t k, uint32_t* first, uint32_t log2w,
+                      uint32_t p, uint32_t n_segs, uint32_t* regs_total, uint32_t* regs_solid, bool* declined) {
+    *declined = true;
+    const int nk = (int)((k + 31) / 32), sms = ctx->num_sms;
+    const cudaStream_t stream = ctx->stream;
+    Scratch B{ctx, {}};
+    BinRuns R(min_plan(k), windows);
+    const uint64_t clear_bytes = 8ULL * R.F + 8 * 16;
+    char* cleared = (char*)B.get(clear_bytes);
+    AggArgs A{};
+    A.data = b->data;
+    A.k = k;
+    A.status = ctx->d_status;
+    A.later_cap = AGG_LATER;
+    A.later = (uint64_t*)B.get(16ULL * A.later_cap * 2 * sms);
+    if (!cleared || !A.later) return FBK_OK;
+    R.hist = (unsigned long long*)cleared;
+    A.counters = R.counters = R.hist + R.F;
+    unsigned long long* h = (unsigned long long*)ctx->h_pinned;
+    CK(ctx, cudaMemsetAsync(ctx->d_status, 0, 4, stream));
+    bool no = false;
+    fbk_status st = bin_runs(ctx, B, R, bank_view(b, 0, n_reads, nullptr), b->max_len, k, windows, cleared, clear_bytes, &A, &no);
+    if (st == FBK_ERR_OOM || no) return FBK_OK;
+    if (st) return st;
+    const uint64_t n_windows = R.n_windows;
+    const double share = h[BC_WINDOWS] ? (double)h[BC_DISTINCT] / (double)h[BC_WINDOWS] : 1.0;
+    if (share > (nk == 1 ? 0.4 : 0.3)) return FBK_OK;
+    const uint64_t distinct = std::min<uint64_t>(n_windows, (uint64_t)(1.1 * share * (double)n_windows) + 65536);
+    const uint64_t target = group_windows(first_entries(nk), n_windows, distinct);
+    A.runs = R.runs;
+    A.stride = 1;
+    A.n_groups = (uint32_t)(n_windows / target + 1);
+    unsigned long long* start = (unsigned long long*)B.get(8ULL * (A.n_groups + 1));
+    A.first = first;
+    A.log2w = log2w;
+    A.cap_rows = distinct + distinct / 8;  // some entries are made for nothing
+    A.firsts = (FirstKey*)B.get(A.cap_rows * sizeof(FirstKey));
+    if (!start || !A.firsts) return FBK_OK;
+    A.start = start;
+    TIMED(ctx, "bins_groups", (k_bin_groups<<<std::min<unsigned>(1024, (R.F + 256) / 256), 256, 0, stream>>>(R.pre, R.F, (uint32_t)target,
+                                                                                                          A.n_groups, start),
+                               cudaGetLastError()));
+    TIMED(ctx, "est_first_keys", agg_launch_nk<AGG_FIRST>(nk, stream, sms, A));
+    CK(ctx, cudaMemcpyAsync(h, A.counters, 8 * BC_N, cudaMemcpyDeviceToHost, stream));
+    CK(ctx, cudaMemcpyAsync(h + BC_N, ctx->d_status, 4, cudaMemcpyDeviceToHost, stream));
+    CK(ctx, cudaStreamSynchronize(stream));
+    if ((uint32_t)h[BC_N] || h[BC_ROWS] > A.cap_rows) return FBK_OK;
+    TIMED(ctx, "est_first_regs", stream_launch(stream, sms, h[BC_ROWS], k_first_regs, (const FirstKey*)A.firsts, (uint64_t)h[BC_ROWS],
+                                               (const uint64_t*)b->off, (const uint32_t*)first, log2w, p, n_segs, regs_total, regs_solid));
+    *declined = false;
     return FBK_OK;
 }
 

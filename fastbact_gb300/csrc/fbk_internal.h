@@ -267,6 +267,9 @@ constexpr uint32_t BINS_MIN_K = 17;
 bool bins_applicable(const fbk_ctx* ctx, const fbk_bank* b, const fbk_build_params* p, uint32_t log2w);
 fbk_status bins_build(fbk_ctx* ctx, const fbk_bank* b, const fbk_build_params* p, const uint64_t* keep_bits, uint32_t log2w,
                       fbk_table** out, bool* declined);
+// The estimator's sample loop over the bins (fbk_bins.cu): k at least BINS_MIN_K.
+fbk_status bins_first(fbk_ctx* ctx, const fbk_bank* b, uint64_t n_reads, uint64_t windows, uint32_t k, uint32_t* first, uint32_t log2w,
+                      uint32_t p, uint32_t n_segs, uint32_t* regs_total, uint32_t* regs_solid, bool* declined);
 
 // host f64 HyperLogLog::estimate from the register sum and zero count (sketch.rs:83-114)
 double hll_estimate_from_sum(double sum, uint64_t zeros, uint32_t p);

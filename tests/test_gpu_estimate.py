@@ -5,7 +5,9 @@ sequential loop: registers and whole numbers, and the floats from the same opera
 The loop stops at the first checkpoint, in a later round, at no checkpoint (the sample ends
 inside a segment), or has fewer pairs than one; small sketches, whose counters are shared by
 many k-mers; every word count of k; and a sample whose reads do not lie in read order in
-its packed words."""
+its packed words.  Samples of more than 8 M k-mers go over the distinct ones (k of every word
+count, counters shared by several k-mers, a round that begins in the middle), unless most of
+them are distinct."""
 import numpy as np
 import pytest
 
@@ -37,3 +39,17 @@ def test_sample_loop_rounds(ctx, genome, cov, k, p, log2w, in_order):
     if not in_order:
         sample = api.BitSeqArena(sample.data, sample.offsets[::-1].copy(), sample.lengths[::-1].copy())
     same(ctx, sample, n, stats, k, p, log2w)
+
+
+@pytest.mark.parametrize("genome,cov,k,p,log2w,errors,distinct", [
+    (2_500_000, 5.0, 21, 14, 23, 0.005, True), (2_500_000, 5.0, 31, 14, 20, 0.005, True), (2_000_000, 6.0, 33, 16, 23, 0.002, True),
+    (1_000_000, 19.0, 77, 14, 16, 0.001, True), (1_000_000, 27.0, 101, 14, 22, 0.001, True), (2_000_000, 10.0, 77, 14, 23, 0.03, False)])
+def test_whole_samples(ctx, genome, cov, k, p, log2w, errors, distinct):
+    prm = api.synth_params(seed=genome + k, genome_len=genome, coverage=cov, gc=0.5, n_repeats=5, repeat_len=2000, sub_rate=errors)
+    _, _, sample, n, stats = api.synth_isolate(prm, sample_pairs=150_000)
+    assert int(np.maximum(sample.lengths[:2 * n].astype(np.int64) - k + 1, 0).sum()) > 8 << 20
+    ctx.timing_reset()
+    ctx.set_timing(True)
+    same(ctx, sample, n, stats, k, p, log2w)
+    ctx.set_timing(False)
+    assert (ctx.timing("est_first_regs")[0] > 0) == distinct
