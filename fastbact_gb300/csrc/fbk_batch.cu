@@ -273,6 +273,32 @@ uint64_t phase_a_bytes(const fbk_batch* B, const BatchIso* it) {
     return gate_bytes(B) + 4096 * 4 + (B->ladder ? 0 : (it->bank->n_words + 9) * 4) + 4096;
 }
 
+// The isolate the autotuners time their candidates on: the one of median size, whose trials
+// cost half or a third of the largest one's.
+size_t tune_pick(const std::vector<BatchIso*>& W) {
+    std::vector<size_t> o(W.size());
+    for (size_t i = 0; i < o.size(); ++i) o[i] = i;
+    std::nth_element(o.begin(), o.begin() + o.size() / 2, o.end(),
+                     [&](size_t a, size_t b) { return W[a]->bank->n_bases < W[b]->bank->n_bases; });
+    return o[o.size() / 2];
+}
+
+// Candidate block sizes and grids (blocks per SM, 0 = the occupancy grid) of an autotuned
+// kernel, one after the other: the block first, then the grid for the block kept.  The two
+// hardly depend on one another, and 4 trials of the 6 pairs are left.  trial(block, blocks per
+// SM) times one and keeps the fastest; it returns the block kept so far.
+template <class Trial>
+fbk_status tune_shapes(Trial&& trial) {
+    int block = 0;
+    fbk_status st = FBK_OK;
+    for (int bl : {128, 256})
+        if (st == FBK_OK) st = trial(bl, 0, &block);
+    const int kept = block;
+    for (int ps : {2, 4})
+        if (st == FBK_OK) st = trial(kept, ps, &block);
+    return st;
+}
+
 // Autotuner: times candidate launch shapes of the pass-1 and solidity kernels on one
 // isolate (its own sketch and bitmap as scratch) and keeps the fastest.
 fbk_status autotune(fbk_batch* B, BatchIso* it) {
@@ -285,8 +311,6 @@ fbk_status autotune(fbk_batch* B, BatchIso* it) {
     st = upload_wave(B, one, w);
     if (st) return st;
     const uint64_t cms_bytes = gate_bytes(B);
-    const int blocks[] = {128, 256};
-    const int per_sm[] = {0, 2, 4};
     const int rows_all[] = {4, 2, 1};
     const int rows_one[] = {4};
     // a ladder serves all rows in one sweep: only block and grid are tuned
@@ -303,27 +327,31 @@ fbk_status autotune(fbk_batch* B, BatchIso* it) {
     };
     float best = 1e30f;
     Shape best1 = B->pass1;
-    for (int rp : rows)
-        for (int bl : blocks)
-            for (int ps : per_sm) {
-                Shape s{bl, ps ? ps * ctx->num_sms : 0, rp};
-                CK(ctx, cudaMemsetAsync(gate, 0, cms_bytes, ctx->stream));
-                float ms = 0;
-                st = timed([&]() -> fbk_status {
-                    if (B->ladder) {
-                        TIMED(ctx, "tune_pass1", launch_batch_lpass1(B->nw, shape_launch(ctx, s), w.iso, w.rb, 1, B->p.k));
-                        return FBK_OK;
-                    }
-                    for (uint32_t r = 0; r < 4; r += (uint32_t)rp)
-                        TIMED(ctx, "tune_pass1", launch_batch_pass1(B->nw, shape_launch(ctx, s), w.iso, w.rb, 1, B->p.k, r, r + rp, 0));
+    for (int rp : rows) {
+        st = tune_shapes([&](int bl, int ps, int* kept) -> fbk_status {
+            Shape s{bl, ps ? ps * ctx->num_sms : 0, rp};
+            CK(ctx, cudaMemsetAsync(gate, 0, cms_bytes, ctx->stream));
+            float ms = 0;
+            fbk_status s3 = timed([&]() -> fbk_status {
+                if (B->ladder) {
+                    TIMED(ctx, "tune_pass1", launch_batch_lpass1(B->nw, shape_launch(ctx, s), w.iso, w.rb, 1, B->p.k));
                     return FBK_OK;
-                }, &ms);
-                if (st) return st;
-                if (ms < best) {
-                    best = ms;
-                    best1 = s;
                 }
+                for (uint32_t r = 0; r < 4; r += (uint32_t)rp)
+                    TIMED(ctx, "tune_pass1", launch_batch_pass1(B->nw, shape_launch(ctx, s), w.iso, w.rb, 1, B->p.k, r, r + rp, 0));
+                return FBK_OK;
+            }, &ms);
+            if (s3) return s3;
+            if (!*kept) *kept = bl;
+            if (ms < best) {
+                best = ms;
+                best1 = s;
+                *kept = bl;
             }
+            return FBK_OK;
+        });
+        if (st) return st;
+    }
     // With a ladder gate the single-isolate pass 1 (its form chosen per key width by the
     // context) is a candidate too: one launch per isolate of the wave.
     bool single = false;
@@ -346,23 +374,27 @@ fbk_status autotune(fbk_batch* B, BatchIso* it) {
     const uint64_t bm_bytes = (it->bank->n_words + 9) * 4;
     best = 1e30f;
     Shape best2 = B->solid;
-    for (int rp : (B->ladder ? std::vector<int>() : rows))
-        for (int bl : blocks)
-            for (int ps : per_sm) {
-                Shape s{bl, ps ? ps * ctx->num_sms : 0, rp};
-                CK(ctx, cudaMemsetAsync(it->bm, 0xFF, bm_bytes, ctx->stream));
-                float ms = 0;
-                st = timed([&]() -> fbk_status {
-                    for (uint32_t r = 0; r < 4; r += (uint32_t)rp)
-                        TIMED(ctx, "tune_solid", launch_batch_solid(B->nw, shape_launch(ctx, s), w.iso, w.rb, 1, B->p.k, r, r + rp));
-                    return FBK_OK;
-                }, &ms);
-                if (st) return st;
-                if (ms < best) {
-                    best = ms;
-                    best2 = s;
-                }
+    for (int rp : (B->ladder ? std::vector<int>() : rows)) {
+        st = tune_shapes([&](int bl, int ps, int* kept) -> fbk_status {
+            Shape s{bl, ps ? ps * ctx->num_sms : 0, rp};
+            CK(ctx, cudaMemsetAsync(it->bm, 0xFF, bm_bytes, ctx->stream));
+            float ms = 0;
+            fbk_status s3 = timed([&]() -> fbk_status {
+                for (uint32_t r = 0; r < 4; r += (uint32_t)rp)
+                    TIMED(ctx, "tune_solid", launch_batch_solid(B->nw, shape_launch(ctx, s), w.iso, w.rb, 1, B->p.k, r, r + rp));
+                return FBK_OK;
+            }, &ms);
+            if (s3) return s3;
+            if (!*kept) *kept = bl;
+            if (ms < best) {
+                best = ms;
+                best2 = s;
+                *kept = bl;
             }
+            return FBK_OK;
+        });
+        if (st) return st;
+    }
     B->pass1 = best1;
     B->pass1_single = single;
     B->solid = best2;
@@ -372,7 +404,7 @@ fbk_status autotune(fbk_batch* B, BatchIso* it) {
     return FBK_OK;
 }
 
-// Phase-B autotuner (ladder gate): on the first phase-B isolate, with its table and
+// Phase-B autotuner (ladder gate): on one phase-B isolate (tune_pick), with its table and
 // record buckets allocated, time the record emit in each form and block shape — flat
 // window stream with blocks of 128 or 256, one lane per read (rolled) — and, when the
 // isolate's pass upserts every bucket in one persistent launch, that launch with blocks
@@ -425,34 +457,29 @@ fbk_status autotune_b(fbk_batch* B, BatchIso* it, bool persistent_upsert) {
     }
     if (st == FBK_OK && persistent_upsert) {
         // the buckets hold the last trial's records (every form writes the same records)
-        const int blocks[] = {128, 256};
-        const int per_sm[] = {0, 2, 4};
         best = 1e30f;
         Shape best_u = B->upsert;
-        for (int bl : blocks)
-            for (int ps : per_sm) {
-                const Shape sh{bl, ps ? ps * ctx->num_sms : 0, 0};
-                cudaError_t e = cudaSuccess;
-                st = FBK_OK;
-                TIMED(ctx, "table_init", launch_table_init(B->nw, launch_cfg(ctx, 256, 0), tbl_dev(it->table)));
-                e = cudaMemsetAsync(it->table->cnt, 0, it->table->cap * 32, ctx->stream);
-                if (e == cudaSuccess) e = cudaMemsetAsync(flags, 0, 24, ctx->stream);
-                if (e != cudaSuccess) {
-                    st = cuda_err(ctx, e, "batch autotuner");
-                    break;
-                }
-                float ms = 0;
-                st = timed([&]() -> fbk_status {
-                    TIMED(ctx, "tune_upsert", launch_upsert_all(B->nw, shape_launch(ctx, sh), bk, 1, 1, tbl_dev(it->table),
-                                                                flags + 1, work, ctx->upsert_all));
-                    return FBK_OK;
-                }, &ms);
-                if (st) break;
-                if (ms < best) {
-                    best = ms;
-                    best_u = sh;
-                }
+        st = tune_shapes([&](int bl, int ps, int* kept) -> fbk_status {
+            const Shape sh{bl, ps ? ps * ctx->num_sms : 0, 0};
+            TIMED(ctx, "table_init", launch_table_init(B->nw, launch_cfg(ctx, 256, 0), tbl_dev(it->table)));
+            cudaError_t e = cudaMemsetAsync(it->table->cnt, 0, it->table->cap * 32, ctx->stream);
+            if (e == cudaSuccess) e = cudaMemsetAsync(flags, 0, 24, ctx->stream);
+            if (e != cudaSuccess) return cuda_err(ctx, e, "batch autotuner");
+            float ms = 0;
+            fbk_status s3 = timed([&]() -> fbk_status {
+                TIMED(ctx, "tune_upsert", launch_upsert_all(B->nw, shape_launch(ctx, sh), bk, 1, 1, tbl_dev(it->table),
+                                                            flags + 1, work, ctx->upsert_all));
+                return FBK_OK;
+            }, &ms);
+            if (s3) return s3;
+            if (!*kept) *kept = bl;
+            if (ms < best) {
+                best = ms;
+                best_u = sh;
+                *kept = bl;
             }
+            return FBK_OK;
+        });
         if (st == FBK_OK) B->upsert = best_u;
     }
     cudaStreamSynchronize(ctx->stream);
@@ -479,10 +506,7 @@ fbk_status phase_a(fbk_batch* B, const std::vector<BatchIso*>& W) {
         if (!(it->cnt || it->lad) || !it->hll12 || (!B->ladder && !it->bm)) return set_err(ctx, FBK_ERR_OOM, "batch sketches");
     }
     if (B->p.autotune && !B->tuned) {
-        BatchIso* big = *std::max_element(W.begin(), W.end(), [](const BatchIso* a, const BatchIso* b) {
-            return a->bank->n_bases < b->bank->n_bases;
-        });
-        fbk_status st = autotune(B, big);
+        fbk_status st = autotune(B, W[tune_pick(W)]);
         if (st) return st;
     }
     WaveBufs w;
@@ -713,7 +737,8 @@ fbk_status phase_b(fbk_batch* B, const std::vector<BatchIso*>& V) {
         if (!work.p) return set_err(ctx, FBK_ERR_OOM, "batch upsert counters");
     }
     if (B->p.autotune && B->ladder && !B->tuned_b) {
-        st = autotune_b(B, V[0], work.p != nullptr && !flt[0].cnt);
+        const size_t j = tune_pick(V);
+        st = autotune_b(B, V[j], work.p != nullptr && !flt[j].cnt);
         if (st) return st;
     }
     const int eform = B->emit_form ? B->emit_form : emit_form(ctx, B->nw);
