@@ -52,13 +52,16 @@ __device__ __forceinline__ uint64_t run_pack(uint64_t off, uint32_t n, bool left
 struct MinPlan {
     uint32_t m, w, skip;
 };
-// m = 15 (k >= 29) or about k / 2, so that a 5-12 Mbp genome repeats few m-mers by chance;
+// m: short enough that a window has many of them (long runs: fewer to log, count and scatter),
+// long enough that a genome repeats few by chance, as a minimizer's places all go to one bin.
+// At 5 and 12 Mbp (5 Mbp, 100x, whole build): k = 21, m = 9 13.2 ms, 10 12.5, 11 12.6, 12 12.9;
+// k = 25, m = 11 12.3, 12 12.4, 14 12.7; k = 31, m = 13 12.5, 15 12.6; k = 45 the same for both.
 // w at most 32: runs of about (w + 1) / 2 windows, short enough that the keys of one
 // minimizer stay a small part of a group (at k = 77 and 100x about 15 distinct k-mers per
 // genome position, 240 per minimizer of a group of 1700).
 MinPlan min_plan(uint32_t k) {
     MinPlan p;
-    p.m = k >= 29 ? 15 : (k + 3) / 2;
+    p.m = k >= 40 ? 15 : std::min(13u, std::max(10u, (k - 3) / 2));
     const uint32_t full = k - p.m + 1;
     p.w = full <= 32 ? full : 32 - ((full ^ 32u) & 1u);
     p.skip = (full - p.w) / 2;
