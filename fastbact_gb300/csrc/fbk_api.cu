@@ -1681,7 +1681,7 @@ static fbk_status build_front_ladder(fbk_ctx* ctx, const fbk_bank* b, const fbk_
         uint64_t* kb = nullptr;
         fbk_status st = make_keep_bits(ctx, b, ss, &kb);
         bool declined = false;
-        if (st == FBK_OK) st = bins_build(ctx, b, p, kb, log2w, out, &declined);
+        if (st == FBK_OK) st = bins_build(ctx, b, p, kb, log2w, nullptr, out, &declined);
         cudaStreamSynchronize(ctx->stream);
         dev_free(ctx, kb);
         if (st != FBK_ERR_OOM && (st || !declined)) return st;  // short of memory: the buckets may need less
@@ -1748,6 +1748,20 @@ FBK_API fbk_status fbk_build_front(fbk_ctx* ctx, const fbk_bank* b, const fbk_bu
     uint64_t* keep = nullptr;
     fbk_bank* cb = nullptr;
     st = make_keep_bits(ctx, b, ss, &keep);
+    if (st == FBK_OK && n_contigs == 0 && ctx->sketch_mode == 1 && nw_of(p->key_bits) && p->k <= max_k_of(p->key_bits) &&
+        bins_applicable(ctx, b, p, log2w)) {
+        bool declined = false;
+        st = bins_build(ctx, b, p, keep, log2w, cms, out, &declined);
+        if (st == FBK_ERR_OOM || (st == FBK_OK && declined)) {
+            st = fbk_cms_clear(cms);  // short of memory: the buckets may need less
+        } else {
+            cudaStreamSynchronize(ctx->stream);
+            dev_free(ctx, keep);
+            if (st == FBK_OK && cms_out) *cms_out = cms;
+            else fbk_cms_release(cms);
+            return st;
+        }
+    }
     if (st == FBK_OK) st = contig_bank_opt(ctx, contig_ascii, contig_offs, n_contigs, &cb);
     if (st == FBK_OK) st = pass1_impl(cms, b, p->k, p->key_bits, keep, 1);
     if (st == FBK_OK && cb) st = pass1_impl(cms, cb, p->k, p->key_bits, nullptr, 10);

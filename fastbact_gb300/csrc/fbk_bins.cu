@@ -361,11 +361,14 @@ struct AggArgs {
     FirstKey* firsts;            // AGG_FIRST: the keys (cap_rows of them)
     uint32_t* first;             // and the estimator's first touches, 4 rows of 2^log2w
     uint32_t log2w;
+    uint32_t* counts;            // AGG_COUNT: the sketch's counters, 4 rows of 2^log2w
+    uint32_t* hll12;             // and its p = 12 registers
 };
 
-// What a launch of k_bin_agg is for: the accumulator rows; the same counts of a part of the
+// What a launch of k_bin_agg is for: the accumulator rows; the same, and the occurrences of the
+// keys seen twice or more into a sketch that the caller keeps; the counts of a part of the
 // bins, for the sizes; or the first two places of every key (the estimator's).
-enum { AGG_BUILD, AGG_SAMPLE, AGG_FIRST };
+enum { AGG_BUILD, AGG_COUNT, AGG_SAMPLE, AGG_FIRST };
 
 constexpr int AGG_THREADS = 512;
 constexpr uint32_t AGG_SMEM = 113000;  // two blocks an SM (228 KB, 1 KB reserved a block)
@@ -385,6 +388,10 @@ __host__ __device__ constexpr uint32_t agg_entries(int nk, bool wide) {
     return (AGG_SMEM - AGG_QUEUE * (AGG_THREADS / 32)) / (8u * nk + (wide ? 36u : 20u) + 8u) & ~127u;
 }
 
+// AGG_COUNT: one word more, the windows that add nothing to the key's first side.
+__host__ __device__ constexpr uint32_t count_entries(int nk, bool wide) {
+    return (AGG_SMEM - AGG_QUEUE * (AGG_THREADS / 32)) / (8u * nk + (wide ? 40u : 24u) + 8u) & ~127u;
+}
 // AGG_FIRST: the key words, its two places and the two slots.
 __host__ __device__ constexpr uint32_t first_entries(int nk) {
     return (AGG_SMEM - AGG_QUEUE * (AGG_THREADS / 32)) / (8u * nk + 16u) & ~127u;
@@ -439,6 +446,20 @@ __device__ __forceinline__ uint32_t sh_min(uint32_t a, uint32_t v) {
 }
 __device__ __forceinline__ uint32_t first_of(bool a, bool b, bool c, bool d) { return a ? 0u : b ? 1u : c ? 2u : d ? 3u : 4u; }
 
+// n occurrences of a key into a sketch that the caller keeps, as its pass 1 adds them (the
+// counters are sums, so a key's occurrences may come at once; the registers see the same keys).
+// 1 Mbp at 50x, k = 31, 2^22 columns: the build with its sketch 2.7 ms over occurrences and
+// records, 1.5 so.
+__device__ __forceinline__ void count_key(uint32_t* counts, uint32_t log2w, uint32_t* hll12, uint64_t fold, uint32_t n) {
+#pragma unroll
+    for (int row = 0; row < 4; ++row) atomicAdd(counts + cms_index(fold, row, log2w), n);
+    const uint64_t h = smix(fold ^ cms_seed(0));
+    if (h & (PASS1_HLL_SAMPLE - 1)) return;
+    uint32_t idx, rho;
+    hll_idx_rho(h, 12, idx, rho);
+    if (__ldca(hll12 + idx) < rho) atomicMax(hll12 + idx, rho);
+}
+
 // A block barrier that every lane of a warp reaches together (loops whose lanes leave at
 // different turns come right before it).
 __device__ __forceinline__ void block_sync() {
@@ -467,7 +488,7 @@ __device__ __forceinline__ void block_sync() {
 template <int NW, int WS, int MODE>
 __global__ void __launch_bounds__(AGG_THREADS, 2) k_bin_agg(AggArgs A) {
     constexpr int NK = NW - WS;
-    constexpr bool SAMPLE = MODE == AGG_SAMPLE, FIRST = MODE == AGG_FIRST;
+    constexpr bool SAMPLE = MODE == AGG_SAMPLE, FIRST = MODE == AGG_FIRST, COUNT = MODE == AGG_COUNT;
     extern __shared__ __align__(16) uint64_t agg_smem[];
     __shared__ uint32_t s_full, s_runs, s_entries, s_later, s_warp[AGG_THREADS / 32], s_alone[agg_entries(1, false) / 32];
     __shared__ unsigned long long s_base, s_low_base, s_next[3];  // next group, its bounds
@@ -498,10 +519,11 @@ __global__ void __launch_bounds__(AGG_THREADS, 2) k_bin_agg(AggArgs A) {
             continue;
         }
         if (SAMPLE && threadIdx.x == 0) atomicAdd(&A.counters[BC_WINDOWS], (unsigned long long)windows);
-        const uint32_t cap = FIRST ? first_entries(NK) : wide ? agg_entries(NK, true) : agg_entries(NK, false);
+        const uint32_t cap = FIRST ? first_entries(NK) : COUNT ? (wide ? count_entries(NK, true) : count_entries(NK, false))
+                                                     : wide ? agg_entries(NK, true) : agg_entries(NK, false);
         const uint32_t cl = FIRST ? 0u : wide ? 3u : 2u;  // log2(words of counts per entry)
         const uint32_t n_buckets = cap / 2;
-        const uint32_t ekey = sh_addr(agg_smem) + AGG_QUEUE * (AGG_THREADS / 32), ecnt = ekey + 8 * NK * cap, epos = ecnt + ((4 * cap) << cl), slots = epos + 4 * cap;
+        const uint32_t ekey = sh_addr(agg_smem) + AGG_QUEUE * (AGG_THREADS / 32), ecnt = ekey + 8 * NK * cap, epos = ecnt + ((4 * cap) << cl), elack = epos + 4 * cap, slots = elack + (COUNT ? 4 * cap : 0);
         auto window_hash = [&](Window<NK>& w, uint32_t g) {
             window_at<NK>(d32, g, k, w.key, w.rc, w.left, w.right);
             w.fold = fold_of<NK>(w.key);
@@ -526,6 +548,7 @@ __global__ void __launch_bounds__(AGG_THREADS, 2) k_bin_agg(AggArgs A) {
             const uint32_t r4 = w.rc ? 4u : 0u, eu = w.right + r4, ev = (w.left ^ 3u) + (r4 ^ 4u);
             sh_add_if(on && has_r, c + 4 * (eu >> nr), 1u << ((eu & nr) << 4));
             sh_add_if(on && has_l, c + 4 * (ev >> nr), 1u << ((ev & nr) << 4));
+            if constexpr (COUNT) sh_add_if(on && !(w.rc ? has_l : has_r), elack + 4 * entry, 1);
         };
         uint64_t lo = 0, width = 1ULL << 32;  // the part of the hash range being counted
         const uint64_t* src = A.runs + e0;    // the group's runs, or the windows put off
@@ -686,6 +709,7 @@ __global__ void __launch_bounds__(AGG_THREADS, 2) k_bin_agg(AggArgs A) {
                                         sh_zero128(ecnt + ((4 * at) << cl));
                                         if (wide) sh_zero128(ecnt + 32 * at + 16);
                                         sh_st(epos + 4 * at, g + 1);
+                                        if constexpr (COUNT) sh_st(elack + 4 * at, 0);
                                     }
                                 } else {
                                     put_off = true;
@@ -789,6 +813,13 @@ __global__ void __launch_bounds__(AGG_THREADS, 2) k_bin_agg(AggArgs A) {
                     if (!SAMPLE) atomicOr(&A.single[(pos - 1) >> 5], 1u << ((pos - 1) & 31));
                     continue;
                 }
+                if constexpr (COUNT) {
+                    // the windows of the key: those on its first side and those that are not
+                    uint64_t f = 0;
+#pragma unroll
+                    for (int q = 0; q < NK; ++q) f ^= sh_ld64(ekey + 8 * (i * NK + q));
+                    count_key(A.counts, A.log2w, A.hll12, f, a + sh_ld(elack + 4 * i));
+                }
                 uint32_t m = 0;
 #pragma unroll
                 for (int q = 0; q < 8; ++q) m = max(m, e[q]);
@@ -885,13 +916,16 @@ __global__ void __launch_bounds__(AGG_THREADS, 2) k_bin_agg(AggArgs A) {
 // for the top level; CLIMB reads the top first, which is small and saves the atomics of the
 // counters that are there already.  Pairs: the two levels of a counter side by side, so that
 // one atomic answers for both and nothing is read first.
+// Or, where the caller keeps the sketch, its counters themselves.
 struct LadderDev {
     uint32_t* bits;
     uint32_t log2w, planes;
     uint64_t top_off;  // words from a counter's first level to its top level
+    uint32_t* counts;  // not null: the counters, and no ladder
+    uint32_t* hll12;
 };
 LadderDev ladder_layout(uint32_t* bits, uint32_t log2w, bool planes) {
-    return {bits, log2w, planes ? 1u : 0u, planes ? (4ULL << log2w) >> 5 : 0ULL};
+    return {bits, log2w, planes ? 1u : 0u, planes ? (4ULL << log2w) >> 5 : 0ULL, nullptr, nullptr};
 }
 struct LadderBits {
     uint32_t wd[4], mk[4];  // word and bit of the first level in the four rows
@@ -910,6 +944,12 @@ __device__ __forceinline__ void ladder_bits(uint64_t fold, const LadderDev& L, L
 __device__ __forceinline__ uint32_t top_bit(const LadderDev& L, uint32_t mk) { return mk << (1 - L.planes); }
 // Whether the key passes the gate: the top level is set in all four rows.
 __device__ __forceinline__ bool ladder_solid(const LadderDev& L, uint64_t fold) {
+    if (L.counts) {
+        uint32_t c[4];
+#pragma unroll
+        for (int row = 0; row < 4; ++row) c[row] = __ldcg(L.counts + cms_index(fold, row, L.log2w));
+        return min(min(c[0], c[1]), min(c[2], c[3])) >= 2;
+    }
     LadderBits b;
     ladder_bits(fold, L, b);
     uint32_t w[4];
@@ -1053,6 +1093,8 @@ __global__ void __launch_bounds__(256) k_singles(const uint64_t* __restrict__ da
                 }
             } else if (MODE == SINGLES_GATE) {
                 if (ladder_solid(L, fold_of<NW - WS>(key))) atomicOr(&s_pass[warp][at >> 5], 1u << (at & 31));
+            } else if (L.counts) {
+                count_key(L.counts, L.log2w, L.hll12, fold_of<NW - WS>(key), 1);
             } else {
                 LadderBits b;
                 ladder_bits(fold_of<NW - WS>(key), L, b);
@@ -1354,7 +1396,7 @@ uint64_t group_windows(uint32_t entries, uint64_t n_windows, uint64_t distinct) 
 
 }  // namespace
 
-fbk_status bins_build(fbk_ctx* ctx, const fbk_bank* b, const fbk_build_params* p, const uint64_t* keep_bits, uint32_t log2w,
+fbk_status bins_build(fbk_ctx* ctx, const fbk_bank* b, const fbk_build_params* p, const uint64_t* keep_bits, uint32_t log2w, fbk_cms* cms,
                       fbk_table** out, bool* declined) {
     *declined = false;
     if (p->min_trans_cov > 0xFFFF) return set_err(ctx, FBK_ERR_INVALID, "thresholds must fit u16");
@@ -1371,7 +1413,7 @@ fbk_status bins_build(fbk_ctx* ctx, const fbk_bank* b, const fbk_build_params* p
     const uint32_t F = R.F;
     // one cleared block: the ladder, the bin and build counters, the windows' bitmaps
     const uint64_t bm_words = (b->n_words + 63) & ~63ULL;
-    const uint64_t lad_bytes = (2 * (4ULL << log2w) / 8 + 255) & ~255ULL;
+    const uint64_t lad_bytes = cms ? 0 : (2 * (4ULL << log2w) / 8 + 255) & ~255ULL;
     const uint64_t clear_bytes = lad_bytes + 8ULL * F + 8 * 16 + 2 * 4 * bm_words;
     static_assert(BC_N <= 16, "build counters");
     char* cleared = (char*)B.get(clear_bytes);
@@ -1412,7 +1454,8 @@ fbk_status bins_build(fbk_ctx* ctx, const fbk_bank* b, const fbk_build_params* p
         filter = may_filter && acc_filter_on(ctx->acc_filter, nw, distinct, n_windows);
     }
     // groups that about fill 0.7 of the entries, with few enough windows for 16-bit counts
-    const uint64_t target = sampled ? group_windows(agg_entries(nk, false), n_windows, distinct) : BINS_SMALL_GROUP;
+    const uint64_t target =
+        sampled ? group_windows(cms ? count_entries(nk, false) : agg_entries(nk, false), n_windows, distinct) : BINS_SMALL_GROUP;
     const uint32_t n_groups = (uint32_t)(n_windows / target + 1);
     unsigned long long* start = (unsigned long long*)B.get(8ULL * (n_groups + 1));
     if (!start) return set_err(ctx, FBK_ERR_OOM, "minimizer bins: groups");
@@ -1432,7 +1475,13 @@ fbk_status bins_build(fbk_ctx* ctx, const fbk_bank* b, const fbk_build_params* p
             delete t;
         }
     } guard{tb};
-    uint64_t rows = (filter ? kept : distinct) + 1, lows = filter ? multi + 1 : 0;
+    // (a sketch that the caller keeps takes the low keys where they are counted)
+    uint64_t rows = (filter ? kept : distinct) + 1, lows = filter && !cms ? multi + 1 : 0;
+    if (cms) {
+        A.counts = cms->cnt;
+        A.hll12 = cms->hll12;
+        A.log2w = log2w;
+    }
     uint64_t* low = nullptr;
     for (int attempt = 0;; ++attempt) {
         // a table of the rows alone: every slot that is read is one, no probing
@@ -1459,7 +1508,8 @@ fbk_status bins_build(fbk_ctx* ctx, const fbk_bank* b, const fbk_build_params* p
               (k_bin_groups<<<std::min<unsigned>(1024, (F + 256) / 256), 256, 0, stream>>>(pre, F, (uint32_t)target, n_groups, start),
                cudaGetLastError()));
         TIMED(ctx, "bins_aggregate", by_width(nw, k, [&](auto a, auto w) {
-                  return agg_launch<decltype(a)::value, decltype(w)::value, AGG_BUILD>(stream, sms, A);
+                  constexpr int NW = decltype(a)::value, WS = decltype(w)::value;
+                  return cms ? agg_launch<NW, WS, AGG_COUNT>(stream, sms, A) : agg_launch<NW, WS, AGG_BUILD>(stream, sms, A);
               }));
         CK(ctx, cudaMemcpyAsync(h, counters, 8 * BC_N, cudaMemcpyDeviceToHost, stream));
         CK(ctx, cudaMemcpyAsync(h + BC_N, ctx->d_status, 4, cudaMemcpyDeviceToHost, stream));
@@ -1467,20 +1517,25 @@ fbk_status bins_build(fbk_ctx* ctx, const fbk_bank* b, const fbk_build_params* p
         if ((uint32_t)h[BC_N] & ST_SPIN_TIMEOUT) return set_err(ctx, FBK_ERR_TIMEOUT, "minimizer bins: a bounded search gave up");
         if ((uint32_t)h[BC_N] & ST_TABLE_FULL) return set_err(ctx, FBK_ERR_TABLE_FULL, "minimizer bins: a group did not fit");
         const uint64_t need = h[BC_ROWS] + (filter ? 0 : h[BC_SINGLES]);
-        if (need <= rows && h[BC_LOW] <= lows) break;
+        if (need <= rows && (cms || h[BC_LOW] <= lows)) break;
         // the sample's estimate was low: again with the counted sizes
         if (attempt == 1) return set_err(ctx, FBK_ERR_TABLE_FULL, "minimizer bins: row counts changed between runs");
         tbl_free_storage(tb);
         if (low) B.drop(low);
         rows = need + 1;
-        lows = filter ? h[BC_LOW] + 1 : 0;
+        lows = filter && !cms ? h[BC_LOW] + 1 : 0;
+        if (cms) {
+            fbk_status st = fbk_cms_clear(cms);
+            if (st) return st;
+        }
         CK(ctx, cudaMemsetAsync(counters, 0, 8 * BC_N, stream));
         CK(ctx, cudaMemsetAsync(single, 0, 4 * bm_words, stream));
     }
-    const uint64_t n_rows = h[BC_ROWS], n_low = h[BC_LOW], n_singles = h[BC_SINGLES];
+    const uint64_t n_rows = h[BC_ROWS], n_low = cms ? 0 : h[BC_LOW], n_singles = h[BC_SINGLES];
     const TableDev td = tbl_dev(tb);
     const SingleMaps maps{valid, single, pass, b->n_words};
-    const LadderDev ladder = ladder_layout(lad, log2w, n_singles > 2ULL << log2w);
+    LadderDev ladder = ladder_layout(lad, log2w, n_singles > 2ULL << log2w);
+    if (cms) ladder.counts = cms->cnt, ladder.hll12 = cms->hll12;
     auto singles = [&](int mode) {
         return by_width(nw, k, [&](auto a, auto w) {
             constexpr int NW = decltype(a)::value, WS = decltype(w)::value;
@@ -1490,14 +1545,16 @@ fbk_status bins_build(fbk_ctx* ctx, const fbk_bank* b, const fbk_build_params* p
         });
     };
     TIMED(ctx, "bins_valid", stream_launch(stream, sms, b->n_reads, k_bin_valid, bv, k, valid));
-    TIMED(ctx, "bins_sketch", by_width(nw, k, [&](auto a, auto w) {
-              constexpr int NW = decltype(a)::value, NK = NW - decltype(w)::value;
-              return stream_launch(stream, sms, n_rows, k_bin_sketch<NW, NK>, (const uint64_t*)td.keys, n_rows, ladder);
-          }));
-    TIMED(ctx, "bins_sketch", by_width(nw, k, [&](auto a, auto w) {
-              constexpr int NK = decltype(a)::value - decltype(w)::value;
-              return stream_launch(stream, sms, n_low, k_bin_sketch<NK, NK>, (const uint64_t*)low, n_low, ladder);
-          }));
+    if (!cms) {
+        TIMED(ctx, "bins_sketch", by_width(nw, k, [&](auto a, auto w) {
+                  constexpr int NW = decltype(a)::value, NK = NW - decltype(w)::value;
+                  return stream_launch(stream, sms, n_rows, k_bin_sketch<NW, NK>, (const uint64_t*)td.keys, n_rows, ladder);
+              }));
+        TIMED(ctx, "bins_sketch", by_width(nw, k, [&](auto a, auto w) {
+                  constexpr int NK = decltype(a)::value - decltype(w)::value;
+                  return stream_launch(stream, sms, n_low, k_bin_sketch<NK, NK>, (const uint64_t*)low, n_low, ladder);
+              }));
+    }
     TIMED(ctx, "bins_singles", singles(SINGLES_CLIMB));
     TIMED(ctx, "bins_singles_gate", singles(SINGLES_GATE));
     TIMED(ctx, "bins_gate", by_width(nw, k, [&](auto a, auto w) {
@@ -1517,6 +1574,7 @@ fbk_status bins_build(fbk_ctx* ctx, const fbk_bank* b, const fbk_build_params* p
     tb->out_mask = (uint8_t*)dev_alloc(ctx, oc);
     if (!tb->out_keys || !tb->out_cov || !tb->out_mask) return set_err(ctx, FBK_ERR_OOM, "solid table output");
     tb->out_cap = oc;
+    if (cms) TIMED(ctx, "cms_clamp", launch_clamp_counters(launch_cfg(ctx, 256, 0), cms->cnt, cms->n));
     fbk_status st = tbl_convert(tb);
     if (st) return st;
     // the pushes of the keys that the filter left out

@@ -11,7 +11,7 @@ import numpy as np
 import pytest
 
 from fastbact_gb300 import api
-from test_gpu_parity import compare_gate_only, rand_seqs
+from test_gpu_parity import compare_build, compare_gate_only, rand_seqs
 
 pytestmark = pytest.mark.gpu
 
@@ -94,6 +94,31 @@ def test_sampled_sizes(ctx, k):
     bank = api.synth_isolate(p, threads=0, sample_pairs=0)[0]
     assert sum(int(np.maximum(a.lengths.astype(np.int64) - k + 1, 0).sum()) for a in bank.arenas) > 4 << 20
     compare_gate_only(ctx, bank, k, api.key_bits_for_k(k), 16, None, 18)
+
+
+@pytest.mark.parametrize("k,kb", [(17, 64), (31, 64), (32, 128), (63, 128), (77, 256), (99, 256), (127, 256)])
+@pytest.mark.parametrize("acc_filter", [0, 2])
+def test_kept_sketch(k, kb, acc_filter):
+    """A build that returns its sketch: every counter, and the rows that it gates, with windows
+    that have a neighbour on one side or none, counts beyond 65535 and keys of every fate; and
+    a second build on that sketch (its distinct count sizes the table)."""
+    seqs = rand_seqs(31, 300, k, 3 * k) + rand_seqs(32, 60, k, k + 1) + [b"A" * 3000] * 25 + [b"T" * 900] * 3 + [b"ACG" * 900] * 50
+    seqs += [rc(s) for s in seqs[::3]] + [s[1:] for s in seqs[:300:4]] + [s[:-2] for s in seqs[:300:5]] + seqs[:60]
+    bank = bank_of([seqs[i] for i in np.random.default_rng(k).permutation(len(seqs))])
+    caps = []
+    for form in (1, 0):
+        c = api.Context(0)
+        try:
+            c.set_tuning(acc_filter=acc_filter, build_form=form)
+            for cb, log2w in ((16, 16), (4, 10)):
+                compare_build(c, bank, k, kb, cb, None, log2w)
+            d = api.DeviceBank(c, bank)
+            _, cms = api.build_cdbg_with_contigs_ext(d, [], k, None, None, ctx=c, key_bits=kb, counter_bits=16, cms_log2_width=16, keep_cms=True)
+            t = api.solid_build(c, d, cms, k)
+            caps.append((t.info(), t.digest()))
+        finally:
+            c.close()
+    assert caps[0] == caps[1]
 
 
 def test_overlapping_reads():
