@@ -13,6 +13,8 @@
 //      multi-isolate launch each — and the SolidKmerNode conversion per isolate;
 //   5. isolates whose buckets or table overflowed are redone by the
 //      single-isolate path, which grows what overflowed.
+// Isolates that fill the device by themselves are built one after the other over minimizer
+// bins instead of 2 to 4 (takes_bins).
 // Each phase can run as one CUDA graph (captured on the context's stream).
 #include <algorithm>
 #include <chrono>
@@ -652,6 +654,17 @@ void release_b(fbk_batch* B, BatchIso* it) {
 
 void finish_iso(fbk_batch* B, BatchIso* it);
 
+fbk_build_params iso_params(const fbk_batch* B) {
+    fbk_build_params bp{};
+    bp.k = B->p.k;
+    bp.key_bits = B->p.key_bits;
+    bp.cms_log2_width = B->p.cms_log2_width;
+    bp.counter_bits = B->p.counter_bits;
+    bp.t_solid = B->p.t_solid;
+    bp.min_trans_cov = B->p.min_trans_cov;
+    return bp;
+}
+
 // The single-isolate path for an isolate whose wave buckets or table overflowed.
 fbk_status fallback(fbk_batch* B, BatchIso* it) {
     fbk_ctx* ctx = B->ctx;
@@ -662,13 +675,7 @@ fbk_status fallback(fbk_batch* B, BatchIso* it) {
     view.log2w = B->p.cms_log2_width;
     view.cbits = B->p.counter_bits;
     view.n = 4ULL << view.log2w;
-    fbk_build_params bp{};
-    bp.k = B->p.k;
-    bp.key_bits = B->p.key_bits;
-    bp.cms_log2_width = B->p.cms_log2_width;
-    bp.counter_bits = B->p.counter_bits;
-    bp.t_solid = B->p.t_solid;
-    bp.min_trans_cov = B->p.min_trans_cov;
+    const fbk_build_params bp = iso_params(B);
     fbk_status st = B->ladder ? solid_build_ladder(ctx, it->bank, it->lad, B->p.cms_log2_width, &bp, it->keep, it->distinct * 2, &it->table)
                               : solid_build(ctx, it->bank, &view, &bp, it->keep, it->distinct * 2, &it->table);
     view.cnt = nullptr;
@@ -902,6 +909,69 @@ fbk_status drain_b(fbk_batch* B, const std::vector<BatchIso*>& W) {
     return FBK_OK;
 }
 
+// Isolates of this many kept k-mers and more fill the device by themselves: they gain nothing
+// from sharing launches, and the single build over minimizer bins takes less time for them
+// than their share of a wave (six isolates of 5 to 60 M k-mers: phases A and B 8.7 ms and
+// 7.3 ms of tuning, the builds 6.3 ms).  Below it a build's own launches and waits for the host
+// (0.13 ms) weigh more.
+constexpr uint64_t BATCH_BINS_FROM = 8u << 20;
+
+// A limit on a wave's bytes, a kept sketch, or a pass-1 form asked for keeps an isolate in the
+// waves.
+bool takes_bins(const fbk_batch* B, const BatchIso* it) {
+    const fbk_build_params bp = iso_params(B);
+    return B->ladder && !B->p.max_wave_bytes && !B->ctx->batch_pass1 && bins_applicable(B->ctx, it->bank, &bp, B->p.cms_log2_width) &&
+           (double)it->bank->windows(B->p.k, B->p.k) * std::min(1.0, it->res.subsample_factor) >= (double)BATCH_BINS_FROM;
+}
+
+// Builds the isolates of W one after the other over minimizer bins; those that the bins decline
+// or have no memory for go to rest.
+fbk_status bins_wave(fbk_batch* B, const std::vector<BatchIso*>& W, std::vector<BatchIso*>& rest) {
+    fbk_ctx* ctx = B->ctx;
+    const uint32_t n = (uint32_t)W.size();
+    std::vector<unsigned long long> counts;
+    {
+        WaveBufs w;
+        fbk_status st = wave_bufs(B, n, false, w);
+        if (st == FBK_OK) st = upload_wave(B, W, w);
+        if (st) return st;
+        st = run_phase(B, &B->stats.ms_phase_a, [&]() -> fbk_status {
+            CK(ctx, cudaMemsetAsync(w.cnt, 0, (uint64_t)n * 64, ctx->stream));
+            TIMED(ctx, "batch_count", launch_batch_count(shape_launch(ctx, B->solid), w.iso, w.rb, n, B->p.k));
+            return FBK_OK;
+        });
+        if (st == FBK_OK) st = stage(B, (uint64_t)n * 64);
+        if (st) return st;
+        CK(ctx, cudaMemcpyAsync(B->h_stage, w.cnt, (uint64_t)n * 64, cudaMemcpyDeviceToHost, ctx->stream));
+        CK(ctx, cudaStreamSynchronize(ctx->stream));
+        const unsigned long long* hc = (const unsigned long long*)B->h_stage;
+        counts.assign(hc, hc + 8ULL * n);
+    }
+    const fbk_build_params bp = iso_params(B);
+    for (uint32_t i = 0; i < n; ++i) {
+        BatchIso* it = W[i];
+        bool declined = false;
+        float ms = 0.f;
+        CK(ctx, cudaEventRecord(B->ev[0], ctx->stream));
+        const fbk_status st = bins_build(ctx, it->bank, &bp, it->keep, B->p.cms_log2_width, nullptr, &it->table, &declined);
+        if (st == FBK_ERR_OOM || (st == FBK_OK && declined)) {
+            ctx->err.clear();
+            rest.push_back(it);
+            continue;
+        }
+        if (st) return st;
+        CK(ctx, cudaEventRecord(B->ev[1], ctx->stream));
+        CK(ctx, cudaEventSynchronize(B->ev[1]));
+        CK(ctx, cudaEventElapsedTime(&ms, B->ev[0], B->ev[1]));
+        B->stats.ms_phase_b += ms;
+        it->res.kmers = counts[8 * i + 1] + counts[8 * i + 2];
+        it->res.wave = (int32_t)B->stats.waves;
+        finish_iso(B, it);
+    }
+    B->stats.waves++;
+    return FBK_OK;
+}
+
 fbk_status run_impl(fbk_batch* B) {
     fbk_ctx* ctx = B->ctx;
     CK(ctx, cudaSetDevice(ctx->device));
@@ -922,10 +992,19 @@ fbk_status run_impl(fbk_batch* B) {
         cudaEventElapsedTime(&t, B->ev[0], B->ev[1]);
         B->stats.ms_estimate += t;
     }
-    std::vector<BatchIso*> todo;
+    std::vector<BatchIso*> todo, large;
     for (auto& up : B->isos)
-        if (up->res.state == 1) todo.push_back(up.get());
+        if (up->res.state == 1) (takes_bins(B, up.get()) ? large : todo).push_back(up.get());
     const uint32_t max_wave = std::max<uint32_t>(1, std::min<uint32_t>(BATCH_MAX_ISO, B->p.max_wave ? B->p.max_wave : 64));
+    for (size_t i = 0; i < large.size(); i += max_wave) {
+        const std::vector<BatchIso*> W(large.begin() + i, large.begin() + std::min<size_t>(i + max_wave, large.size()));
+        const fbk_status st = bins_wave(B, W, todo);
+        if (st) {
+            for (BatchIso* it : W)
+                if (it->res.state != 3) it->res.state = -1, it->res.status = st;
+            return st;
+        }
+    }
     size_t next = 0;
     while (next < todo.size()) {
         // phase-A wave: isolates whose sketches and bitmaps fill at most half of the

@@ -167,8 +167,8 @@ FBK_API fbk_status fbk_ctx_event_elapsed(fbk_ctx* ctx, int slot_a, int slot_b, d
  * 3 = 2 ahead over a flattened window stream, 4 = one lane per read with rolled k-mers
  * (the default), 5 = the same at two blocks per SM for every key width), "acc_filter"
  * (keys that cannot become SolidKmerNodes stay out of the table, see fbk_table_flags:
- * 0 never, 1 where it pays, 2 always), "build_form" (1, the default: builds that do not
- * return their sketch run over minimizer bins where those apply; 0: over record buckets, as
+ * 0 never, 1 where it pays, 2 always), "build_form" (1, the default: builds run over
+ * minimizer bins where those apply; 0: over record buckets, as
  * does every build of a context on which an option of the record buckets was set),
  * "upsert_all" (1: an unfiltered pass upserts every
  * bucket in one persistent launch), "upsert_queue" (1: filtered upserts queue the
@@ -506,7 +506,7 @@ typedef struct {
      * (pass1_rows 0: the ladder pass 1 runs as one single-isolate launch per isolate) */
     int32_t pass1_block, pass1_grid, pass1_rows, solid_block, solid_grid, solid_rows;
     int32_t emit_block, emit_grid, upsert_block, upsert_grid;
-    int32_t tuned;
+    int32_t tuned;      /* 0 while no isolate has needed a wave (large ones are built on their own) */
     int32_t emit_form;  /* record emit in use: 3 flat window stream, 4 one lane per read (rolled) */
     double tune_ms;
 } fbk_batch_stats;
