@@ -75,62 +75,93 @@ __device__ __forceinline__ uint32_t rev2_32(uint32_t x) {
 }
 
 constexpr int RUN_CHUNKS = 6;  // windows per tile: 6 x 32
+constexpr uint32_t RUN_QUEUE = 64;  // runs of a warp that wait for their bin, a power of two
 
-// One warp per read, lane = window.  The hashes of a tile's m-mers stay in registers (lane
-// j of chunk c holds m-mer 32 c + j); a sliding minimum over w of them takes log2(w) steps
-// of one shuffle each.  Bound by instruction issue: about 20 instructions per m-mer for
-// its hash, 3 per step of the minimum.
+// The hashes of up to 32 NC m-mers from base g0 on (lane j of chunk c has m-mer 32 c + j), and
+// the minimum over each w of them that follow one another: h[i] <- min of h[i .. i + 2^s), then
+// of the two windows of 2^s that cover w.  Lanes past the last m-mer repeat it: no window asks
+// for theirs.
+template <int NC>
+__device__ __forceinline__ void run_minima(const uint32_t* __restrict__ d32, uint32_t g0, uint32_t n_mers, uint32_t msh, uint32_t mmask,
+                                           uint32_t w, uint32_t (&out)[RUN_CHUNKS + 1]) {
+    const uint32_t lane = threadIdx.x & 31;
+    uint32_t h[NC];
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {
+        const uint32_t i = g0 + (c + 1 < NC ? 32 * c + lane : min(32 * c + lane, n_mers - 1));
+        const uint32_t x = __funnelshift_r(d32[i >> 4], d32[(i >> 4) + 1], (i & 15) << 1);
+        const uint32_t c0 = min(rev2_32(x) >> msh, ~x & mmask);
+        uint32_t z = (c0 ^ 0x3C6EF372u) * 0x9E3779B1u;
+        z ^= z >> 15;
+        h[c] = z * 0x85EBCA77u;
+    }
+    auto step = [&](uint32_t by) {
+        const uint32_t from = (lane + by) & 31;
+        const bool next = lane < by;
+#pragma unroll
+        for (int c = 0; c < NC; ++c) h[c] = min(h[c], __shfl_sync(0xffffffffu, next ? (c + 1 < NC ? h[c + 1 < NC ? c + 1 : c] : 0xFFFFFFFFu) : h[c], from));
+    };
+    uint32_t span = 1;
+    for (; 2 * span <= w; span *= 2) step(span);
+    if (w > span) step(w - span);
+#pragma unroll
+    for (int c = 0; c < NC; ++c) out[c] = h[c];
+}
+
+// One warp per read, lane = window; a sliding minimum over the w m-mers of a window takes
+// log2(w) steps of one shuffle each, with the read's hashes in registers.  Runs that end wait
+// in shared memory until there are 32, which are binned, counted and logged together: 2 runs
+// end in 32 windows at k of 46 and more.  Bound by instruction issue: about 25 instructions
+// per 32 m-mers for their hashes, 4 per step of the minimum, 40 for the ends of runs.
+// 5 Mbp at 100x, 500 M bases: k = 31 2.66 ms with a run binned by the lane that ends it and the
+// chunks counted at run time, 2.09 so, 1.98 with the next read's length and place loaded ahead;
+// k = 77 2.18, 1.73, 1.64.
 __global__ void __launch_bounds__(256) k_bin_runs(BankDev b, uint32_t k, MinPlan mp, uint32_t n_bins, uint64_t* __restrict__ log,
                                                   uint32_t* __restrict__ log_n, uint32_t cap_w, unsigned long long* __restrict__ hist,
                                                   unsigned long long* __restrict__ need) {
+    __shared__ uint4 s_queue[8][RUN_QUEUE];  // first base, windows | left << 12 | right << 13, minimizer
     const uint32_t lane = threadIdx.x & 31;
     const uint64_t gw = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
     const uint32_t* __restrict__ d32 = reinterpret_cast<const uint32_t*>(b.data);
     const uint32_t msh = 32 - 2 * mp.m, mmask = 0xFFFFFFFFu >> msh;
+    uint4* queue = s_queue[threadIdx.x >> 5];
     uint64_t* out = log + gw * cap_w;
-    uint32_t n_out = 0;  // warp-uniform
+    uint32_t n_out = 0, n_in = 0;  // warp-uniform: runs logged, runs ended
+    auto flush = [&](uint32_t n) {  // the n oldest of the queue
+        __syncwarp();
+        if (lane < n) {
+            const uint4 e = queue[(n_out + lane) % RUN_QUEUE];
+            const uint32_t windows = e.y & 0xFFFu;
+            const uint32_t z = e.z ^ (e.z >> 16);
+            const uint32_t bin = __umulhi(z * 0xC2B2AE3Du, n_bins);
+            if (n_out + lane < cap_w) out[n_out + lane] = run_pack(e.x, windows, (e.y >> 12) & 1u, (e.y >> 13) & 1u, bin);
+            atomicAdd(&hist[bin], (1ull << 32) | windows);
+        }
+        n_out += n;
+        __syncwarp();
+    };
+    uint32_t len_next = 0, off_next = 0;  // of the warp's next read, loaded ahead (the bank holds fewer than 2^32 bases)
+    if (b.r_begin + gw < b.r_end) len_next = b.len[b.r_begin + gw], off_next = (uint32_t)b.off[b.r_begin + gw];
     for (uint64_t r = b.r_begin + gw; r < b.r_end; r += nwarps) {
-        const uint32_t len = b.len[r];
+        const uint32_t len = len_next, off = off_next;
+        if (r + nwarps < b.r_end) len_next = b.len[r + nwarps], off_next = (uint32_t)b.off[r + nwarps];
         if (len < k || !bank_keep(b, r)) continue;
-        const uint64_t off = b.off[r];
         const uint32_t nk = len - k + 1;
         uint32_t start = 0, prev_min = 0;  // first window of the open run; minimizer of the last window seen
         for (uint32_t q0 = 0; q0 <= nk; q0 += 32 * RUN_CHUNKS) {
             const uint32_t n_mers = min(nk - q0, 32u * RUN_CHUNKS) + mp.w - 1;  // q0 == nk: no window left, only the end
-            const uint32_t g0 = (uint32_t)off + q0 + mp.skip;  // the bank holds fewer than 2^32 bases
+            const uint32_t g0 = off + q0 + mp.skip;
             uint32_t h[RUN_CHUNKS + 1];
-#pragma unroll
-            for (int c = 0; c <= RUN_CHUNKS; ++c) {
-                h[c] = 0xFFFFFFFFu;
-                if (32u * c < n_mers) {  // lanes past the last m-mer repeat it: no window asks for theirs
-                    const uint32_t i = g0 + min(32 * c + lane, n_mers - 1);
-                    const uint32_t x = __funnelshift_r(d32[i >> 4], d32[(i >> 4) + 1], (i & 15) << 1);
-                    const uint32_t c0 = min(rev2_32(x) >> msh, ~x & mmask);
-                    uint32_t z = (c0 ^ 0x3C6EF372u) * 0x9E3779B1u;
-                    z ^= z >> 15;
-                    h[c] = z * 0x85EBCA77u;
-                }
-            }
-            // h[i] <- min of h[i .. i + 2^s), then of the two windows of 2^s that cover w
-            uint32_t span = 1;
-            while (2 * span <= mp.w) {
-#pragma unroll
-                for (int c = 0; c <= RUN_CHUNKS; ++c) {
-                    if (32u * c >= n_mers) break;
-                    const uint32_t nx = c < RUN_CHUNKS ? h[c < RUN_CHUNKS ? c + 1 : c] : 0xFFFFFFFFu;
-                    h[c] = min(h[c], __shfl_sync(0xffffffffu, lane < span ? nx : h[c], (lane + span) & 31));
-                }
-                span *= 2;
-            }
-            const uint32_t rest = mp.w - span;
-            if (rest) {
-#pragma unroll
-                for (int c = 0; c <= RUN_CHUNKS; ++c) {
-                    if (32u * c >= n_mers) break;
-                    const uint32_t nx = c < RUN_CHUNKS ? h[c < RUN_CHUNKS ? c + 1 : c] : 0xFFFFFFFFu;
-                    h[c] = min(h[c], __shfl_sync(0xffffffffu, lane < rest ? nx : h[c], (lane + rest) & 31));
-                }
+            const uint32_t nc = (n_mers + 31) / 32;
+            switch (nc) {
+                case 1: run_minima<1>(d32, g0, n_mers, msh, mmask, mp.w, h); break;
+                case 2: run_minima<2>(d32, g0, n_mers, msh, mmask, mp.w, h); break;
+                case 3: run_minima<3>(d32, g0, n_mers, msh, mmask, mp.w, h); break;
+                case 4: run_minima<4>(d32, g0, n_mers, msh, mmask, mp.w, h); break;
+                case 5: run_minima<5>(d32, g0, n_mers, msh, mmask, mp.w, h); break;
+                case 6: run_minima<6>(d32, g0, n_mers, msh, mmask, mp.w, h); break;
+                default: run_minima<7>(d32, g0, n_mers, msh, mmask, mp.w, h); break;
             }
 #pragma unroll
             for (int c = 0; c < RUN_CHUNKS; ++c) {
@@ -145,18 +176,17 @@ __global__ void __launch_bounds__(256) k_bin_runs(BankDev b, uint32_t k, MinPlan
                 if (cut) {
                     const uint32_t below = mask & ((1u << lane) - 1);
                     const uint32_t s = below ? qc + 31 - __clz(below) : start;
-                    uint32_t z = before ^ (before >> 16);
-                    const uint32_t bin = __umulhi(z * 0xC2B2AE3Du, n_bins);
-                    const uint32_t at = n_out + __popc(below);
-                    if (at < cap_w) out[at] = run_pack(off + s, q - s, s > 0, q < nk, bin);
-                    atomicAdd(&hist[bin], (1ull << 32) | (q - s));
+                    queue[(n_in + __popc(below)) % RUN_QUEUE] =
+                        make_uint4(off + s, (q - s) | (s > 0 ? 1u << 12 : 0u) | (q < nk ? 1u << 13 : 0u), before, 0);
                 }
-                n_out += __popc(mask);
+                n_in += __popc(mask);
                 if (mask) start = qc + 31 - __clz(mask);
                 prev_min = __shfl_sync(0xffffffffu, h[c], 31);
+                if (n_in - n_out >= 32) flush(32);
             }
         }
     }
+    flush(n_in - n_out);
     if (lane == 0) {
         log_n[gw] = min(n_out, cap_w);
         if (n_out > cap_w) atomicMax(need, (unsigned long long)n_out);
