@@ -28,7 +28,16 @@
 // Why this shape: the occurrence-wise passes (fbk_k_ladder.cu, fbk_k_roll.cu, fbk_k_pass.cu)
 // spend 8 random L2 loads on the gate and a table probe and 2 L2 atomics per occurrence, and
 // an SM serves one such lane a cycle.  Shared memory serves 32 lanes in 3-4 cycles, and the
-// gate's loads fall on the distinct k-mers (4-10 times fewer at 100x).
+// gate's loads fall on the distinct k-mers (4-10 times fewer at 100x).  Device time at 5 Mbp
+// and 100x (485 M bases; 418 / 373 / 305 / 232 M windows), 2^24 columns, 0.5% errors:
+//   k                     21     33     55     77
+//   over occurrences    20.4   23.3   20.8   21.3 ms
+//   here                11.9   13.1   11.6   11.8
+//     runs, scatter      3.4    2.6    1.9    1.9
+//     aggregate          5.2    5.8    6.2    6.3
+//     sketch, gate       2.2    2.7    2.9    3.2
+// The same entry takes a sketch that the caller keeps (AGG_COUNT) and the estimator's sample
+// loop (bins_first).
 #include <algorithm>
 #include <cmath>
 
@@ -99,7 +108,10 @@ __device__ __forceinline__ void run_minima(const uint32_t* __restrict__ d32, uin
         const uint32_t from = (lane + by) & 31;
         const bool next = lane < by;
 #pragma unroll
-        for (int c = 0; c < NC; ++c) h[c] = min(h[c], __shfl_sync(0xffffffffu, next ? (c + 1 < NC ? h[c + 1 < NC ? c + 1 : c] : 0xFFFFFFFFu) : h[c], from));
+        for (int c = 0; c < NC; ++c) {
+            const uint32_t nx = c + 1 < NC ? h[c + 1 < NC ? c + 1 : c] : 0xFFFFFFFFu;
+            h[c] = min(h[c], __shfl_sync(0xffffffffu, next ? nx : h[c], from));
+        }
     };
     uint32_t span = 1;
     for (; 2 * span <= w; span *= 2) step(span);
@@ -256,7 +268,9 @@ __global__ void __launch_bounds__(256) k_bin_scan(const unsigned long long* __re
 }
 
 // Moves every logged run to its bin's range.  One returning atomic and one 8-byte store per
-// run; the bins' open ends (8 MB of sectors at most) stay in L2 until full.
+// run; the bins' open ends (8 MB of sectors at most) stay in L2 until full.  Bound by the L2
+// (59% of its peak, DRAM 19%, issue 15%): 5 Mbp at 100x, 64 M runs of k = 21 1.4 ms, 14 M of
+// k = 77 0.27.  Eight runs a lane, or half and a quarter of the bins, took as long.
 __global__ void __launch_bounds__(256) k_bin_scatter(const uint64_t* __restrict__ log, const uint32_t* __restrict__ log_n, uint32_t cap_w,
                                                      uint32_t* __restrict__ cursor, uint64_t* __restrict__ runs, uint64_t cap) {
     const uint32_t lane = threadIdx.x & 31;
@@ -515,6 +529,10 @@ __device__ __forceinline__ void block_sync() {
 // queue of the warp and are resolved 32 at a time, so that the longer searches and the
 // entering of new keys run on full warps.  No lane waits for another: a new key's entry is
 // complete before its slot is.
+// 5 Mbp at 100x: 418 M windows of k = 21 5.2 ms, 232 M of k = 77 6.3 ms, where the records' emit,
+// count and upsert took 12.7 and 15.8.  Slots probed one at a time 6.1 and 11.4 ms, four at once
+// with keys in the slots 5.3 and 7.7, with entries of their own 6.5 and 6.3, and with the queue
+// as it is; 1, 3 or 4 blocks an SM and other fills within 5%.
 template <int NW, int WS, int MODE>
 __global__ void __launch_bounds__(AGG_THREADS, 2) k_bin_agg(AggArgs A) {
     constexpr int NK = NW - WS;
@@ -553,7 +571,8 @@ __global__ void __launch_bounds__(AGG_THREADS, 2) k_bin_agg(AggArgs A) {
                                                      : wide ? agg_entries(NK, true) : agg_entries(NK, false);
         const uint32_t cl = FIRST ? 0u : wide ? 3u : 2u;  // log2(words of counts per entry)
         const uint32_t n_buckets = cap / 2;
-        const uint32_t ekey = sh_addr(agg_smem) + AGG_QUEUE * (AGG_THREADS / 32), ecnt = ekey + 8 * NK * cap, epos = ecnt + ((4 * cap) << cl), elack = epos + 4 * cap, slots = elack + (COUNT ? 4 * cap : 0);
+        const uint32_t ekey = sh_addr(agg_smem) + AGG_QUEUE * (AGG_THREADS / 32), ecnt = ekey + 8 * NK * cap;
+        const uint32_t epos = ecnt + ((4 * cap) << cl), elack = epos + 4 * cap, slots = elack + (COUNT ? 4 * cap : 0);
         auto window_hash = [&](Window<NK>& w, uint32_t g) {
             window_at<NK>(d32, g, k, w.key, w.rc, w.left, w.right);
             w.fold = fold_of<NK>(w.key);
@@ -991,7 +1010,9 @@ __device__ __forceinline__ bool ladder_solid(const LadderDev& L, uint64_t fold) 
     return ok;
 }
 
-// Keys seen twice or more set their counters' top level.  Keys of STRIDE words, of which the
+// Keys seen twice or more set their counters' top level (at 100x about 11 M of them: 0.33 ms,
+// four random loads and as many atomics in L2 a key, where pass 1 went over every window: 6.5 ms
+// at k = 21, 4.6 at k = 77).  Keys of STRIDE words, of which the
 // last NK are read.
 template <int STRIDE, int NK>
 __global__ void __launch_bounds__(256) k_bin_sketch(const uint64_t* __restrict__ keys, uint64_t n, LadderDev L) {
@@ -1048,6 +1069,9 @@ enum { SINGLES_CLIMB, SINGLES_GATE, SINGLES_ROWS };
 //          already passes whatever else comes.
 //   GATE:  the others ask again once every key has been counted.
 //   ROWS:  those that pass next to a solid window become accumulator rows.
+// Bound by lanes into L2, four a key and mode (5 Mbp at 100x: CLIMB 1.2 and GATE 0.5 ms at k = 21,
+// 2.0 and 0.7 at k = 77).  Asking two rows of the gate first and the others only if those pass
+// took as long.
 template <int NW, int WS, int MODE>
 __global__ void __launch_bounds__(256) k_singles(const uint64_t* __restrict__ data, SingleMaps M, uint32_t k, LadderDev L,
                                                  TableDev tb, uint64_t cap_rows, unsigned long long* __restrict__ n_rows) {
@@ -1350,6 +1374,7 @@ struct BinRuns {
     unsigned long long* pre = nullptr;            // (runs << 32 | windows) before each bin
     uint64_t* runs = nullptr;
     uint64_t n_windows = 0;
+    bool est = false;  // of an estimate: timed under its names
     BinRuns(const MinPlan& m, uint64_t windows) : mp(m) {
         while (F < RUN_MAX_BINS && (uint64_t)F * 1500 < windows) F <<= 1;
     }
@@ -1383,21 +1408,21 @@ fbk_status bin_runs(fbk_ctx* ctx, Scratch& B, BinRuns& R, const BankDev& bv, uin
         R.runs = (uint64_t*)B.get(8 * n_warps * cap_w);
         if (!log || !R.runs) return set_err(ctx, FBK_ERR_OOM, "minimizer bins: runs");
         CK(ctx, cudaMemsetAsync(cleared, 0, clear_bytes, stream));
-        TIMED(ctx, "bins_runs", (k_bin_runs<<<(unsigned)n_blocks, 256, 0, stream>>>(bv, k, mp, F, log, log_n, (uint32_t)cap_w, R.hist,
-                                                                                    R.counters + BC_NEED),
-                                 cudaGetLastError()));
+        TIMED(ctx, R.est ? "est_runs" : "bins_runs",
+              (k_bin_runs<<<(unsigned)n_blocks, 256, 0, stream>>>(bv, k, mp, F, log, log_n, (uint32_t)cap_w, R.hist, R.counters + BC_NEED),
+               cudaGetLastError()));
         const unsigned tiles = (F + SCAN_TILE - 1) / SCAN_TILE;
-        TIMED(ctx, "bins_scan", (k_bin_scan_sums<<<tiles, 256, 0, stream>>>(R.hist, F, part), cudaGetLastError()));
-        TIMED(ctx, "bins_scan", (k_bin_scan<<<tiles, 256, 0, stream>>>(R.hist, F, part, R.pre, cursor), cudaGetLastError()));
-        TIMED(ctx, "bins_scatter", (k_bin_scatter<<<(unsigned)n_blocks, 256, 0, stream>>>(log, log_n, (uint32_t)cap_w, cursor, R.runs,
-                                                                                          n_warps * cap_w),
-                                    cudaGetLastError()));
+        TIMED(ctx, R.est ? "est_scan" : "bins_scan", (k_bin_scan_sums<<<tiles, 256, 0, stream>>>(R.hist, F, part), cudaGetLastError()));
+        TIMED(ctx, R.est ? "est_scan" : "bins_scan", (k_bin_scan<<<tiles, 256, 0, stream>>>(R.hist, F, part, R.pre, cursor), cudaGetLastError()));
+        TIMED(ctx, R.est ? "est_scatter" : "bins_scatter",
+              (k_bin_scatter<<<(unsigned)n_blocks, 256, 0, stream>>>(log, log_n, (uint32_t)cap_w, cursor, R.runs, n_warps * cap_w),
+               cudaGetLastError()));
         if (sample) {
             sample->runs = R.runs;
             sample->n_groups = std::min<uint32_t>(F, 1024);
             sample->stride = F / sample->n_groups;
             sample->start = R.pre;
-            TIMED(ctx, "bins_sample", agg_launch_nk<AGG_SAMPLE>((int)((k + 31) / 32), stream, sms, *sample));
+            TIMED(ctx, R.est ? "est_sample" : "bins_sample", agg_launch_nk<AGG_SAMPLE>((int)((k + 31) / 32), stream, sms, *sample));
         }
         CK(ctx, cudaMemcpyAsync(h, R.counters, 8 * BC_N, cudaMemcpyDeviceToHost, stream));
         CK(ctx, cudaMemcpyAsync(h + BC_N, R.pre + F, 8, cudaMemcpyDeviceToHost, stream));
@@ -1636,6 +1661,7 @@ fbk_status bins_first(fbk_ctx* ctx, const fbk_bank* b, uint64_t n_reads, uint64_
     const cudaStream_t stream = ctx->stream;
     Scratch B{ctx, {}};
     BinRuns R(min_plan(k), windows);
+    R.est = true;
     const uint64_t clear_bytes = 8ULL * R.F + 8 * 16;
     char* cleared = (char*)B.get(clear_bytes);
     AggArgs A{};
@@ -1668,7 +1694,7 @@ fbk_status bins_first(fbk_ctx* ctx, const fbk_bank* b, uint64_t n_reads, uint64_
     A.firsts = (FirstKey*)B.get(A.cap_rows * sizeof(FirstKey));
     if (!start || !A.firsts) return FBK_OK;
     A.start = start;
-    TIMED(ctx, "bins_groups", (k_bin_groups<<<std::min<unsigned>(1024, (R.F + 256) / 256), 256, 0, stream>>>(R.pre, R.F, (uint32_t)target,
+    TIMED(ctx, "est_groups", (k_bin_groups<<<std::min<unsigned>(1024, (R.F + 256) / 256), 256, 0, stream>>>(R.pre, R.F, (uint32_t)target,
                                                                                                           A.n_groups, start),
                                cudaGetLastError()));
     TIMED(ctx, "est_first_keys", agg_launch_nk<AGG_FIRST>(nk, stream, sms, A));
