@@ -928,32 +928,13 @@ bool takes_bins(const fbk_batch* B, const BatchIso* it) {
 // or have no memory for go to rest.
 fbk_status bins_wave(fbk_batch* B, const std::vector<BatchIso*>& W, std::vector<BatchIso*>& rest) {
     fbk_ctx* ctx = B->ctx;
-    const uint32_t n = (uint32_t)W.size();
-    std::vector<unsigned long long> counts;
-    {
-        WaveBufs w;
-        fbk_status st = wave_bufs(B, n, false, w);
-        if (st == FBK_OK) st = upload_wave(B, W, w);
-        if (st) return st;
-        st = run_phase(B, &B->stats.ms_phase_a, [&]() -> fbk_status {
-            CK(ctx, cudaMemsetAsync(w.cnt, 0, (uint64_t)n * 64, ctx->stream));
-            TIMED(ctx, "batch_count", launch_batch_count(shape_launch(ctx, B->solid), w.iso, w.rb, n, B->p.k));
-            return FBK_OK;
-        });
-        if (st == FBK_OK) st = stage(B, (uint64_t)n * 64);
-        if (st) return st;
-        CK(ctx, cudaMemcpyAsync(B->h_stage, w.cnt, (uint64_t)n * 64, cudaMemcpyDeviceToHost, ctx->stream));
-        CK(ctx, cudaStreamSynchronize(ctx->stream));
-        const unsigned long long* hc = (const unsigned long long*)B->h_stage;
-        counts.assign(hc, hc + 8ULL * n);
-    }
     const fbk_build_params bp = iso_params(B);
-    for (uint32_t i = 0; i < n; ++i) {
-        BatchIso* it = W[i];
+    for (BatchIso* it : W) {
         bool declined = false;
         float ms = 0.f;
         CK(ctx, cudaEventRecord(B->ev[0], ctx->stream));
-        const fbk_status st = bins_build(ctx, it->bank, &bp, it->keep, B->p.cms_log2_width, nullptr, &it->table, &declined);
+        const fbk_status st = bins_build(ctx, it->bank, &bp, it->keep, B->p.cms_log2_width, nullptr, &it->table, &declined,
+                                         &it->res.kmers);
         if (st == FBK_ERR_OOM || (st == FBK_OK && declined)) {
             ctx->err.clear();
             rest.push_back(it);
@@ -964,7 +945,6 @@ fbk_status bins_wave(fbk_batch* B, const std::vector<BatchIso*>& W, std::vector<
         CK(ctx, cudaEventSynchronize(B->ev[1]));
         CK(ctx, cudaEventElapsedTime(&ms, B->ev[0], B->ev[1]));
         B->stats.ms_phase_b += ms;
-        it->res.kmers = counts[8 * i + 1] + counts[8 * i + 2];
         it->res.wave = (int32_t)B->stats.waves;
         finish_iso(B, it);
     }

@@ -373,10 +373,10 @@ __device__ __forceinline__ uint64_t fold_of(const uint64_t (&w)[NK]) {
     return f;
 }
 
-// Counters of a build (u64): rows, low rows, keys seen once, adjacent solid windows; of the
-// sample: distinct keys, those seen twice, those that can become solid, windows; log words a
-// warp needed; groups handed out (aggregate, sample).
-enum { BC_ROWS, BC_LOW, BC_SINGLES, BC_PAIRS, BC_DISTINCT, BC_MULTI, BC_KEPT, BC_WINDOWS, BC_NEED, BC_WORK, BC_WORK_S, BC_N };
+// Counters of a build (u64): rows, low rows, keys seen once, adjacent solid windows, reads of one
+// window; of the sample: distinct keys, those seen twice, those that can become solid, windows;
+// log words a warp needed; groups handed out (aggregate, sample).
+enum { BC_ROWS, BC_LOW, BC_SINGLES, BC_PAIRS, BC_LONE, BC_DISTINCT, BC_MULTI, BC_KEPT, BC_WINDOWS, BC_NEED, BC_WORK, BC_WORK_S, BC_N };
 
 struct FirstKey {
     uint64_t raw;        // canonical ntHash
@@ -1034,10 +1034,13 @@ __global__ void __launch_bounds__(256) k_bin_sketch(const uint64_t* __restrict__
 
 // The windows a read has, as bits over the bases (a window's bit is its first base's).
 // Windows of different reads are never adjacent: k - 1 bases without one lie between.
-__global__ void __launch_bounds__(256) k_bin_valid(BankDev b, uint32_t k, uint32_t* __restrict__ valid) {
+__global__ void __launch_bounds__(256) k_bin_valid(BankDev b, uint32_t k, uint32_t* __restrict__ valid,
+                                                   unsigned long long* __restrict__ lone) {
+    uint32_t n_lone = 0;
     for (uint64_t r = b.r_begin + (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; r < b.r_end; r += (uint64_t)gridDim.x * blockDim.x) {
         const uint32_t len = b.len[r];
         if (len < k || !bank_keep(b, r)) continue;
+        n_lone += len == k;
         uint64_t g = b.off[r];
         const uint64_t end = g + (len - k + 1);
         while (g < end) {
@@ -1047,6 +1050,8 @@ __global__ void __launch_bounds__(256) k_bin_valid(BankDev b, uint32_t k, uint32
             g += m;
         }
     }
+    n_lone = __reduce_add_sync(0xffffffffu, n_lone);
+    if ((threadIdx.x & 31) == 0 && n_lone) atomicAdd(lone, (unsigned long long)n_lone);
 }
 
 // The three bitmaps: the windows there are, those of keys seen once, and of these the ones
@@ -1452,7 +1457,7 @@ uint64_t group_windows(uint32_t entries, uint64_t n_windows, uint64_t distinct) 
 }  // namespace
 
 fbk_status bins_build(fbk_ctx* ctx, const fbk_bank* b, const fbk_build_params* p, const uint64_t* keep_bits, uint32_t log2w, fbk_cms* cms,
-                      fbk_table** out, bool* declined) {
+                      fbk_table** out, bool* declined, uint64_t* kmers) {
     *declined = false;
     if (p->min_trans_cov > 0xFFFF) return set_err(ctx, FBK_ERR_INVALID, "thresholds must fit u16");
     const int nw = key_words(p->key_bits);
@@ -1599,7 +1604,7 @@ fbk_status bins_build(fbk_ctx* ctx, const fbk_bank* b, const fbk_build_params* p
             return stream_launch(stream, sms, b->n_words, kern, (const uint64_t*)b->data, maps, k, ladder, td, rows, counters + BC_ROWS);
         });
     };
-    TIMED(ctx, "bins_valid", stream_launch(stream, sms, b->n_reads, k_bin_valid, bv, k, valid));
+    TIMED(ctx, "bins_valid", stream_launch(stream, sms, b->n_reads, k_bin_valid, bv, k, valid, counters + BC_LONE));
     if (!cms) {
         TIMED(ctx, "bins_sketch", by_width(nw, k, [&](auto a, auto w) {
                   constexpr int NW = decltype(a)::value, NK = NW - decltype(w)::value;
@@ -1621,6 +1626,7 @@ fbk_status bins_build(fbk_ctx* ctx, const fbk_bank* b, const fbk_build_params* p
     CK(ctx, cudaMemcpyAsync(h, counters, 8 * BC_N, cudaMemcpyDeviceToHost, stream));
     CK(ctx, cudaStreamSynchronize(stream));
     const uint64_t pushes = 2 * h[BC_PAIRS];
+    if (kmers) *kmers = 2 * n_windows - h[BC_LONE];  // pass 2 leaves out the reads of one window
     tb->cap = h[BC_ROWS];
     // rows of the conversion: a subset of those with an edge count of min_trans_cov
     const uint64_t oc = std::min<uint64_t>(tb->cap, kept) + 16;

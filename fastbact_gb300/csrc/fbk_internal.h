@@ -262,11 +262,12 @@ fbk_status solid_build_ladder(fbk_ctx* ctx, const fbk_bank* b, uint32_t* ladder,
                               const uint64_t* keep_bits, uint64_t distinct_hint, fbk_table** out);
 
 // The build front end over minimizer bins (fbk_bins.cu); *declined is set when the reads'
-// shape does not suit it and the caller should take the record buckets.
+// shape does not suit it and the caller should take the record buckets; kmers: the occurrences
+// that passes 1 and 2 go over.
 constexpr uint32_t BINS_MIN_K = 17;
 bool bins_applicable(const fbk_ctx* ctx, const fbk_bank* b, const fbk_build_params* p, uint32_t log2w);
 fbk_status bins_build(fbk_ctx* ctx, const fbk_bank* b, const fbk_build_params* p, const uint64_t* keep_bits, uint32_t log2w, fbk_cms* cms,
-                      fbk_table** out, bool* declined);
+                      fbk_table** out, bool* declined, uint64_t* kmers = nullptr);
 // The estimator's sample loop over the bins (fbk_bins.cu): k at least BINS_MIN_K.
 fbk_status bins_first(fbk_ctx* ctx, const fbk_bank* b, uint64_t n_reads, uint64_t windows, uint32_t k, uint32_t* first, uint32_t log2w,
                       uint32_t p, uint32_t n_segs, uint32_t* regs_total, uint32_t* regs_solid, bool* declined);
