@@ -544,6 +544,9 @@ __global__ void __launch_bounds__(AGG_THREADS, 2) k_bin_agg(AggArgs A) {
     const uint32_t k = A.k;
     const uint32_t queue = sh_addr(agg_smem) + (threadIdx.x >> 5) * AGG_QUEUE;
     const uint32_t* __restrict__ d32 = reinterpret_cast<const uint32_t*>(A.data);
+    // A sample is launched before the host has looked whether every run was logged.  One that
+    // was not leaves a hole in its bin's range, and a hole is no run: nothing of it is read.
+    if (SAMPLE && A.counters[BC_NEED]) return;
     unsigned long long tot_single = 0, tot_multi = 0, tot_kept = 0;
     auto fetch = [&]() {  // thread 0: the block's next group
         const unsigned long long g = atomicAdd(&A.counters[SAMPLE ? BC_WORK_S : BC_WORK], 1ULL);
@@ -1387,7 +1390,7 @@ struct BinRuns {
 
 // Cuts the reads of bv into runs (windows: no fewer than they hold) and scatters them by bin;
 // with a sample, counts the keys of some bins.  The counters and n_windows are on the host
-// then, in ctx->h_pinned.  Clears the caller's block first.
+// then, in ctx->h_pinned.  Clears the caller's block and the context's status first.
 fbk_status bin_runs(fbk_ctx* ctx, Scratch& B, BinRuns& R, const BankDev& bv, uint32_t max_len, uint32_t k, uint64_t windows, char* cleared,
                     uint64_t clear_bytes, AggArgs* sample, bool* declined) {
     const MinPlan mp = R.mp;
@@ -1413,6 +1416,7 @@ fbk_status bin_runs(fbk_ctx* ctx, Scratch& B, BinRuns& R, const BankDev& bv, uin
         R.runs = (uint64_t*)B.get(8 * n_warps * cap_w);
         if (!log || !R.runs) return set_err(ctx, FBK_ERR_OOM, "minimizer bins: runs");
         CK(ctx, cudaMemsetAsync(cleared, 0, clear_bytes, stream));
+        CK(ctx, cudaMemsetAsync(ctx->d_status, 0, 4, stream));
         TIMED(ctx, R.est ? "est_runs" : "bins_runs",
               (k_bin_runs<<<(unsigned)n_blocks, 256, 0, stream>>>(bv, k, mp, F, log, log_n, (uint32_t)cap_w, R.hist, R.counters + BC_NEED),
                cudaGetLastError()));
@@ -1496,7 +1500,6 @@ fbk_status bins_build(fbk_ctx* ctx, const fbk_bank* b, const fbk_build_params* p
     if (!A.later) return set_err(ctx, FBK_ERR_OOM, "minimizer bins");
     unsigned long long* h = (unsigned long long*)ctx->h_pinned;
     const bool may_filter = p->min_trans_cov >= 2 && ctx->acc_filter != 0;
-    CK(ctx, cudaMemsetAsync(ctx->d_status, 0, 4, stream));
     A.mtc = may_filter ? p->min_trans_cov : 0;
     fbk_status rs = bin_runs(ctx, B, R, bv, b->max_len, k, windows, cleared, clear_bytes, sampled ? &A : nullptr, declined);
     if (rs || *declined) return rs;
@@ -1680,7 +1683,6 @@ fbk_status bins_first(fbk_ctx* ctx, const fbk_bank* b, uint64_t n_reads, uint64_
     R.hist = (unsigned long long*)cleared;
     A.counters = R.counters = R.hist + R.F;
     unsigned long long* h = (unsigned long long*)ctx->h_pinned;
-    CK(ctx, cudaMemsetAsync(ctx->d_status, 0, 4, stream));
     bool no = false;
     fbk_status st = bin_runs(ctx, B, R, bank_view(b, 0, n_reads, nullptr), b->max_len, k, windows, cleared, clear_bytes, &A, &no);
     if (st == FBK_ERR_OOM || no) return FBK_OK;

@@ -141,3 +141,39 @@ def test_overlapping_reads():
         u.release()
     ctx.close()
     assert got[0] == got[1]
+
+
+def uneven_reads(seed, genome_len, n, length, long_ones, rate=0.002):
+    """n reads of about `length` bases and a few long ones, from a genome, with errors."""
+    rng = np.random.default_rng(seed)
+    g = np.frombuffer(rand_seqs(seed, 1, genome_len, genome_len)[0], np.uint8)
+    lens = list(rng.integers(length - length // 8, length + length // 8, n))
+    for L in long_ones:
+        lens.insert(int(rng.integers(len(lens))), L)
+    out = []
+    for L in lens:
+        a = int(rng.integers(0, genome_len - L + 1))
+        r = g[a:a + L].copy()
+        e = rng.random(L) < rate
+        r[e] = np.frombuffer(b"ACGT", np.uint8)[rng.integers(0, 4, int(e.sum()))]
+        out.append(rc(r.tobytes()) if rng.random() < 0.5 else r.tobytes())
+    return out
+
+
+@pytest.mark.parametrize("k", [21, 31, 77])
+@pytest.mark.parametrize("keep", [False, True])
+@pytest.mark.parametrize("n,length,long_ones,binned", [(640, 7200, (150_000, 90_000), True), (8000, 620, (1_000_000,), False)])
+def test_reads_of_uneven_length(k, keep, n, length, long_ones, binned):
+    """A warp of k_bin_runs meets reads of many times the mean length: its log is too short and
+    the runs are logged again with room for it, or, where that would take the logs of thousands
+    of warps to the length of one, the build goes over the record buckets."""
+    c = api.Context(0)
+    try:
+        seqs = uneven_reads(k, 1_200_000, n, length, long_ones)
+        assert sum(len(s) - k + 1 for s in seqs) > 4 << 20
+        c.set_timing(True)
+        (compare_build if keep else compare_gate_only)(c, bank_of(seqs), k, api.key_bits_for_k(k), 16, None, 20)
+        assert c.timing("bins_runs")[1] == (2 if binned else 1)
+        assert (c.timing("bins_aggregate")[0] > 0) == binned and (c.timing("pass2_emit")[0] > 0) != binned
+    finally:
+        c.close()

@@ -13,6 +13,7 @@ import pytest
 
 from fastbact_gb300 import api
 from oracle import orc
+from test_gpu_bins import uneven_reads
 from test_gpu_parity import sample_reads
 
 pytestmark = pytest.mark.gpu
@@ -53,3 +54,22 @@ def test_whole_samples(ctx, genome, cov, k, p, log2w, errors, distinct):
     same(ctx, sample, n, stats, k, p, log2w)
     ctx.set_timing(False)
     assert (ctx.timing("est_first_regs")[0] > 0) == distinct
+
+
+@pytest.mark.parametrize("k", [21, 31])
+@pytest.mark.parametrize("long_ones,runs", [((120_000, 80_000), 2), ((1_000_000, 7_500), 1)])
+def test_samples_of_uneven_length(ctx, k, long_ones, runs):
+    """Reads of many times the mean length: the runs of one warp do not fit its log, which is
+    made longer, or the sample goes over its occurrences."""
+    seqs = uneven_reads(k, 1_200_000, 1400, 7500, long_ones)
+    sample = api.BitSeqArena.from_seqs(seqs)
+    n = len(seqs) // 2
+    lens = [len(s) for s in seqs]
+    stats = api.ExactCountStats(n, sum(lens[::2]), sum(lens[1::2]), sum(lens), min(lens), max(lens), float(np.mean(lens)), int(np.median(lens)))
+    assert sum(len(s) - k + 1 for s in seqs) > 8 << 20
+    ctx.timing_reset()
+    ctx.set_timing(True)
+    same(ctx, sample, n, stats, k, 14, 20)
+    ctx.set_timing(False)
+    assert ctx.timing("est_runs")[1] == runs
+    assert (ctx.timing("est_first_keys")[0] > 0) == (runs == 2)
