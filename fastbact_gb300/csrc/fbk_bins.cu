@@ -1698,7 +1698,10 @@ fbk_status bins_first(fbk_ctx* ctx, const fbk_bank* b, uint64_t n_reads, uint64_
     unsigned long long* start = (unsigned long long*)B.get(8ULL * (A.n_groups + 1));
     A.first = first;
     A.log2w = log2w;
-    A.cap_rows = distinct + distinct / 8;  // some entries are made for nothing
+    // Entries made for nothing come on top: a key is entered once for every warp that meets it
+    // before the first one's slot is published (1400 reads of 7.5 kb, k = 21: a third of the keys;
+    // 300,000 reads of 150: a fifth).  The groups' fill leaves them 1 / 0.7 of the keys' room.
+    A.cap_rows = distinct + distinct / 2;
     A.firsts = (FirstKey*)B.get(A.cap_rows * sizeof(FirstKey));
     if (!start || !A.firsts) return FBK_OK;
     A.start = start;

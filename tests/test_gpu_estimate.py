@@ -73,3 +73,19 @@ def test_samples_of_uneven_length(ctx, k, long_ones, runs):
     ctx.set_timing(False)
     assert ctx.timing("est_runs")[1] == runs
     assert (ctx.timing("est_first_keys")[0] > 0) == (runs == 2)
+
+
+@pytest.mark.parametrize("n,length", [(1400, 7500), (70_000, 150)])
+def test_keys_met_by_many_warps_at_once(ctx, n, length):
+    """Deep samples, whose k-mers are entered several times before the first entry is seen: the
+    distinct ones find room all the same."""
+    seqs = uneven_reads(n, 1_200_000, n, length, ())
+    sample = api.BitSeqArena.from_seqs(seqs)
+    lens = [len(s) for s in seqs]
+    stats = api.ExactCountStats(n // 2, sum(lens[::2]), sum(lens[1::2]), sum(lens), min(lens), max(lens), float(np.mean(lens)),
+                                int(np.median(lens)))
+    ctx.timing_reset()
+    ctx.set_timing(True)
+    same(ctx, sample, n // 2, stats, 21, 14, 20)
+    ctx.set_timing(False)
+    assert ctx.timing("est_first_keys")[1] == ctx.timing("est_first_regs")[1] > 0
