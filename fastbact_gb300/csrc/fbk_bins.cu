@@ -293,13 +293,21 @@ __global__ void __launch_bounds__(256) k_bin_scatter(const uint64_t* __restrict_
 }
 
 // Groups of consecutive bins of about `target` windows: bin i belongs to group
-// floor(windows before it / target).  start[g] = the prefix (runs << 32 | windows) at the
-// first bin of group g, start[n_groups] = the totals.
+// floor(windows before it / target), and one of 2 target windows and more, which reaches past
+// the next group, to that one alone.  (A frequent k-mer's bin with ordinary ones before it: its
+// group has wide counts and so fewer entries, and where the keys did not fit, all of its windows
+// were counted twice.  Poly-G in 5% of 1.2 M reads, k = 21: 14.5 or 27.6 ms a build before.)
+// start[g] = the prefix (runs << 32 | windows) at the first bin of group g, start[n_groups] =
+// the totals.
 __global__ void k_bin_groups(const unsigned long long* __restrict__ pre, uint32_t n, uint32_t target, uint32_t n_groups,
                              unsigned long long* __restrict__ start) {
+    auto group = [&](uint32_t i) {
+        const uint32_t before = (uint32_t)pre[i], windows = (uint32_t)pre[i + 1] - before;
+        return before / target + (windows / 2 >= target);
+    };
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i <= n; i += gridDim.x * blockDim.x) {
-        const uint32_t lo = i ? (uint32_t)(pre[i - 1] & 0xFFFFFFFFull) / target + 1 : 0;
-        const uint32_t hi = i < n ? (uint32_t)(pre[i] & 0xFFFFFFFFull) / target : n_groups;
+        const uint32_t lo = i ? group(i - 1) + 1 : 0;
+        const uint32_t hi = i < n ? group(i) : n_groups;
         for (uint32_t g = lo; g <= hi && g <= n_groups; ++g) start[g] = pre[i];
     }
 }

@@ -177,3 +177,16 @@ def test_reads_of_uneven_length(k, keep, n, length, long_ones, binned):
         assert (c.timing("bins_aggregate")[0] > 0) == binned and (c.timing("pass2_emit")[0] > 0) != binned
     finally:
         c.close()
+
+
+@pytest.mark.parametrize("k", [21, 77])
+@pytest.mark.parametrize("share", [0.02, 0.1])
+def test_frequent_kmer(ctx, k, share):
+    """One k-mer many times a group's windows, among more than 4 M ordinary ones: its bin has a
+    group of its own, between those of the bins before and after it."""
+    seqs = uneven_reads(k, 150_000, 36_000, 200, (), 0.004)
+    n = int(share * len(seqs))
+    seqs[100:100 + n] = [b"G" * len(s) for s in seqs[100:100 + n]]
+    seqs[200:200 + n // 8] = [s[:30] + s[30:31].replace(b"G", b"T") + s[31:] for s in seqs[200:200 + n // 8]]
+    assert sum(len(s) - k + 1 for s in seqs) > 4 << 20
+    compare_gate_only(ctx, bank_of(seqs), k, api.key_bits_for_k(k), 16, None, 18)
