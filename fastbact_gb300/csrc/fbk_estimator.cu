@@ -235,6 +235,13 @@ uint32_t est_next(const EstAt& at, const EstPlan& pl, uint32_t hi) {
 // host take 0.15 of that at any size).
 constexpr uint64_t EST_BINS_FROM = 8u << 20;
 
+// A sample with longer reads is taken in one round: a read is one warp's, and every round waits
+// for its longest.  Log-normal reads, 5 Mbp genome, k = 21: longest 8 kb 5.6 ms in rounds, 4.1 at
+// once (and for a genome of 400 kb, deep enough in the first round, 1.6 and 3.4); 30 kb 15.0 and
+// 6.0, 150 kb 17.7 and 10.0.  (By occurrences at once 14.8 and 31.7; with 1% errors, which take
+// 150 kb through three rounds, 36.5 against 32.0.)
+constexpr uint32_t EST_ROUND_READS = 16384;
+
 // Sample loop on a device-resident sample bank whose first 2*n_use reads are the
 // pairs, R1 then R2; lengths is the host copy of those reads' lengths.  It runs in rounds
 // of whole segments, so that a sample that is deep enough early (a 300 kbp genome after
@@ -273,7 +280,7 @@ fbk_status estimate_impl(fbk_ctx* ctx, const fbk_bank* bank, const uint32_t* len
     Launch L = launch_cfg(ctx, 256, 0);
     std::vector<double> h_sums(2 * n_segs);
     std::vector<unsigned long long> h_zeros(2 * n_segs);
-    uint32_t seg_lo = 0, seg_hi = 1, final_seg = 0;
+    uint32_t seg_lo = 0, seg_hi = bank->max_len > EST_ROUND_READS ? n_segs : 1, final_seg = 0;
     for (;;) {
         const BankDev bv = bank_view(bank, seg_lo ? 2 * est_seg_end(seg_lo - 1, n_use) : 0, 2 * est_seg_end(seg_hi - 1, n_use), nullptr);
         const uint64_t m_lo = seg_lo ? pl.m_seg[seg_lo - 1] : 0, m_hi = pl.m_seg[seg_hi - 1];

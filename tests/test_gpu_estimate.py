@@ -89,3 +89,18 @@ def test_keys_met_by_many_warps_at_once(ctx, n, length):
     same(ctx, sample, n // 2, stats, 21, 14, 20)
     ctx.set_timing(False)
     assert ctx.timing("est_first_keys")[1] == ctx.timing("est_first_regs")[1] > 0
+
+
+@pytest.mark.parametrize("genome,longest,rounds", [(100_000, 20_000, 1), (600_000, 20_000, 1), (600_000, 10_000, 2)])
+def test_long_reads_in_one_round(ctx, genome, longest, rounds):
+    """A sample with a long read is taken at once, whether the loop stops at its first checkpoint
+    or at its end."""
+    seqs = uneven_reads(genome, genome, 16_000, 400, (longest, 300))
+    sample = api.BitSeqArena.from_seqs(seqs)
+    n, lens = len(seqs) // 2, [len(s) for s in seqs]
+    stats = api.ExactCountStats(n, sum(lens[::2]), sum(lens[1::2]), sum(lens), min(lens), max(lens), float(np.mean(lens)), int(np.median(lens)))
+    ctx.timing_reset()
+    ctx.set_timing(True)
+    assert same(ctx, sample, n, stats, 21, 14, 18) == (6000 if genome == 100_000 else n)
+    ctx.set_timing(False)
+    assert ctx.timing("est_firstpos")[1] == rounds
