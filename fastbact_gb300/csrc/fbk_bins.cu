@@ -1585,12 +1585,15 @@ fbk_status bins_build(fbk_ctx* ctx, const fbk_bank* b, const fbk_build_params* p
         CK(ctx, cudaMemcpyAsync(h, counters, 8 * BC_N, cudaMemcpyDeviceToHost, stream));
         CK(ctx, cudaMemcpyAsync(h + BC_N, ctx->d_status, 4, cudaMemcpyDeviceToHost, stream));
         CK(ctx, cudaStreamSynchronize(stream));
-        if ((uint32_t)h[BC_N] & ST_SPIN_TIMEOUT) return set_err(ctx, FBK_ERR_TIMEOUT, "minimizer bins: a bounded search gave up");
-        if ((uint32_t)h[BC_N] & ST_TABLE_FULL) return set_err(ctx, FBK_ERR_TABLE_FULL, "minimizer bins: a group did not fit");
+        // Keys that no hash tells apart (more of one fold and one minimizer than a block holds and
+        // puts off), a bounded search that gave up: the record buckets' table takes them.
+        *declined = (uint32_t)h[BC_N] != 0;
+        if (*declined) return FBK_OK;
         const uint64_t need = h[BC_ROWS] + (filter ? 0 : h[BC_SINGLES]);
         if (need <= rows && (cms || h[BC_LOW] <= lows)) break;
         // the sample's estimate was low: again with the counted sizes
-        if (attempt == 1) return set_err(ctx, FBK_ERR_TABLE_FULL, "minimizer bins: row counts changed between runs");
+        *declined = attempt == 1;
+        if (*declined) return FBK_OK;
         tbl_free_storage(tb);
         if (low) B.drop(low);
         rows = need + 1;

@@ -261,9 +261,10 @@ fbk_status solid_build(fbk_ctx* ctx, const fbk_bank* b, const fbk_cms* cms, cons
 fbk_status solid_build_ladder(fbk_ctx* ctx, const fbk_bank* b, uint32_t* ladder, uint32_t log2w, const fbk_build_params* p,
                               const uint64_t* keep_bits, uint64_t distinct_hint, fbk_table** out);
 
-// The build front end over minimizer bins (fbk_bins.cu); *declined is set when the reads'
-// shape does not suit it and the caller should take the record buckets; kmers: the occurrences
-// that passes 1 and 2 go over.
+// The build front end over minimizer bins (fbk_bins.cu); *declined is set when the reads or
+// their keys do not suit it and the caller should take the record buckets (a sketch that the
+// caller keeps then holds part of the counts: it is cleared first); kmers: the occurrences that
+// passes 1 and 2 go over.
 constexpr uint32_t BINS_MIN_K = 17;
 bool bins_applicable(const fbk_ctx* ctx, const fbk_bank* b, const fbk_build_params* p, uint32_t log2w);
 fbk_status bins_build(fbk_ctx* ctx, const fbk_bank* b, const fbk_build_params* p, const uint64_t* keep_bits, uint32_t log2w, fbk_cms* cms,

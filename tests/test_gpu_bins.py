@@ -143,6 +143,23 @@ def test_overlapping_reads():
     assert got[0] == got[1]
 
 
+def one_fold(n, seed=5):
+    """n reads, twice each, whose first 63-mers share their minimizer and the fold of their two
+    words, which is all that any hash of a key sees."""
+    rng = np.random.default_rng(seed)
+    code = np.zeros(256, np.uint8)
+    code[list(b"ACGT")] = range(4)
+    x = code[np.frombuffer(low_minimizer(), np.uint8)]
+    w0 = rng.integers(0, 4, (n, 31)).astype(np.uint8)
+    w0[:, 0] = 0                            # with the last base below: smaller than their reverse complements
+    w0[:, 16:31] = x
+    c = rng.integers(0, 4, 32).astype(np.uint8)
+    c[31] = x[14]
+    w1 = np.concatenate([np.zeros((n, 1), np.uint8), w0], 1) ^ c
+    reads = np.concatenate([w0, w1, rng.integers(0, 4, (n, 1)).astype(np.uint8)], 1)
+    return [bytes(r) for r in np.frombuffer(b"ACGT", np.uint8)[reads]] * 2
+
+
 def uneven_reads(seed, genome_len, n, length, long_ones, rate=0.002):
     """n reads of about `length` bases and a few long ones, from a genome, with errors."""
     rng = np.random.default_rng(seed)
@@ -190,3 +207,16 @@ def test_frequent_kmer(ctx, k, share):
     seqs[200:200 + n // 8] = [s[:30] + s[30:31].replace(b"G", b"T") + s[31:] for s in seqs[200:200 + n // 8]]
     assert sum(len(s) - k + 1 for s in seqs) > 4 << 20
     compare_gate_only(ctx, bank_of(seqs), k, api.key_bits_for_k(k), 16, None, 18)
+
+
+@pytest.mark.parametrize("keep", [False, True])
+def test_keys_of_one_fold(keep):
+    """14,000 keys that no hash tells apart: a group of them cannot be taken in parts, and the
+    build goes over the record buckets."""
+    c = api.Context(0)
+    try:
+        c.set_timing(True)
+        (compare_build if keep else compare_gate_only)(c, bank_of(one_fold(14_000) + rand_seqs(9, 100, 80, 200)), 63, 128, 16, None, 18)
+        assert c.timing("bins_aggregate")[1] == 1 and c.timing("pass2_emit")[1] > 0
+    finally:
+        c.close()
