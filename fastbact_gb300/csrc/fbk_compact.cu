@@ -12,7 +12,8 @@
 //   3. every (boundary node, direction, out-edge) start finds its path's length and end by
 //      descending those tables, one thread per start, with no shared marks: a unitig
 //      reachable from both ends is kept from the end whose (row, direction, edge) is smaller
-//      — the same set of unitigs, decided without ordering;
+//      — the same set of unitigs, decided without ordering — and one that is its own reverse
+//      complement, which has one end, up to its middle;
 //   4. the bases of the kept paths are written eight to a thread, each thread jumping to its
 //      place, already in the orientation of min(sequence, reverse complement);
 //   5. the 1-in-1-out nodes no path visited (isolated cycles, few) and the overlap
@@ -325,6 +326,13 @@ struct Jumps {
     int n;
 };
 
+// The node d steps on from `at`, on a path that has it.
+__device__ __forceinline__ uint32_t steps_on(const Jumps& J, uint32_t at, uint32_t d) {
+    for (int l = 0; l < J.n; ++l)
+        if ((d >> l) & 1u) at = J.t[l][at];
+    return at;
+}
+
 // A path (build.rs:349-445): its first 1-in-1-out node (NO_NODE: none), how many of them, and
 // how it is stored: 0 as walked, 1 reverse complemented, 2 decided once it is written.
 struct Path {
@@ -355,7 +363,7 @@ __global__ void __launch_bounds__(256) k_paths(Rows R, Jumps J, uint32_t k, cons
                     nodes += 1ULL << l;
                 }
             }
-            if (nodes > R.n + 1) {  // a path longer than the node count: impossible for valid rows
+            if (nodes > 2 * R.n) {  // more than there are directed nodes: impossible for valid rows
                 atomicOr(status, ST_SPIN_TIMEOUT);
                 nodes = 1;
             }
@@ -366,7 +374,15 @@ __global__ void __launch_bounds__(256) k_paths(Rows R, Jumps J, uint32_t k, cons
         if (r >= 0) {
             // boundary end: the walk from (r, !c_rc, rc_p) covers the same unitig
             const uint32_t m = R.mask[r], back = c_rc ? m & 15u : (m >> 4) & 15u;
-            if ((back >> rc_p) & 1u) keep = start <= (((uint64_t)r << 4) | ((uint64_t)(c_rc ? 0u : 1u) << 3) | rc_p);
+            const uint64_t other = ((uint64_t)r << 4) | ((uint64_t)(c_rc ? 0u : 1u) << 3) | rc_p;
+            if ((back >> rc_p) & 1u) keep = start <= other;
+            if (start == other && p.nodes) {
+                // its own reverse complement: past its middle every edge has been used already,
+                // in the other direction, and the walk ends there (build.rs:349-445)
+                p.nodes = (p.nodes + 1) / 2;
+                const uint32_t at = steps_on(J, p.first, p.nodes - 1);
+                take_edge<NW>(R, k, at >> 1, at & 1u, only_edge(R.mask[at >> 1], at & 1u), f, rv, rc_p, c_rc);
+            }
         }
         // min(sequence, reverse complement) (build.rs:438-439): their first k bases decide
         p.flip = kless<NW>(rv, head) ? 1u : keq<NW>(rv, head) ? 2u : 0u;
@@ -403,11 +419,7 @@ __global__ void __launch_bounds__(256) k_path_bases(Rows R, Jumps J, uint32_t k,
             const uint64_t end = min(p1, off[s] + L);
             uint32_t j = (uint32_t)(p - off[s]);
             uint32_t at = path.first;
-            if (j > k) {  // node j - k (1-based)
-                const uint32_t d = j - k - 1;
-                for (int l = 0; l < J.n; ++l)
-                    if ((d >> l) & 1u) at = J.t[l][at];
-            }
+            if (j > k) at = steps_on(J, at, j - k - 1);  // node j - k (1-based)
             unsigned long long c = 0;
             Key<NW> head;
             if (j < k) {
@@ -735,7 +747,7 @@ fbk_status compact_impl(fbk_table* t, fbk_unitigs* U) {
         CK(ctx, cudaMemcpyAsync(h + 1, ctx->d_status, 4, cudaMemcpyDeviceToHost, ctx->stream));
         CK(ctx, cudaStreamSynchronize(ctx->stream));
         total = h[0];
-        if ((uint32_t)h[1]) return set_err(ctx, FBK_ERR_INVALID, "compaction: node index full or a path longer than the node count");
+        if ((uint32_t)h[1]) return set_err(ctx, FBK_ERR_INVALID, "compaction: node index full or a path of more nodes than there are");
         uint8_t* seqs = (uint8_t*)B.get(std::max<uint64_t>(total, 1));
         if (!seqs) return set_err(ctx, FBK_ERR_OOM, "compaction sequences");
         if (total)

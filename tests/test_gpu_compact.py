@@ -24,3 +24,27 @@ def test_path_lengths_and_hairpins(ctx, k, kb):
     reads = [s for s in seqs for _ in range(4)]
     bank = api.ReadBank(merged_reads=api.BitSeqArena.from_seqs(reads))
     compare_compaction(ctx, bank, k, kb, 16, None, 14)
+
+
+@pytest.mark.parametrize("k,kb", [(5, 64), (20, 64), (21, 64), (31, 64), (32, 128), (33, 128), (64, 256), (77, 256), (127, 256)])
+@pytest.mark.parametrize("extra", [1, 2, 3, 4, 5, 40, 301])
+def test_palindromic_contigs(ctx, k, kb, extra):
+    """A contig that is its own reverse complement passes every row twice: the walk stops at its
+    middle, an edge (odd k) or a k-mer (even k) that is its own reverse complement."""
+    x = rand_seqs(40 + extra, 1, k // 2 + extra, k // 2 + extra)[0]
+    y = rand_seqs(3, 1, 3 * k, 3 * k)[0]
+    for seqs in ([x + x[::-1].translate(COMP)], [x + x[::-1].translate(COMP), y]):
+        if k == 5 and (extra > 4 or len(seqs) > 1):  # the short words meet: branches
+            continue
+        bank = api.ReadBank(merged_reads=api.BitSeqArena.from_seqs([s for s in seqs for _ in range(4)]))
+        compare_compaction(ctx, bank, k, kb, 16, None, 14)
+
+
+@pytest.mark.parametrize("k,kb", [(21, 64), (32, 128), (77, 256)])
+def test_hairpin_on_a_branch(ctx, k, kb):
+    """A palindromic path that leaves a branching node and comes back to it by the same edge."""
+    a, b, x = (rand_seqs(70 + i, 1, 2 * k + i, 2 * k + i)[0] for i in range(3))
+    stem = a + x
+    seqs = [stem + stem[::-1].translate(COMP), a + b]
+    bank = api.ReadBank(merged_reads=api.BitSeqArena.from_seqs([s for s in seqs for _ in range(4)]))
+    compare_compaction(ctx, bank, k, kb, 16, None, 14)
