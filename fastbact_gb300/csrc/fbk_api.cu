@@ -420,7 +420,7 @@ FBK_API fbk_status fbk_ctx_set_tuning(fbk_ctx* ctx, const char* name, double v) 
     else if (n == "filter_sizing" && (v == 0 || v == 1)) ctx->filter_sizing = (int)v;
     else if (n == "filter_load" && v >= 0.02 && v <= 0.9) ctx->filter_load = v;
     else if (n == "acc_filter" && (v == 0 || v == 1 || v == 2)) ctx->acc_filter = (int)v;
-    else if (n == "build_form" && (v == 0 || v == 1)) ctx->build_form = (int)v;
+    else if (n == "build_form" && (v == 0 || v == 1)) ctx->build_form = (int)v, ctx->records_tuned = false;
     else if (n == "upsert_all" && (v == 0 || v == 1 || v == 2)) ctx->upsert_all = (int)v;
     // the pass kernels are compiled for blocks of at most 256 threads
     else if (n == "block_pass1" && v >= 32 && v <= 256 && ((int)v % 32) == 0) ctx->block_pass1 = (int)v;
@@ -454,7 +454,7 @@ FBK_API fbk_status fbk_ctx_get_tuning(const fbk_ctx* ctx, const char* name, doub
     else if (n == "filter_sizing") *v = ctx->filter_sizing;
     else if (n == "filter_load") *v = ctx->filter_load;
     else if (n == "acc_filter") *v = ctx->acc_filter;
-    else if (n == "build_form") *v = ctx->build_form;
+    else if (n == "build_form") *v = ctx->records_tuned ? 0 : ctx->build_form;
     else if (n == "upsert_all") *v = ctx->upsert_all;
     else if (n == "block_pass1") *v = ctx->block_pass1;
     else if (n == "grid_pass1") *v = ctx->grid_pass1;

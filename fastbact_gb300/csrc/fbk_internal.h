@@ -100,9 +100,9 @@ struct fbk_ctx {
     // where a bucket holds more survivors than bucket 0 predicted).
     int filter_sizing = 1;
     double filter_load = 0.3;
-    // Builds that do not return their sketch: 1 (default) minimizer bins (fbk_bins.cu) where
-    // they apply, 0 record buckets.  Setting any option of the record buckets (bucket_bytes,
-    // ladder_ilp, ...) takes the context's builds there too.
+    // Builds without prior contigs: 1 (default) minimizer bins (fbk_bins.cu) where they apply,
+    // 0 record buckets.  Setting any option of the record buckets (bucket_bytes, ladder_ilp,
+    // ...) takes the context's builds there too, until build_form is set again.
     int build_form = 1;
     bool records_tuned = false;
     int batch_pass1 = 0;                  // batches with a ladder gate: 0 autotuned, 1 one multi-isolate launch, 2 a launch per isolate

@@ -168,9 +168,9 @@ FBK_API fbk_status fbk_ctx_event_elapsed(fbk_ctx* ctx, int slot_a, int slot_b, d
  * (the default), 5 = the same at two blocks per SM for every key width), "acc_filter"
  * (keys that cannot become SolidKmerNodes stay out of the table, see fbk_table_flags:
  * 0 never, 1 where it pays, 2 always), "build_form" (1, the default: builds run over
- * minimizer bins where those apply; 0: over record buckets, as
- * does every build of a context on which an option of the record buckets was set),
- * "upsert_all" (1: an unfiltered pass upserts every
+ * minimizer bins where those apply; 0: over record buckets.  Setting an option of the
+ * record buckets takes the context's builds there too, and build_form then reads 0,
+ * until it is set to 1 again), "upsert_all" (1: an unfiltered pass upserts every
  * bucket in one persistent launch), "upsert_queue" (1: filtered upserts queue the
  * filter's survivors per warp before probing), "filter_sizing" (1: a filtered pass sizes
  * its table from the first bucket's survivors, at load "filter_load"), "batch_pass1"

@@ -220,3 +220,26 @@ def test_keys_of_one_fold(keep):
         assert c.timing("bins_aggregate")[1] == 1 and c.timing("pass2_emit")[1] > 0
     finally:
         c.close()
+
+
+def test_record_options_and_the_form():
+    """An option of the record buckets takes the builds there, which build_form tells and undoes."""
+    c = api.Context(0)
+    try:
+        bank = bank_of(rand_seqs(1, 50, 100, 200) * 2)
+
+        def binned():
+            c.timing_reset()
+            c.set_timing(True)
+            api.build_cdbg_ext(bank, 31, None, 10_000, ctx=c, counter_bits=16, cms_log2_width=12).release()
+            return c.timing("bins_aggregate")[0] > 0
+
+        assert c.get_tuning("build_form") == 1 and binned()
+        c.set_tuning(bucket_bytes=c.get_tuning("bucket_bytes"))
+        assert c.get_tuning("build_form") == 0 and not binned()
+        c.set_tuning(build_form=1)
+        assert c.get_tuning("build_form") == 1 and binned()
+        c.set_tuning(build_form=0)
+        assert c.get_tuning("build_form") == 0 and not binned()
+    finally:
+        c.close()
