@@ -317,6 +317,8 @@ FBK_API fbk_status fbk_ctx_fork(fbk_ctx* parent, fbk_ctx** out) {
     c->filter_load = parent->filter_load;
     c->acc_filter = parent->acc_filter;
     c->upsert_all = parent->upsert_all;
+    c->build_form = parent->build_form;
+    c->records_tuned = parent->records_tuned;
     cudaError_t e = cudaSetDevice(c->device);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaMalloc((void**)&c->d_status, 64);

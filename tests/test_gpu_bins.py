@@ -7,9 +7,12 @@ ones (windows with no neighbour, with one, with two, of the same k-mers and of t
 complements), more distinct keys than a group's entries (windows put off to a later turn, and
 a group taken in parts), groups of more than 65535 windows (wide counts), reads cut into
 several runs, and reads that overlap in the packed words (left to the record buckets)."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
+from fastbact_gb300 import _native as N
 from fastbact_gb300 import api
 from test_gpu_parity import compare_build, compare_gate_only, rand_seqs
 
@@ -242,4 +245,19 @@ def test_record_options_and_the_form():
         c.set_tuning(build_form=0)
         assert c.get_tuning("build_form") == 0 and not binned()
     finally:
+        c.close()
+
+
+@pytest.mark.parametrize("option", [dict(build_form=0), dict(load_factor=0.5), {}])
+def test_a_fork_builds_in_its_parents_form(option):
+    c = api.Context(0)
+    h = C.c_void_p()
+    try:
+        c.set_tuning(**option)
+        N.check(N.lib().fbk_ctx_fork(c.handle, C.byref(h)), c.handle, "fork")
+        v = C.c_double()
+        N.check(N.lib().fbk_ctx_get_tuning(h, b"build_form", C.byref(v)), h, "get_tuning")
+        assert v.value == c.get_tuning("build_form") == (0 if option else 1)
+    finally:
+        N.lib().fbk_ctx_destroy(h)
         c.close()
