@@ -293,21 +293,21 @@ __device__ __forceinline__ int64_t take_edge(const Rows& R, uint32_t k, uint64_t
 }
 __device__ __forceinline__ uint32_t only_edge(uint32_t m, uint32_t dir) { return __ffs(dir ? (m >> 4) & 15u : m & 15u) - 1; }
 
-// The successor of every directed 1-in-1-out node, where it is one too.
+// The successor of a directed 1-in-1-out node, where it is one too.
+template <int NW>
+__device__ __forceinline__ uint32_t next_node(const Rows& R, uint32_t k, uint32_t at) {
+    const uint32_t m = R.mask[at >> 1];
+    if (!one_in_one_out(m)) return NO_NODE;
+    Key<NW> f, rv;
+    uint32_t rc_p;
+    bool c_rc;
+    const int64_t r = take_edge<NW>(R, k, at >> 1, at & 1u, only_edge(m, at & 1u), f, rv, rc_p, c_rc);
+    return r >= 0 && one_in_one_out(R.mask[r]) ? (uint32_t)(r << 1) | (c_rc ? 1u : 0u) : NO_NODE;
+}
 template <int NW>
 __global__ void __launch_bounds__(256) k_next(Rows R, uint32_t k, uint32_t* __restrict__ next) {
-    for (uint64_t s = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; s < 2 * R.n; s += (uint64_t)gridDim.x * blockDim.x) {
-        const uint32_t m = R.mask[s >> 1];
-        uint32_t to = NO_NODE;
-        if (one_in_one_out(m)) {
-            Key<NW> f, rv;
-            uint32_t rc_p;
-            bool c_rc;
-            const int64_t r = take_edge<NW>(R, k, s >> 1, (uint32_t)s & 1u, only_edge(m, (uint32_t)s & 1u), f, rv, rc_p, c_rc);
-            if (r >= 0 && one_in_one_out(R.mask[r])) to = (uint32_t)(r << 1) | (c_rc ? 1u : 0u);
-        }
-        next[s] = to;
-    }
+    for (uint64_t s = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; s < 2 * R.n; s += (uint64_t)gridDim.x * blockDim.x)
+        next[s] = next_node<NW>(R, k, (uint32_t)s);
 }
 // Table l + 1 from table l; any: whether an entry is left.
 __global__ void __launch_bounds__(256) k_double(const uint32_t* __restrict__ in, uint32_t* __restrict__ out, uint64_t n, uint32_t* any) {
@@ -320,15 +320,24 @@ __global__ void __launch_bounds__(256) k_double(const uint32_t* __restrict__ in,
     if (__any_sync(0xffffffffu, some) && (threadIdx.x & 31) == 0) atomicOr(any, 1u);
 }
 
+// The tables there is memory for, the highest of them taken as often as need be; without any
+// the successors are looked up one by one.
 constexpr int MAX_TABLES = 33;
 struct Jumps {
     const uint32_t* t[MAX_TABLES];  // t[l][s]: 2^l steps on from s
     int n;
 };
+template <int NW>
+__device__ __forceinline__ uint32_t jump(const Rows& R, const Jumps& J, uint32_t k, int l, uint32_t at) {
+    return J.n ? J.t[l][at] : next_node<NW>(R, k, at);
+}
 
 // The node d steps on from `at`, on a path that has it.
-__device__ __forceinline__ uint32_t steps_on(const Jumps& J, uint32_t at, uint32_t d) {
-    for (int l = 0; l < J.n; ++l)
+template <int NW>
+__device__ __forceinline__ uint32_t steps_on(const Rows& R, const Jumps& J, uint32_t k, uint32_t at, uint32_t d) {
+    const int top = J.n ? J.n - 1 : 0;
+    for (uint32_t i = d >> top; i; --i) at = jump<NW>(R, J, k, top, at);
+    for (int l = 0; l < top; ++l)
         if ((d >> l) & 1u) at = J.t[l][at];
     return at;
 }
@@ -356,12 +365,14 @@ __global__ void __launch_bounds__(256) k_paths(Rows R, Jumps J, uint32_t k, cons
             p.first = (uint32_t)(r << 1) | (c_rc ? 1u : 0u);
             uint32_t at = p.first;
             uint64_t nodes = 1;
-            for (int l = J.n - 1; l >= 0; --l) {
-                const uint32_t nx = J.t[l][at];
+            const int top = J.n ? J.n - 1 : 0;
+            for (int l = top; l >= 0;) {
+                const uint32_t nx = jump<NW>(R, J, k, l, at);
                 if (nx != NO_NODE) {
                     at = nx;
                     nodes += 1ULL << l;
                 }
+                if (l < top || nx == NO_NODE || nodes > 2 * R.n) --l;
             }
             if (nodes > 2 * R.n) {  // more than there are directed nodes: impossible for valid rows
                 atomicOr(status, ST_SPIN_TIMEOUT);
@@ -380,7 +391,7 @@ __global__ void __launch_bounds__(256) k_paths(Rows R, Jumps J, uint32_t k, cons
                 // its own reverse complement: past its middle every edge has been used already,
                 // in the other direction, and the walk ends there (build.rs:349-445)
                 p.nodes = (p.nodes + 1) / 2;
-                const uint32_t at = steps_on(J, p.first, p.nodes - 1);
+                const uint32_t at = steps_on<NW>(R, J, k, p.first, p.nodes - 1);
                 take_edge<NW>(R, k, at >> 1, at & 1u, only_edge(R.mask[at >> 1], at & 1u), f, rv, rc_p, c_rc);
             }
         }
@@ -419,7 +430,7 @@ __global__ void __launch_bounds__(256) k_path_bases(Rows R, Jumps J, uint32_t k,
             const uint64_t end = min(p1, off[s] + L);
             uint32_t j = (uint32_t)(p - off[s]);
             uint32_t at = path.first;
-            if (j > k) at = steps_on(J, at, j - k - 1);  // node j - k (1-based)
+            if (j > k) at = steps_on<NW>(R, J, k, at, j - k - 1);  // node j - k (1-based)
             unsigned long long c = 0;
             Key<NW> head;
             if (j < k) {
@@ -442,7 +453,7 @@ __global__ void __launch_bounds__(256) k_path_bases(Rows R, Jumps J, uint32_t k,
                     b = only_edge(R.mask[row], at & 1u);
                     c += R.cov[row];
                     visited[row] = 1;
-                    at = J.t[0][at];
+                    at = jump<NW>(R, J, k, 0, at);
                 }
                 seqs[off[s] + (path.flip == 1 ? L - 1 - j : j)] = "ACGT"[path.flip == 1 ? 3u - b : b];
             }
@@ -662,19 +673,34 @@ fbk_status compact_impl(fbk_table* t, fbk_unitigs* U) {
     Launch L = launch_cfg(ctx, 256, 0);
     uint64_t cap = 1;
     while (cap < 2 * n) cap <<= 1;
+    Jumps J{};
     struct Bufs {
         fbk_ctx* c;
+        Jumps* J;
         std::vector<void*> p;
+        // where memory is short the highest tables make room: the paths are found with fewer
         void* get(uint64_t b) {
             void* q = dev_alloc(c, b);
+            while (!q && J->n) {
+                void* t = (void*)J->t[--J->n];
+                p.erase(std::find(p.begin(), p.end(), t));
+                cudaStreamSynchronize(c->stream);
+                dev_free(c, t);
+                q = dev_alloc(c, b);
+            }
             if (q) p.push_back(q);
             return q;
+        }
+        uint32_t* table(uint64_t b) {
+            void* q = dev_alloc(c, b);
+            if (q) p.push_back(q);
+            return (uint32_t*)q;
         }
         ~Bufs() {
             cudaStreamSynchronize(c->stream);
             for (void* q : p) dev_free(c, q);
         }
-    } B{ctx, {}};
+    } B{ctx, &J, {}};
     uint32_t* idx = (uint32_t*)B.get(cap * 4);
     uint8_t* visited = (uint8_t*)B.get(n);
     uint64_t* pre = (uint64_t*)B.get((n + 1) * 8);
@@ -682,10 +708,7 @@ fbk_status compact_impl(fbk_table* t, fbk_unitigs* U) {
     uint64_t* part = (uint64_t*)B.get(tiles * 8);
     uint32_t* any = (uint32_t*)B.get(4 * MAX_TABLES);
     uint8_t* flag = (uint8_t*)B.get(n);
-    Jumps J{};
-    auto table = [&]() { return (uint32_t*)B.get(2 * n * 4); };
-    uint32_t* last = table();
-    if (!idx || !visited || !pre || !part || !any || !flag || !last) return set_err(ctx, FBK_ERR_OOM, "compaction index");
+    if (!idx || !visited || !pre || !part || !any || !flag) return set_err(ctx, FBK_ERR_OOM, "compaction index");
     CK(ctx, cudaMemsetAsync(idx, 0, cap * 4, ctx->stream));
     CK(ctx, cudaMemsetAsync(visited, 0, n, ctx->stream));
     CK(ctx, cudaMemsetAsync(any, 0, 4 * MAX_TABLES, ctx->stream));
@@ -696,30 +719,32 @@ fbk_status compact_impl(fbk_table* t, fbk_unitigs* U) {
                                  cudaGetLastError()));
     TIMED(ctx, "compact_count", (k_tile_sums<<<(unsigned)tiles, 256, 0, ctx->stream>>>(StartCount{t->out_mask}, n, part), cudaGetLastError()));
     TIMED(ctx, "compact_count", (k_tile_prefix<<<(unsigned)tiles, 256, 0, ctx->stream>>>(StartCount{t->out_mask}, n, part, pre), cudaGetLastError()));
-    TIMED(ctx, "compact_next", (k_next<NW><<<L.grid, L.block, 0, ctx->stream>>>(R, k, last), cudaGetLastError()));
-    J.t[J.n++] = last;
-    // Tables until none of their entries is left (a path of 2^l nodes needs l + 1 of them; an
-    // isolated cycle never runs out, so there are at most as many as the nodes can fill).
-    // The host looks after every four.
     uint64_t* h = (uint64_t*)ctx->h_pinned;
-    for (bool more = true; more;) {
-        for (int q = 0; q < 4 && more; ++q) {
-            if ((1ULL << (J.n - 1)) > n) {
-                more = false;
-                break;
-            }
-            uint32_t* up = table();
-            if (!up) return set_err(ctx, FBK_ERR_OOM, "compaction tables");
-            TIMED(ctx, "compact_next", (k_double<<<L.grid, L.block, 0, ctx->stream>>>(last, up, 2 * n, any + J.n), cudaGetLastError()));
-            J.t[J.n++] = last = up;
-        }
-        if (!more) break;
-        CK(ctx, cudaMemcpyAsync(h, any + J.n - 1, 4, cudaMemcpyDeviceToHost, ctx->stream));
-        CK(ctx, cudaStreamSynchronize(ctx->stream));
-        more = *(uint32_t*)h != 0;
-    }
     CK(ctx, cudaMemcpyAsync(h, pre + n, 8, cudaMemcpyDeviceToHost, ctx->stream));
-    CK(ctx, cudaStreamSynchronize(ctx->stream));
+    // Tables until none of their entries is left (a path of 2^l nodes needs l + 1 of them; an
+    // isolated cycle never runs out, so there are at most as many as the nodes can fill), or
+    // there is no path, or no memory for more: 8 bytes a row each, of at most half of what a
+    // pool has free, which other contexts may share.  The host looks after every four.
+    uint64_t room = ~0ULL, largest = 0;
+    if (ctx->pool && ctx->pool->active()) fbk_ctx_pool_free(ctx, &room, &largest), room /= 2;
+    for (bool more = true; more;) {
+        for (int q = J.n ? 0 : -1; q < 4 && more; ++q) {
+            uint32_t* up = nullptr;
+            if ((J.n == 0 || (1ULL << (J.n - 1)) <= n) && room >= 8 * n * (J.n + 1ULL)) up = B.table(8 * n);
+            more = up != nullptr;
+            if (!up) break;
+            if (J.n == 0) {
+                TIMED(ctx, "compact_next", (k_next<NW><<<L.grid, L.block, 0, ctx->stream>>>(R, k, up), cudaGetLastError()));
+            } else {
+                TIMED(ctx, "compact_next", (k_double<<<L.grid, L.block, 0, ctx->stream>>>(J.t[J.n - 1], up, 2 * n, any + J.n),
+                                            cudaGetLastError()));
+            }
+            J.t[J.n++] = up;
+        }
+        if (more) CK(ctx, cudaMemcpyAsync(h + 1, any + J.n - 1, 4, cudaMemcpyDeviceToHost, ctx->stream));
+        CK(ctx, cudaStreamSynchronize(ctx->stream));
+        more = more && h[0] && *(uint32_t*)(h + 1) != 0;
+    }
     const uint64_t n_starts = h[0];
     U->linear_walks = n_starts;
     std::vector<uint32_t> hlen(n_starts);

@@ -2,8 +2,12 @@
 (no 1-in-1-out node, one, and around the powers of two), at the word edges of the key, and
 for a path whose first k bases equal its reverse complement's, against the oracle (sequences, edges and
 coverages, as test_gpu_parity.compare_compaction compares them)."""
+import ctypes as C
+
+import numpy as np
 import pytest
 
+from fastbact_gb300 import _native as N
 from fastbact_gb300 import api
 from test_gpu_parity import compare_compaction, rand_seqs
 
@@ -48,3 +52,46 @@ def test_hairpin_on_a_branch(ctx, k, kb):
     seqs = [stem + stem[::-1].translate(COMP), a + b]
     bank = api.ReadBank(merged_reads=api.BitSeqArena.from_seqs([s for s in seqs for _ in range(4)]))
     compare_compaction(ctx, bank, k, kb, 16, None, 14)
+
+
+@pytest.mark.parametrize("k,kb", [(31, 64), (77, 256)])
+def test_less_memory_than_tables(k, kb):
+    """A pool with room for some of the tables, for one, and for none: the same unitigs from
+    fewer of them, an isolated cycle (whose tables never run out) among them."""
+    x, line, ring = (rand_seqs(90 + i, 1, n, n)[0] for i, n in enumerate((3000, 60_000, 40_000)))
+    pal = x + x[::-1].translate(COMP)
+    seqs = [s[i:i + 250] for s in (line, ring + ring[:300], pal) for i in range(0, len(s) - 249, 25)] + [line[-300:], pal[:300]] * 2
+    seqs += [rand_seqs(200 + m, 1, k + 1 + m, k + 1 + m)[0] for m in (0, 1, 2, 7, 8, 9, 40)] * 4
+    c = api.Context(0, pool_bytes=512 << 20)
+
+    def largest():
+        free, block = C.c_uint64(), C.c_uint64()
+        N.check(N.lib().fbk_ctx_pool_free(c.handle, C.byref(free), C.byref(block)), c.handle)
+        return block.value
+
+    try:
+        bank = api.ReadBank(merged_reads=api.BitSeqArena.from_seqs(seqs))
+        table = api.build_cdbg_with_contigs_ext(bank, [], k, None, None, ctx=c, key_bits=kb, counter_bits=16, cms_log2_width=18)
+        n = table.info()[1]
+        seq, cov, circ, edges = api.compact(table)
+        want = sorted(zip(seq, cov.tolist(), circ.tolist()))
+        assert circ.sum() == 1 and max(map(len, seq)) > 50_000
+        index = 4 * (1 << (2 * n - 1).bit_length())
+        counts = []
+        c.set_timing(True)
+        for rest in (1 << 40, 120 * n, 60 * n, 32 * n, 22 * n, 12 * n):   # besides the index; the last holds no table
+            fill, p = [], 18
+            while p >= 4:                   # a sketch of 4 << p bytes at a time
+                if largest() - (4 << p) >= index + rest:
+                    fill.append(api.HyperLogLog(p, c))
+                else:
+                    p -= 1
+            c.timing_reset()
+            seq, cov, circ, edges = api.compact(table)
+            counts.append(c.timing("compact_next")[1])
+            assert sorted(zip(seq, cov.tolist(), circ.tolist())) == want
+            for f in fill:
+                f.release()
+        assert counts[-1] == 0 and sorted(counts, reverse=True) == counts and len(set(counts)) > 3
+    finally:
+        c.close()
