@@ -551,7 +551,9 @@ cudaError_t copy_h2d_from(fbk_ctx* ctx, void* dst, size_t bytes, const std::func
     if (bytes < STAGE_MIN) {
         std::vector<char> all(bytes);
         *ok = read(all.data(), 0, bytes);
-        return *ok ? cudaMemcpyAsync(dst, all.data(), bytes, cudaMemcpyHostToDevice, ctx->stream) : cudaSuccess;
+        if (!*ok) return cudaSuccess;
+        const cudaError_t e = cudaMemcpyAsync(dst, all.data(), bytes, cudaMemcpyHostToDevice, ctx->stream);
+        return e == cudaSuccess ? cudaStreamSynchronize(ctx->stream) : e;  // the bytes go with this scope
     }
     std::atomic<bool> good{true};
     const cudaError_t e = staged_h2d(ctx, dst, bytes, [&](void* slot, size_t o, size_t n) {

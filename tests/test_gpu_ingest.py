@@ -5,6 +5,7 @@ scores (repeats), adapters at every place, short and long ends of bad quality, a
 at the edges of its tiles; texts with '\\r' and without a last newline, from memory and from
 files."""
 import ctypes as C
+import os
 
 import numpy as np
 import pytest
@@ -81,3 +82,45 @@ def test_pairs_match_oracle(ctx, tmp_path, n, opts):
         assert np.array_equal(x, y)
     bank.release()
     crlf.release()
+
+
+@pytest.mark.parametrize("n", [40, 30_000])  # below and above the size that goes through the staging slots
+def test_files_that_cannot_be_read(ctx, tmp_path, n):
+    """A pipe, a closed or write-only descriptor and a directory in either place are refused;
+    the same files are read afterwards, their positions unmoved."""
+    ps = pairs(7, 40) * (n // 40)
+    paths = [tmp_path / "e_1.fq", tmp_path / "e_2.fq"]
+    for m, p in enumerate(paths):
+        p.write_bytes(text(ps, m))
+    assert (paths[0].stat().st_size > 4 << 20) == (n > 40)
+
+    def ingest(fd1, fd2):
+        h, st = C.c_void_p(), N.IngestStatsC()
+        N.check(N.lib().fbk_ingest_fastq_fd_device(ctx.handle, fd1, fd2, 1.0, 1, 20, 1, 1, 0, C.byref(h), C.byref(st)), ctx.handle)
+        return api.DeviceBank.from_handle(ctx, h), st
+
+    r, w = os.pipe()
+    write_only, folder = os.open(paths[1], os.O_WRONLY), os.open(tmp_path, os.O_RDONLY)
+    good = [os.open(p, os.O_RDONLY) for p in paths]
+    os.lseek(good[0], 17, os.SEEK_SET)
+    closed = os.dup(r)
+    os.close(closed)
+    try:
+        for bad in (r, closed, write_only, folder):
+            for fds in ((bad, good[1]), (good[0], bad)):
+                with pytest.raises(N.FbkError, match="FBK_ERR_IO"):
+                    ingest(*fds)
+        bank, st = ingest(*good)
+        assert st.input_read_pairs == len(ps) and os.lseek(good[0], 0, os.SEEK_CUR) == 17
+        a, b = (np.frombuffer(p.read_bytes(), np.uint8) for p in paths)
+        h, st = C.c_void_p(), N.IngestStatsC()
+        N.check(N.lib().fbk_ingest_fastq_device(ctx.handle, N.ptr(a), a.size, N.ptr(b), b.size, 1.0, 1, 20, 1, 1, 0, C.byref(h), C.byref(st)),
+                ctx.handle)
+        memory = api.DeviceBank.from_handle(ctx, h)
+        for x, y in zip(bank.export(), memory.export()):
+            assert np.array_equal(x, y)
+        bank.release()
+        memory.release()
+    finally:
+        for fd in (r, w, write_only, folder, *good):
+            os.close(fd)
