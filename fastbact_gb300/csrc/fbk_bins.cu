@@ -9,9 +9,11 @@
 //      bin of its minimizer;
 //   2. the runs are scattered by bin (k_bin_scan*, k_bin_scatter): all occurrences of a
 //      k-mer lie in one bin;
-//   3. k_bin_agg takes groups of consecutive bins, about as many as fill a hash table in
-//      shared memory, reads their windows' bases from the packed bank again and adds up,
-//      per distinct canonical k-mer, its 8 edge counts (build.rs:243-289 without the gate).
+//   3. the windows of bins with many times the others' are scattered again, by their keys
+//      (split_heavy); k_bin_agg takes those and groups of consecutive bins, about as many as
+//      fill a hash table in shared memory, reads their windows' bases from the packed bank
+//      again and adds up, per distinct canonical k-mer, its 8 edge counts (build.rs:243-289
+//      without the gate).
 //      A key seen twice or more becomes a row of a dense array; of a key seen once, only
 //      its place in the bank is kept, as a bit of a bitmap over the bases;
 //   4. every distinct key enters the pass-1 sketch with its whole count at once
@@ -225,9 +227,10 @@ __global__ void __launch_bounds__(256) k_bin_scan_sums(const unsigned long long*
         part[blockIdx.x] = v;
     }
 }
+// big (not null): the windows in bins of more than 2^13, 2^15 and 2^17 of them.
 __global__ void __launch_bounds__(256) k_bin_scan(const unsigned long long* __restrict__ hist, uint32_t n,
                                                   const unsigned long long* __restrict__ part, unsigned long long* __restrict__ pre,
-                                                  uint32_t* __restrict__ cursor) {
+                                                  uint32_t* __restrict__ cursor, unsigned long long* __restrict__ big) {
     __shared__ unsigned long long s[8], s_base;
     const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     unsigned long long v = 0;
@@ -264,6 +267,11 @@ __global__ void __launch_bounds__(256) k_bin_scan(const unsigned long long* __re
         }
         p += x[j];
         if (i0 + j == n - 1) pre[n] = p;
+        const uint32_t windows = (uint32_t)x[j];
+        if (big && windows > 1u << 13) {  // rare
+            for (int c = 0; c < 3; ++c)
+                if (windows > 1u << (13 + 2 * c)) atomicAdd(&big[c], (unsigned long long)windows);
+        }
     }
 }
 
@@ -381,10 +389,106 @@ __device__ __forceinline__ uint64_t fold_of(const uint64_t (&w)[NK]) {
     return f;
 }
 
+// Heavy bins.  A minimizer that is frequent in the genome (poly-A, the short words of an AT-rich
+// one) brings many keys into one bin, which is one block's: it took them in parts as large as its
+// table, each over all of the bin's windows.  So the windows of a bin of more than three
+// target groups are scattered again, most as runs of one window, over sub-bins of about `target`
+// windows by a hash of the key, and these are groups of their own.  Reads of 150 bases at 60x, the
+// whole build over records / with heavy bins taken in parts / so, in ms:
+//   5 Mbp, GC 0.15, k = 21                       12.9 / 45.2 / 10.2
+//   5 Mbp, GC 0.2, a tract of A or T every 500   17.1 / 53.2 /  9.6   (k = 77 13.3 / 27.3 / 7.7)
+//   12 Mbp, GC 0.2, a tract every 1000           41.4 / 116  / 24.8   (k = 31 33.7 / 56.8 / 17.5)
+// Bins of 2^13 windows and fewer stay whole (0.03 ms of a block's time a part).  Pieces of such a
+// bin's runs:
+struct HeavyPiece {
+    uint32_t begin, end;  // runs
+    uint32_t sub, parts;  // sub-bins [sub, sub + parts)
+};
+constexpr uint32_t HEAVY_PIECE = 1024;  // runs
+// counts: pieces, sub-bins.
+__global__ void k_heavy_pieces(const unsigned long long* __restrict__ pre, uint32_t n, uint32_t target, uint32_t from,
+                               HeavyPiece* __restrict__ pieces, uint32_t cap, uint32_t* __restrict__ counts) {
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const unsigned long long a = pre[i], b = pre[i + 1];
+        const uint32_t windows = (uint32_t)b - (uint32_t)a;
+        if (windows <= from) continue;
+        const uint32_t r0 = (uint32_t)(a >> 32), r1 = (uint32_t)(b >> 32), np = (r1 - r0 + HEAVY_PIECE - 1) / HEAVY_PIECE;
+        const uint32_t parts = windows / target + 1, sub = atomicAdd(counts + 1, parts), p = atomicAdd(counts, np);
+        for (uint32_t q = 0; q < np && p + q < cap; ++q)
+            pieces[p + q] = {r0 + q * HEAVY_PIECE, min(r1, r0 + (q + 1) * HEAVY_PIECE), sub, parts};
+    }
+}
+
+// Counts the windows of the pieces by sub-bin (PUT: moves them there), a block per piece, a warp
+// per 32 runs, a lane per window.  Windows of one sub-bin that meet in a warp share an atomic.
+template <int NK, bool PUT>
+__global__ void __launch_bounds__(256) k_heavy_split(const uint64_t* __restrict__ data, const uint64_t* __restrict__ runs,
+                                                     const HeavyPiece* __restrict__ pieces, const uint32_t* __restrict__ counts, uint32_t cap,
+                                                     uint32_t k, unsigned long long* __restrict__ hist, uint32_t* __restrict__ cursor,
+                                                     uint64_t* __restrict__ out, uint64_t cap_out) {
+    const uint32_t lane = threadIdx.x & 31;
+    const uint32_t* __restrict__ d32 = reinterpret_cast<const uint32_t*>(data);
+    const uint32_t n_pieces = min(counts[0], cap);
+    for (uint32_t p = blockIdx.x; p < n_pieces; p += gridDim.x) {
+        const HeavyPiece piece = pieces[p];
+        for (uint32_t r = piece.begin + (threadIdx.x & ~31u); r < piece.end; r += 256) {
+            const uint64_t e = r + lane < piece.end ? runs[r + lane] : 0;
+            const uint32_t n = (uint32_t)(e >> 32) & 0xFFFu;
+            uint32_t inc = n;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(0xffffffffu, inc, o);
+                if (lane >= (uint32_t)o) inc += y;
+            }
+            // (the windows of the runs one after another, as in k_bin_agg)
+            const uint32_t total = __shfl_sync(0xffffffffu, inc, 31), first = inc - n, shift = (uint32_t)e - first;
+            const uint32_t edge_l = (e >> 44) & 1u ? 0xFFFFFFFFu : first, edge_r = (e >> 45) & 1u ? 0xFFFFFFFFu : inc - 1;
+            for (uint32_t base = 0, before = 0; base < total; base += 32) {
+                const uint32_t rel = first - base;
+                const uint32_t starts = __reduce_or_sync(0xffffffffu, n && rel < 32 ? 1u << rel : 0u);
+                const int run = (int)(before + __popc(starts & ((2u << lane) - 1))) - 1;
+                before += __popc(starts);
+                const bool live = base + lane < total;
+                const uint32_t x = min(base + lane, total - 1);
+                const uint32_t g = __shfl_sync(0xffffffffu, shift, run) + x;
+                const bool has_l = __shfl_sync(0xffffffffu, edge_l, run) != x, has_r = __shfl_sync(0xffffffffu, edge_r, run) != x;
+                uint64_t key[NK];
+                bool rc;
+                uint32_t bl, br;
+                window_at<NK>(d32, g, k, key, rc, bl, br);
+                // (not the hash that places a key in a block's table or that takes a group in parts)
+                const uint64_t f = fold_of<NK>(key);
+                const uint32_t sub = live ? piece.sub + __umulhi((uint32_t)(((f ^ (f >> 29)) * 0xD6E8FEB86659FD93ULL) >> 32), piece.parts) : 0xFFFFFFFFu;
+                // windows of a run that follow one another into the same sub-bin (poly-G) stay a run
+                const uint32_t sub_before = __shfl_up_sync(0xffffffffu, sub, 1);
+                const int run_before = __shfl_up_sync(0xffffffffu, run, 1);
+                const bool head = live && (lane == 0 || run != run_before || sub != sub_before);
+                const uint32_t heads = __ballot_sync(0xffffffffu, head), lives = __ballot_sync(0xffffffffu, live);
+                const uint32_t same = __match_any_sync(0xffffffffu, sub);  // its first lane is a head
+                const int leader = __ffs(same) - 1;
+                const uint32_t n_same = __popc(same & heads);
+                if constexpr (PUT) {
+                    uint32_t at = 0;
+                    if (live && (int)lane == leader) at = atomicAdd(&cursor[sub], n_same);
+                    at = __shfl_sync(0xffffffffu, at, leader) + __popc(same & heads & ((1u << lane) - 1));
+                    const uint32_t above = heads & ~((2u << lane) - 1);
+                    const uint32_t len = (above ? __ffs(above) - 1 : __popc(lives)) - lane;
+                    const bool last_r = __shfl_sync(0xffffffffu, has_r, min(lane + (head ? len : 1u) - 1, 31u));
+                    if (head && at < cap_out) out[at] = run_pack(g, len, has_l, last_r, 0);
+                } else if (live && (int)lane == leader) {
+                    atomicAdd(&hist[sub], ((unsigned long long)n_same << 32) | (uint32_t)__popc(same));
+                }
+            }
+        }
+    }
+}
+
 // Counters of a build (u64): rows, low rows, keys seen once, adjacent solid windows, reads of one
 // window; of the sample: distinct keys, those seen twice, those that can become solid, windows;
-// log words a warp needed; groups handed out (aggregate, sample).
-enum { BC_ROWS, BC_LOW, BC_SINGLES, BC_PAIRS, BC_LONE, BC_DISTINCT, BC_MULTI, BC_KEPT, BC_WINDOWS, BC_NEED, BC_WORK, BC_WORK_S, BC_N };
+// log words a warp needed; groups handed out (aggregate, sample); windows in large bins
+// (k_bin_scan).
+enum { BC_ROWS, BC_LOW, BC_SINGLES, BC_PAIRS, BC_LONE, BC_DISTINCT, BC_MULTI, BC_KEPT, BC_WINDOWS, BC_NEED, BC_WORK, BC_WORK_S,
+       BC_BIG, BC_N = BC_BIG + 3 };
 
 struct FirstKey {
     uint64_t raw;        // canonical ntHash
@@ -396,6 +500,9 @@ struct AggArgs {
     const unsigned long long* start;  // group g: runs and windows [start[g], start[g + stride])
     uint32_t stride;                  // 1; in a sample group g is bin g * stride of the bins' prefixes
     uint32_t n_groups;
+    const uint64_t* heavy_runs;               // the first n_heavy groups: sub-bins of the heavy bins (HeavyBins)
+    const unsigned long long* heavy_start;
+    uint32_t n_heavy, heavy_from;             // a group of more windows than that is a heavy bin, and passed over
     uint32_t k;
     uint32_t mtc;                // 0: every key seen twice is a row; else those with an edge count of mtc, the rest are low
     uint32_t* single;            // bit g: the window at base g holds a key seen once
@@ -407,7 +514,7 @@ struct AggArgs {
     uint64_t* low_keys;          // NK words each
     uint64_t cap_low;
     uint64_t* later;             // two lists of later_cap runs a block (see k_bin_agg)
-    uint32_t later_cap;
+    uint32_t later_cap, max_blocks;
     unsigned long long* counters;
     uint32_t* status;
     FirstKey* firsts;            // AGG_FIRST: the keys (cap_rows of them)
@@ -559,20 +666,25 @@ __global__ void __launch_bounds__(AGG_THREADS, 2) k_bin_agg(AggArgs A) {
     auto fetch = [&]() {  // thread 0: the block's next group
         const unsigned long long g = atomicAdd(&A.counters[SAMPLE ? BC_WORK_S : BC_WORK], 1ULL);
         s_next[0] = g;
-        if (g < A.n_groups) {
-            s_next[1] = A.start[g * A.stride];
-            s_next[2] = A.start[g * A.stride + 1];
+        if (g < A.n_heavy) {
+            s_next[1] = A.heavy_start[g];
+            s_next[2] = A.heavy_start[g + 1];
+        } else if (g < A.n_heavy + A.n_groups) {
+            s_next[1] = A.start[(g - A.n_heavy) * A.stride];
+            s_next[2] = A.start[(g - A.n_heavy) * A.stride + 1];
         }
     };
     if (threadIdx.x == 0) fetch();
     block_sync();
-    while (s_next[0] < A.n_groups) {
+    while (s_next[0] < A.n_heavy + A.n_groups) {
         const unsigned long long p0 = s_next[1], p1 = s_next[2];
-        const uint32_t e0 = (uint32_t)(p0 >> 32), n_runs = (uint32_t)(p1 >> 32) - e0;
+        const bool sub = s_next[0] < A.n_heavy;
+        const uint64_t* runs = (sub ? A.heavy_runs : A.runs) + (uint32_t)(p0 >> 32);
+        const uint32_t n_runs = (uint32_t)(p1 >> 32) - (uint32_t)(p0 >> 32);
         const uint32_t windows = (uint32_t)p1 - (uint32_t)p0;
         const bool wide = !FIRST && windows > AGG_NARROW_MAX;
         block_sync();  // everyone has read s_next
-        if (n_runs == 0 || (SAMPLE && wide)) {
+        if (n_runs == 0 || (!sub && windows > A.heavy_from)) {
             if (threadIdx.x == 0) fetch();
             block_sync();
             continue;
@@ -611,7 +723,7 @@ __global__ void __launch_bounds__(AGG_THREADS, 2) k_bin_agg(AggArgs A) {
             if constexpr (COUNT) sh_add_if(on && !(w.rc ? has_l : has_r), elack + 4 * entry, 1);
         };
         uint64_t lo = 0, width = 1ULL << 32;  // the part of the hash range being counted
-        const uint64_t* src = A.runs + e0;    // the group's runs, or the windows put off
+        const uint64_t* src = runs;           // the group's runs, or the windows put off
         uint32_t n_src = n_runs;
         uint64_t* later = A.later + (uint64_t)blockIdx.x * 2 * A.later_cap;
         bool fetched = false;
@@ -807,7 +919,7 @@ __global__ void __launch_bounds__(AGG_THREADS, 2) k_bin_agg(AggArgs A) {
             if (s_full) {
                 block_sync();
                 // from the start of this part of the group, in halves
-                src = A.runs + e0;
+                src = runs;
                 n_src = n_runs;
                 if (width == 1) {
                     // more keys of one hash value than a table holds
@@ -944,7 +1056,7 @@ __global__ void __launch_bounds__(AGG_THREADS, 2) k_bin_agg(AggArgs A) {
                 src = later + A.later_cap;
                 n_src = n_later;
             } else {
-                src = A.runs + e0;
+                src = runs;
                 n_src = n_runs;
                 lo += width;
             }
@@ -1307,19 +1419,19 @@ int resident_grid(K kernel, int block, size_t smem, int sms) {
 }
 
 template <int NW, int WS, int MODE>
-cudaError_t agg_launch(cudaStream_t st, int sms, const AggArgs& A) {
+cudaError_t agg_launch(cudaStream_t st, const AggArgs& A) {
     auto kern = k_bin_agg<NW, WS, MODE>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)AGG_SMEM);
     if (e != cudaSuccess) return e;
-    const int grid = std::min<int>(2 * sms, (int)std::max<uint32_t>(1, A.n_groups));  // later holds that many
+    const int grid = (int)std::min<uint64_t>(A.max_blocks, std::max<uint64_t>(1, (uint64_t)A.n_heavy + A.n_groups));
     kern<<<grid, AGG_THREADS, AGG_SMEM, st>>>(A);
     return cudaGetLastError();
 }
 // The modes that write no rows know a key by its significant words alone.
 template <int MODE>
-cudaError_t agg_launch_nk(int nk, cudaStream_t st, int sms, const AggArgs& A) {
-    return nk == 1 ? agg_launch<1, 0, MODE>(st, sms, A) : nk == 2 ? agg_launch<2, 0, MODE>(st, sms, A)
-           : nk == 3 ? agg_launch<3, 0, MODE>(st, sms, A) : agg_launch<4, 0, MODE>(st, sms, A);
+cudaError_t agg_launch_nk(int nk, cudaStream_t st, const AggArgs& A) {
+    return nk == 1 ? agg_launch<1, 0, MODE>(st, A) : nk == 2 ? agg_launch<2, 0, MODE>(st, A)
+           : nk == 3 ? agg_launch<3, 0, MODE>(st, A) : agg_launch<4, 0, MODE>(st, A);
 }
 template <class Kern, class... Args>
 cudaError_t stream_launch(cudaStream_t st, int sms, uint64_t n_threads, Kern kern, Args... args) {
@@ -1430,7 +1542,7 @@ fbk_status bin_runs(fbk_ctx* ctx, Scratch& B, BinRuns& R, const BankDev& bv, uin
                cudaGetLastError()));
         const unsigned tiles = (F + SCAN_TILE - 1) / SCAN_TILE;
         TIMED(ctx, R.est ? "est_scan" : "bins_scan", (k_bin_scan_sums<<<tiles, 256, 0, stream>>>(R.hist, F, part), cudaGetLastError()));
-        TIMED(ctx, R.est ? "est_scan" : "bins_scan", (k_bin_scan<<<tiles, 256, 0, stream>>>(R.hist, F, part, R.pre, cursor), cudaGetLastError()));
+        TIMED(ctx, R.est ? "est_scan" : "bins_scan", (k_bin_scan<<<tiles, 256, 0, stream>>>(R.hist, F, part, R.pre, cursor, R.counters + BC_BIG), cudaGetLastError()));
         TIMED(ctx, R.est ? "est_scatter" : "bins_scatter",
               (k_bin_scatter<<<(unsigned)n_blocks, 256, 0, stream>>>(log, log_n, (uint32_t)cap_w, cursor, R.runs, n_warps * cap_w),
                cudaGetLastError()));
@@ -1439,7 +1551,9 @@ fbk_status bin_runs(fbk_ctx* ctx, Scratch& B, BinRuns& R, const BankDev& bv, uin
             sample->n_groups = std::min<uint32_t>(F, 1024);
             sample->stride = F / sample->n_groups;
             sample->start = R.pre;
-            TIMED(ctx, R.est ? "est_sample" : "bins_sample", agg_launch_nk<AGG_SAMPLE>((int)((k + 31) / 32), stream, sms, *sample));
+            // (a heavy bin is no sample of the others, and its keys would be taken in parts)
+            sample->heavy_from = (uint32_t)std::min<uint64_t>(AGG_NARROW_MAX, std::max<uint64_t>(8192, 8 * windows / F));
+            TIMED(ctx, R.est ? "est_sample" : "bins_sample", agg_launch_nk<AGG_SAMPLE>((int)((k + 31) / 32), stream, *sample));
         }
         CK(ctx, cudaMemcpyAsync(h, R.counters, 8 * BC_N, cudaMemcpyDeviceToHost, stream));
         CK(ctx, cudaMemcpyAsync(h + BC_N, R.pre + F, 8, cudaMemcpyDeviceToHost, stream));
@@ -1464,6 +1578,55 @@ fbk_status bin_runs(fbk_ctx* ctx, Scratch& B, BinRuns& R, const BankDev& bv, uin
 uint64_t group_windows(uint32_t entries, uint64_t n_windows, uint64_t distinct) {
     const uint64_t t = (uint64_t)(0.7 * (double)entries * (double)std::max<uint64_t>(n_windows, 1) / (double)std::max<uint64_t>(distinct, 1));
     return std::max<uint64_t>(512, std::min<uint64_t>(t, 60000));
+}
+
+// The heavy bins' windows by sub-bin, for groups of `target` windows; A then takes them first and
+// passes their bins over.  h: the counters on the host.  Where there is no memory for it, A
+// keeps the bins as they are.
+fbk_status split_heavy(fbk_ctx* ctx, Scratch& B, const BinRuns& R, const unsigned long long* h, uint64_t target, AggArgs& A) {
+    A.n_heavy = 0;
+    A.heavy_from = 0xFFFFFFFFu;
+    // a group of ordinary bins stays below three targets (k_bin_groups)
+    const uint32_t from = (uint32_t)std::max<uint64_t>(3 * target, 1u << 13);
+    const uint64_t windows = h[BC_BIG + (from >= 1u << 17 ? 2 : from >= 1u << 15 ? 1 : 0)];  // no fewer than they have
+    if (!windows) return FBK_OK;
+    const cudaStream_t stream = ctx->stream;
+    const uint32_t cap = (uint32_t)(windows / HEAVY_PIECE + windows / from + 1), n_sub = (uint32_t)(windows / target + windows / from + 1);
+    const uint32_t tiles = (n_sub + SCAN_TILE - 1) / SCAN_TILE;
+    HeavyPiece* pieces = (HeavyPiece*)B.get(sizeof(HeavyPiece) * cap);
+    unsigned long long* hist = (unsigned long long*)B.get(8ULL * (n_sub + 1));  // and the two counts
+    unsigned long long* pre = (unsigned long long*)B.get(8ULL * (n_sub + 1 + tiles));
+    uint32_t* cursor = (uint32_t*)B.get(4ULL * n_sub);
+    uint64_t* runs = (uint64_t*)B.get(8 * windows);
+    if (!pieces || !hist || !pre || !cursor || !runs) return FBK_OK;
+    uint32_t* counts = (uint32_t*)(hist + n_sub);
+    CK(ctx, cudaMemsetAsync(hist, 0, 8ULL * (n_sub + 1), stream));
+    auto split = [&](auto put) {
+        constexpr bool PUT = decltype(put)::value;
+        auto launch = [&](auto nk) {
+            auto kern = k_heavy_split<decltype(nk)::value, PUT>;
+            kern<<<(unsigned)std::min<uint64_t>(resident_grid(kern, 256, 0, ctx->num_sms), cap), 256, 0, stream>>>(
+                A.data, R.runs, pieces, counts, cap, A.k, hist, cursor, runs, windows);
+            return cudaGetLastError();
+        };
+        using std::integral_constant;
+        const uint32_t nk = (A.k + 31) / 32;
+        return nk == 1 ? launch(integral_constant<int, 1>{}) : nk == 2 ? launch(integral_constant<int, 2>{})
+               : nk == 3 ? launch(integral_constant<int, 3>{}) : launch(integral_constant<int, 4>{});
+    };
+    TIMED(ctx, R.est ? "est_heavy" : "bins_heavy",
+          (k_heavy_pieces<<<std::min<unsigned>(1024, (R.F + 255) / 256), 256, 0, stream>>>(R.pre, R.F, (uint32_t)target, from, pieces, cap, counts),
+           cudaGetLastError()));
+    TIMED(ctx, R.est ? "est_heavy" : "bins_heavy", split(std::false_type{}));
+    TIMED(ctx, R.est ? "est_heavy" : "bins_heavy", (k_bin_scan_sums<<<tiles, 256, 0, stream>>>(hist, n_sub, pre + n_sub + 1), cudaGetLastError()));
+    TIMED(ctx, R.est ? "est_heavy" : "bins_heavy",
+          (k_bin_scan<<<tiles, 256, 0, stream>>>(hist, n_sub, pre + n_sub + 1, pre, cursor, nullptr), cudaGetLastError()));
+    TIMED(ctx, R.est ? "est_heavy" : "bins_heavy", split(std::true_type{}));
+    A.heavy_runs = runs;
+    A.heavy_start = pre;
+    A.n_heavy = n_sub;
+    A.heavy_from = from;
+    return FBK_OK;
 }
 
 }  // namespace
@@ -1504,7 +1667,8 @@ fbk_status bins_build(fbk_ctx* ctx, const fbk_bank* b, const fbk_build_params* p
     A.counters = counters;
     A.status = ctx->d_status;
     A.later_cap = sampled ? AGG_LATER : 4096;
-    A.later = (uint64_t*)B.get(16ULL * A.later_cap * (sampled ? 2 * sms : std::min<uint64_t>(2 * sms, windows / BINS_SMALL_GROUP + 1)));
+    A.max_blocks = (uint32_t)(sampled ? 2 * sms : std::min<uint64_t>(2 * sms, windows / BINS_SMALL_GROUP + 1));
+    A.later = (uint64_t*)B.get(16ULL * A.later_cap * A.max_blocks);
     if (!A.later) return set_err(ctx, FBK_ERR_OOM, "minimizer bins");
     unsigned long long* h = (unsigned long long*)ctx->h_pinned;
     const bool may_filter = p->min_trans_cov >= 2 && ctx->acc_filter != 0;
@@ -1530,6 +1694,9 @@ fbk_status bins_build(fbk_ctx* ctx, const fbk_bank* b, const fbk_build_params* p
     const uint32_t n_groups = (uint32_t)(n_windows / target + 1);
     unsigned long long* start = (unsigned long long*)B.get(8ULL * (n_groups + 1));
     if (!start) return set_err(ctx, FBK_ERR_OOM, "minimizer bins: groups");
+    A.runs = runs;
+    rs = split_heavy(ctx, B, R, h, target, A);
+    if (rs) return rs;
     fbk_table* tb = new fbk_table();
     tb->ctx = ctx;
     tb->nw = (uint32_t)nw;
@@ -1563,7 +1730,6 @@ fbk_status bins_build(fbk_ctx* ctx, const fbk_bank* b, const fbk_build_params* p
         if (lows) low = (uint64_t*)B.get(lows * 8 * nk);
         if (!tb->keys || (nw > 2 && !tb->tags) || !tb->cnt || (lows && !low)) return set_err(ctx, FBK_ERR_OOM, "solid table rows");
         const TableDev td = tbl_dev(tb);
-        A.runs = runs;
         A.start = start;
         A.stride = 1;
         A.n_groups = n_groups;
@@ -1580,7 +1746,7 @@ fbk_status bins_build(fbk_ctx* ctx, const fbk_bank* b, const fbk_build_params* p
                cudaGetLastError()));
         TIMED(ctx, "bins_aggregate", by_width(nw, k, [&](auto a, auto w) {
                   constexpr int NW = decltype(a)::value, WS = decltype(w)::value;
-                  return cms ? agg_launch<NW, WS, AGG_COUNT>(stream, sms, A) : agg_launch<NW, WS, AGG_BUILD>(stream, sms, A);
+                  return cms ? agg_launch<NW, WS, AGG_COUNT>(stream, A) : agg_launch<NW, WS, AGG_BUILD>(stream, A);
               }));
         CK(ctx, cudaMemcpyAsync(h, counters, 8 * BC_N, cudaMemcpyDeviceToHost, stream));
         CK(ctx, cudaMemcpyAsync(h + BC_N, ctx->d_status, 4, cudaMemcpyDeviceToHost, stream));
@@ -1689,7 +1855,8 @@ fbk_status bins_first(fbk_ctx* ctx, const fbk_bank* b, uint64_t n_reads, uint64_
     A.k = k;
     A.status = ctx->d_status;
     A.later_cap = AGG_LATER;
-    A.later = (uint64_t*)B.get(16ULL * A.later_cap * 2 * sms);
+    A.max_blocks = 2 * (uint32_t)sms;
+    A.later = (uint64_t*)B.get(16ULL * A.later_cap * A.max_blocks);
     if (!cleared || !A.later) return FBK_OK;
     R.hist = (unsigned long long*)cleared;
     A.counters = R.counters = R.hist + R.F;
@@ -1716,10 +1883,12 @@ fbk_status bins_first(fbk_ctx* ctx, const fbk_bank* b, uint64_t n_reads, uint64_
     A.firsts = (FirstKey*)B.get(A.cap_rows * sizeof(FirstKey));
     if (!start || !A.firsts) return FBK_OK;
     A.start = start;
+    st = split_heavy(ctx, B, R, h, target, A);
+    if (st) return st;
     TIMED(ctx, "est_groups", (k_bin_groups<<<std::min<unsigned>(1024, (R.F + 256) / 256), 256, 0, stream>>>(R.pre, R.F, (uint32_t)target,
                                                                                                           A.n_groups, start),
                                cudaGetLastError()));
-    TIMED(ctx, "est_first_keys", agg_launch_nk<AGG_FIRST>(nk, stream, sms, A));
+    TIMED(ctx, "est_first_keys", agg_launch_nk<AGG_FIRST>(nk, stream, A));
     CK(ctx, cudaMemcpyAsync(h, A.counters, 8 * BC_N, cudaMemcpyDeviceToHost, stream));
     CK(ctx, cudaMemcpyAsync(h + BC_N, ctx->d_status, 4, cudaMemcpyDeviceToHost, stream));
     CK(ctx, cudaStreamSynchronize(stream));

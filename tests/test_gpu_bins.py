@@ -261,3 +261,32 @@ def test_a_fork_builds_in_its_parents_form(option):
     finally:
         N.lib().fbk_ctx_destroy(h)
         c.close()
+
+
+def at_rich_reads(seed, genome_len, n, gc):
+    """150-base reads of a genome whose few frequent words are the minimizers of many k-mers, with
+    tracts of one base and errors."""
+    rng = np.random.default_rng(seed)
+    g = rng.choice(np.frombuffer(b"ACGT", np.uint8), genome_len, p=[(1 - gc) / 2, gc / 2, gc / 2, (1 - gc) / 2])
+    for a in rng.integers(0, genome_len - 40, genome_len // 400):
+        g[a:a + int(rng.integers(8, 30))] = ord("A")
+    out = []
+    for a in rng.integers(0, genome_len - 150, n):
+        r = g[a:a + 150].copy()
+        r[rng.random(150) < 0.004] = ord("C")
+        out.append(rc(r.tobytes()) if rng.random() < 0.5 else r.tobytes())
+    return out
+
+
+@pytest.mark.parametrize("k", [17, 21, 33, 77, 99])
+@pytest.mark.parametrize("keep,genome_len,n", [(False, 80_000, 16_000), (True, 80_000, 16_000), (False, 300_000, 70_000)])
+def test_frequent_minimizers(k, keep, genome_len, n):
+    """Bins of many keys, scattered again over sub-bins, with and without a sample of the bins."""
+    seqs = at_rich_reads(k, genome_len, n, 0.08) + [b"G" * 150] * 300 + [b"AC" * 75] * 300
+    c = api.Context(0)
+    try:
+        c.set_timing(True)
+        (compare_build if keep else compare_gate_only)(c, bank_of(seqs), k, api.key_bits_for_k(k), 16, None, 18)
+        assert c.timing("bins_heavy")[1] == 5 and c.timing("bins_aggregate")[1] >= 1 and c.timing("pass2")[1] == 0
+    finally:
+        c.close()

@@ -13,7 +13,7 @@ import pytest
 
 from fastbact_gb300 import api
 from oracle import orc
-from test_gpu_bins import uneven_reads
+from test_gpu_bins import at_rich_reads, uneven_reads
 from test_gpu_parity import sample_reads
 
 pytestmark = pytest.mark.gpu
@@ -104,3 +104,17 @@ def test_long_reads_in_one_round(ctx, genome, longest, rounds):
     assert same(ctx, sample, n, stats, 21, 14, 18) == (6000 if genome == 100_000 else n)
     ctx.set_timing(False)
     assert ctx.timing("est_firstpos")[1] == rounds
+
+
+@pytest.mark.parametrize("k", [21, 33])
+def test_frequent_minimizers(ctx, k):
+    """A sample of more than 8 M k-mers whose bins hold many keys each."""
+    seqs = at_rich_reads(k, 1_000_000, 80_000, 0.1)
+    sample = api.BitSeqArena.from_seqs(seqs)
+    lens = [len(s) for s in seqs]
+    stats = api.ExactCountStats(len(seqs) // 2, sum(lens[::2]), sum(lens[1::2]), sum(lens), min(lens), max(lens), 150.0, 150)
+    ctx.timing_reset()
+    ctx.set_timing(True)
+    same(ctx, sample, len(seqs) // 2, stats, k, 14, 20)
+    ctx.set_timing(False)
+    assert ctx.timing("est_heavy")[1] >= 5 and ctx.timing("est_first_regs")[1] >= 1
