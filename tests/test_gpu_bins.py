@@ -290,3 +290,53 @@ def test_frequent_minimizers(k, keep, genome_len, n):
         assert c.timing("bins_heavy")[1] == 5 and c.timing("bins_aggregate")[1] >= 1 and c.timing("pass2")[1] == 0
     finally:
         c.close()
+
+
+@pytest.mark.parametrize("k,keep,acc_filter", [(31, False, 0), (31, True, 1), (77, False, 1), (31, False, 2), (127, True, 2)])
+def test_short_of_memory(k, keep, acc_filter):
+    """Pools of every size between too small and ample: what the record buckets build is built,
+    whether the bins find their memory, in part of their steps or not at all."""
+    bank = bank_of(uneven_reads(k, 100_000, 32_000, 120 + k, (), 0.004))
+    got = {}
+    for mb in (16, 48, 64, 80, 96, 112, 128, 144, 160, 176, 192, 208, 224, 256, 320, 448, 1024):
+        for form in (0, 1):
+            c = api.Context(0, pool_bytes=mb << 20)
+            try:
+                c.set_tuning(build_form=form, acc_filter=acc_filter)
+                c.set_timing(True)
+                t, cms = api.build_cdbg_with_contigs_ext(bank, [], k, None, None, ctx=c, counter_bits=16, cms_log2_width=20, keep_cms=True) if keep \
+                    else (api.build_cdbg_ext(bank, k, None, 100_000, ctx=c, counter_bits=16, cms_log2_width=20), None)
+                got[mb, form] = (t.info()[1], t.digest(), t.pushes(), cms.export().tobytes() if keep else None)
+                got[mb, "route"] = (c.timing("bins_aggregate")[1] > 0, c.timing("pass2")[1] > 0)
+            except N.FbkError as e:
+                assert N.STATUS_NAMES[e.status] == "FBK_ERR_OOM", e
+                got[mb, form] = None
+            finally:
+                c.close()
+        if got[mb, 0] is not None or got[mb, 1] is not None:
+            assert got[mb, 1] == (got[mb, 0] or got[mb, 1])
+    done = {v for key, v in got.items() if key[1] in (0, 1)}
+    assert len(done - {None}) == 1 and None in done
+    routes = [v for key, v in got.items() if key[1] == "route"]
+    assert routes[0] == (False, True) and routes[-1] == (True, False)
+
+
+@pytest.mark.parametrize("k", [63, 77])
+@pytest.mark.parametrize("keep", [False, True])
+@pytest.mark.parametrize("acc_filter", [0, 2])
+def test_a_sample_that_tells_too_little(k, keep, acc_filter):
+    """Many distinct keys in one bin that is no part of the sample: the rows do not suffice, and
+    the keys are counted again with the counted sizes."""
+    x = low_minimizer()
+    flank = rand_seqs(4, 16_000, k - 17, k - 15)
+    seqs = uneven_reads(k, 20_000, 30_000, 230, (), 0.0) + [flank[i] + x + flank[i + 1] for i in range(0, 16_000, 2)] * 2
+    assert sum(max(0, len(s) - k + 1) for s in seqs) > 4 << 20
+    c = api.Context(0)
+    try:
+        c.set_tuning(acc_filter=acc_filter)
+        c.set_timing(True)
+        (compare_build if keep else compare_gate_only)(c, bank_of(seqs), k, api.key_bits_for_k(k), 16, None, 20)
+        # (filtered, the keys seen twice are only listed for the sketch, and not at all for one that is kept)
+        assert c.timing("bins_aggregate")[1] == (1 if keep and acc_filter else 2) and c.timing("pass2")[1] == 0
+    finally:
+        c.close()
