@@ -1490,7 +1490,10 @@ bool bins_applicable(const fbk_ctx* ctx, const fbk_bank* b, const fbk_build_para
 
 // Up to this many windows no sample is taken: rows are allocated for every window.
 constexpr uint64_t BINS_SAMPLE_FROM = 4u << 20;
-constexpr uint64_t BINS_SMALL_GROUP = 6000;  // windows of a group then
+// Windows of a group then: as many groups as blocks are resident, of 512 to 6000 windows.  (6000
+// for all: 100 reads of distinct k-mers, k = 55, 0.29 ms, 0.20 so, 0.35 over records; 3000 reads
+// of 3 Mbp, k = 77, 0.36, 0.21 and 0.32.)
+uint64_t small_group(uint64_t windows, int sms) { return std::max<uint64_t>(512, std::min<uint64_t>(6000, windows / (2 * (uint64_t)sms))); }
 
 namespace {
 
@@ -1666,8 +1669,9 @@ fbk_status bins_build(fbk_ctx* ctx, const fbk_bank* b, const fbk_build_params* p
     A.single = single;
     A.counters = counters;
     A.status = ctx->d_status;
-    A.later_cap = sampled ? AGG_LATER : 4096;
-    A.max_blocks = (uint32_t)(sampled ? 2 * sms : std::min<uint64_t>(2 * sms, windows / BINS_SMALL_GROUP + 1));
+    const uint64_t small = small_group(windows, sms);
+    A.later_cap = sampled ? AGG_LATER : (uint32_t)std::min<uint64_t>(4096, 2 * small);
+    A.max_blocks = (uint32_t)(sampled ? 2 * sms : std::min<uint64_t>(2 * sms, windows / small + 1));
     A.later = (uint64_t*)B.get(16ULL * A.later_cap * A.max_blocks);
     if (!A.later) return set_err(ctx, FBK_ERR_OOM, "minimizer bins");
     unsigned long long* h = (unsigned long long*)ctx->h_pinned;
@@ -1690,7 +1694,7 @@ fbk_status bins_build(fbk_ctx* ctx, const fbk_bank* b, const fbk_build_params* p
     }
     // groups that about fill 0.7 of the entries, with few enough windows for 16-bit counts
     const uint64_t target =
-        sampled ? group_windows(cms ? count_entries(nk, false) : agg_entries(nk, false), n_windows, distinct) : BINS_SMALL_GROUP;
+        sampled ? group_windows(cms ? count_entries(nk, false) : agg_entries(nk, false), n_windows, distinct) : small;
     const uint32_t n_groups = (uint32_t)(n_windows / target + 1);
     unsigned long long* start = (unsigned long long*)B.get(8ULL * (n_groups + 1));
     if (!start) return set_err(ctx, FBK_ERR_OOM, "minimizer bins: groups");
