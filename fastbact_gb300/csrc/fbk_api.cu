@@ -1220,17 +1220,23 @@ FBK_API fbk_status fbk_hll_release(fbk_hll* h) {
 // ===========================================================================
 static void table_free_storage(fbk_table* t) {
     fbk_ctx* ctx = t->ctx;
-    if (t->tags != t->keys) dev_free(ctx, t->tags);
+    if (!t->one_block) {
+        if (t->tags != t->keys) dev_free(ctx, t->tags);
+        dev_free(ctx, t->cnt);
+    }
     dev_free(ctx, t->keys);
-    dev_free(ctx, t->cnt);
     dev_free(ctx, t->cov);
     t->keys = t->tags = nullptr;
     t->cnt = t->cov = nullptr;
+    t->one_block = false;
 }
 static void table_free_out(fbk_table* t) {
+    if (!t->out_one_block) {
+        dev_free(t->ctx, t->out_cov);
+        dev_free(t->ctx, t->out_mask);
+    }
     dev_free(t->ctx, t->out_keys);
-    dev_free(t->ctx, t->out_cov);
-    dev_free(t->ctx, t->out_mask);
+    t->out_one_block = false;
     t->out_keys = nullptr;
     t->out_cov = nullptr;
     t->out_mask = nullptr;

@@ -1458,14 +1458,30 @@ cudaError_t by_width(int nw, uint32_t k, Fn&& f) {
 struct Scratch {  // device buffers of one build, freed when it ends
     fbk_ctx* c;
     std::vector<void*> p;
+    char *at = nullptr, *end = nullptr;  // what is left of a block that buffers share
+    // A block for buffers of `bytes` in all, rounded: a context without a pool pays for every
+    // allocation (0.02 ms and more with its release).
+    static uint64_t rounded(uint64_t bytes) { return (bytes + 255) & ~255ULL; }
+    void share(uint64_t bytes) {
+        at = (char*)dev_alloc(c, 256 + bytes);
+        if (!at) return;
+        p.push_back(at);
+        end = at + 256 + bytes;
+        at += 256;  // none of them begins where the block does
+    }
     void* get(uint64_t bytes) {
+        if (bytes && rounded(bytes) <= (uint64_t)(end - at)) {
+            at += rounded(bytes);
+            return at - rounded(bytes);
+        }
         void* q = dev_alloc(c, bytes);
         if (q) p.push_back(q);
         return q;
     }
     void drop(void* q) {
-        for (auto& x : p)
-            if (x == q) x = nullptr;
+        const auto it = std::find(p.begin(), p.end(), q);
+        if (it == p.end()) return;  // the block's: it goes with the block
+        p.erase(it);
         cudaStreamSynchronize(c->stream);
         dev_free(c, q);
     }
@@ -1506,30 +1522,39 @@ struct BinRuns {
     uint64_t* runs = nullptr;
     uint64_t n_windows = 0;
     bool est = false;  // of an estimate: timed under its names
-    BinRuns(const MinPlan& m, uint64_t windows) : mp(m) {
+    // The warps of k_bin_runs and the runs a warp's log holds.
+    uint64_t n_blocks = 0, cap_w = 0;
+    BinRuns(uint32_t k, uint64_t windows, uint64_t n_reads, uint32_t max_len, int sms) : mp(min_plan(k)) {
         while (F < RUN_MAX_BINS && (uint64_t)F * 1500 < windows) F <<= 1;
+        const uint64_t max_warps = (uint64_t)resident_grid(k_bin_runs, 256, 0, sms) * 8;
+        n_blocks = std::max<uint64_t>(1, std::min<uint64_t>(max_warps, n_reads) / 8);
+        // a run holds about (w + 1) / 2 windows, and one more ends with every read
+        cap_w = (uint64_t)(1.3 * ((2.0 * windows) / (mp.w + 1) + n_reads) / (8 * n_blocks)) + 128 + std::min<uint64_t>(max_len / 4, 2048);
+        // and at most one with every window of the longest reads
+        cap_w = std::min<uint64_t>(cap_w, (n_reads / (8 * n_blocks) + 1) * (max_len >= k ? max_len - k + 1 : 1));
+    }
+    // What bin_runs needs, but for the two logs and with them.
+    uint64_t bytes(bool logs) const {
+        return Scratch::rounded(8ULL * (F + 1 + (F + SCAN_TILE - 1) / SCAN_TILE)) + Scratch::rounded(4ULL * F) + Scratch::rounded(32 * n_blocks) +
+               (logs ? 2 * Scratch::rounded(64 * n_blocks * cap_w) : 0);
     }
 };
 
 // Cuts the reads of bv into runs (windows: no fewer than they hold) and scatters them by bin;
 // with a sample, counts the keys of some bins.  The counters and n_windows are on the host
 // then, in ctx->h_pinned.  Clears the caller's block and the context's status first.
-fbk_status bin_runs(fbk_ctx* ctx, Scratch& B, BinRuns& R, const BankDev& bv, uint32_t max_len, uint32_t k, uint64_t windows, char* cleared,
-                    uint64_t clear_bytes, AggArgs* sample, bool* declined) {
+fbk_status bin_runs(fbk_ctx* ctx, Scratch& B, BinRuns& R, const BankDev& bv, uint32_t k, uint64_t windows, char* cleared, uint64_t clear_bytes,
+                    AggArgs* sample, bool* declined) {
     const MinPlan mp = R.mp;
     const uint32_t F = R.F;
     const int sms = ctx->num_sms;
     const cudaStream_t stream = ctx->stream;
-    const uint64_t n_reads = bv.r_end - bv.r_begin;
     R.pre = (unsigned long long*)B.get(8ULL * (F + 1 + (F + SCAN_TILE - 1) / SCAN_TILE));
     uint32_t* cursor = (uint32_t*)B.get(4ULL * F);
     if (!R.pre || !cursor) return set_err(ctx, FBK_ERR_OOM, "minimizer bins");
     unsigned long long* part = R.pre + F + 1;
-    const uint64_t max_warps = (uint64_t)resident_grid(k_bin_runs, 256, 0, sms) * 8;
-    const uint64_t n_blocks = std::max<uint64_t>(1, std::min<uint64_t>(max_warps, n_reads) / 8);
-    const uint64_t n_warps = n_blocks * 8;
-    // a run holds about (w + 1) / 2 windows, and one more ends with every read
-    uint64_t cap_w = (uint64_t)(1.3 * ((2.0 * windows) / (mp.w + 1) + n_reads) / n_warps) + 128 + std::min<uint64_t>(max_len / 4, 2048);
+    const uint64_t n_blocks = R.n_blocks, n_warps = 8 * n_blocks;
+    uint64_t cap_w = R.cap_w;
     uint32_t* log_n = (uint32_t*)B.get(4 * n_warps);
     if (!log_n) return set_err(ctx, FBK_ERR_OOM, "minimizer bins");
     unsigned long long* h = (unsigned long long*)ctx->h_pinned;
@@ -1643,17 +1668,24 @@ fbk_status bins_build(fbk_ctx* ctx, const fbk_bank* b, const fbk_build_params* p
     const int nk = nw - (int)((64u * (uint32_t)nw - 2u * k) >> 6);
     const uint64_t windows = b->windows(k, k);  // upper bound (subsampling keeps fewer)
     const bool sampled = windows > BINS_SAMPLE_FROM;
-    const MinPlan mp = min_plan(k);
     const int sms = ctx->num_sms;
     const cudaStream_t stream = ctx->stream;
     Scratch B{ctx, {}};
-    BinRuns R(mp, windows);
+    BinRuns R(k, windows, b->n_reads, b->max_len, sms);
     const uint32_t F = R.F;
     // one cleared block: the ladder, the bin and build counters, the windows' bitmaps
     const uint64_t bm_words = (b->n_words + 63) & ~63ULL;
     const uint64_t lad_bytes = cms ? 0 : (2 * (4ULL << log2w) / 8 + 255) & ~255ULL;
     const uint64_t clear_bytes = lad_bytes + 8ULL * F + 8 * 16 + 2 * 4 * bm_words;
     static_assert(BC_N <= 16, "build counters");
+    const uint64_t small = small_group(windows, sms);
+    AggArgs A{};
+    A.later_cap = sampled ? AGG_LATER : (uint32_t)std::min<uint64_t>(4096, 2 * small);
+    A.max_blocks = (uint32_t)(sampled ? 2 * sms : std::min<uint64_t>(2 * sms, windows / small + 1));
+    const uint64_t later_bytes = 16ULL * A.later_cap * A.max_blocks;
+    // (a sampled build's logs go before its rows come)
+    B.share(Scratch::rounded(clear_bytes) + Scratch::rounded(4 * bm_words) + Scratch::rounded(later_bytes) + R.bytes(!sampled) +
+            (sampled ? 0 : Scratch::rounded(8 * (windows / small + 2))));
     char* cleared = (char*)B.get(clear_bytes);
     uint32_t* pass = (uint32_t*)B.get(4 * bm_words);
     if (!cleared || !pass) return set_err(ctx, FBK_ERR_OOM, "minimizer bins");
@@ -1663,21 +1695,17 @@ fbk_status bins_build(fbk_ctx* ctx, const fbk_bank* b, const fbk_build_params* p
     uint32_t* single = (uint32_t*)(counters + 16);
     uint32_t* valid = single + bm_words;
     const BankDev bv = bank_view(b, 0, b->n_reads, keep_bits);
-    AggArgs A{};
     A.data = b->data;
     A.k = k;
     A.single = single;
     A.counters = counters;
     A.status = ctx->d_status;
-    const uint64_t small = small_group(windows, sms);
-    A.later_cap = sampled ? AGG_LATER : (uint32_t)std::min<uint64_t>(4096, 2 * small);
-    A.max_blocks = (uint32_t)(sampled ? 2 * sms : std::min<uint64_t>(2 * sms, windows / small + 1));
-    A.later = (uint64_t*)B.get(16ULL * A.later_cap * A.max_blocks);
+    A.later = (uint64_t*)B.get(later_bytes);
     if (!A.later) return set_err(ctx, FBK_ERR_OOM, "minimizer bins");
     unsigned long long* h = (unsigned long long*)ctx->h_pinned;
     const bool may_filter = p->min_trans_cov >= 2 && ctx->acc_filter != 0;
     A.mtc = may_filter ? p->min_trans_cov : 0;
-    fbk_status rs = bin_runs(ctx, B, R, bv, b->max_len, k, windows, cleared, clear_bytes, sampled ? &A : nullptr, declined);
+    fbk_status rs = bin_runs(ctx, B, R, bv, k, windows, cleared, clear_bytes, sampled ? &A : nullptr, declined);
     if (rs || *declined) return rs;
     const uint64_t n_windows = R.n_windows;
     uint64_t* runs = R.runs;
@@ -1728,11 +1756,15 @@ fbk_status bins_build(fbk_ctx* ctx, const fbk_bank* b, const fbk_build_params* p
     for (int attempt = 0;; ++attempt) {
         // a table of the rows alone: every slot that is read is one, no probing
         tb->cap = rows;
-        tb->keys = (uint64_t*)dev_alloc(ctx, rows * 8 * nw);
-        if (nw > 2) tb->tags = tag_in_key((uint32_t)nw, k) ? tb->keys : (uint64_t*)dev_alloc(ctx, rows * 8);
-        tb->cnt = (uint32_t*)dev_alloc(ctx, rows * 32);
+        const uint64_t key_bytes = Scratch::rounded(rows * 8 * nw), tag_bytes = nw > 2 && !tag_in_key((uint32_t)nw, k) ? Scratch::rounded(rows * 8) : 0;
+        tb->keys = (uint64_t*)dev_alloc(ctx, key_bytes + tag_bytes + rows * 32);
+        tb->one_block = true;
+        if (tb->keys) {
+            if (nw > 2) tb->tags = tb->keys + (tag_bytes ? key_bytes / 8 : 0);
+            tb->cnt = (uint32_t*)((char*)tb->keys + key_bytes + tag_bytes);
+        }
         if (lows) low = (uint64_t*)B.get(lows * 8 * nk);
-        if (!tb->keys || (nw > 2 && !tb->tags) || !tb->cnt || (lows && !low)) return set_err(ctx, FBK_ERR_OOM, "solid table rows");
+        if (!tb->keys || (lows && !low)) return set_err(ctx, FBK_ERR_OOM, "solid table rows");
         const TableDev td = tbl_dev(tb);
         A.start = start;
         A.stride = 1;
@@ -1814,10 +1846,11 @@ fbk_status bins_build(fbk_ctx* ctx, const fbk_bank* b, const fbk_build_params* p
     tb->cap = h[BC_ROWS];
     // rows of the conversion: a subset of those with an edge count of min_trans_cov
     const uint64_t oc = std::min<uint64_t>(tb->cap, kept) + 16;
-    tb->out_keys = (uint64_t*)dev_alloc(ctx, oc * 8 * nw);
-    tb->out_cov = (uint16_t*)dev_alloc(ctx, oc * 2);
-    tb->out_mask = (uint8_t*)dev_alloc(ctx, oc);
-    if (!tb->out_keys || !tb->out_cov || !tb->out_mask) return set_err(ctx, FBK_ERR_OOM, "solid table output");
+    tb->out_keys = (uint64_t*)dev_alloc(ctx, oc * (8 * nw + 2 + 1));
+    tb->out_one_block = true;
+    if (!tb->out_keys) return set_err(ctx, FBK_ERR_OOM, "solid table output");
+    tb->out_cov = (uint16_t*)(tb->out_keys + oc * nw);
+    tb->out_mask = (uint8_t*)(tb->out_cov + oc);
     tb->out_cap = oc;
     if (cms) TIMED(ctx, "cms_clamp", launch_clamp_counters(launch_cfg(ctx, 256, 0), cms->cnt, cms->n));
     fbk_status st = tbl_convert(tb);
@@ -1850,7 +1883,7 @@ fbk_status bins_first(fbk_ctx* ctx, const fbk_bank* b, uint64_t n_reads, uint64_
     const int nk = (int)((k + 31) / 32), sms = ctx->num_sms;
     const cudaStream_t stream = ctx->stream;
     Scratch B{ctx, {}};
-    BinRuns R(min_plan(k), windows);
+    BinRuns R(k, windows, n_reads, b->max_len, sms);
     R.est = true;
     const uint64_t clear_bytes = 8ULL * R.F + 8 * 16;
     char* cleared = (char*)B.get(clear_bytes);
@@ -1866,7 +1899,7 @@ fbk_status bins_first(fbk_ctx* ctx, const fbk_bank* b, uint64_t n_reads, uint64_
     A.counters = R.counters = R.hist + R.F;
     unsigned long long* h = (unsigned long long*)ctx->h_pinned;
     bool no = false;
-    fbk_status st = bin_runs(ctx, B, R, bank_view(b, 0, n_reads, nullptr), b->max_len, k, windows, cleared, clear_bytes, &A, &no);
+    fbk_status st = bin_runs(ctx, B, R, bank_view(b, 0, n_reads, nullptr), k, windows, cleared, clear_bytes, &A, &no);
     if (st == FBK_ERR_OOM || no) return FBK_OK;
     if (st) return st;
     const uint64_t n_windows = R.n_windows;

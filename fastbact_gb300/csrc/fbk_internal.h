@@ -171,6 +171,7 @@ struct fbk_table {
     uint16_t* out_cov = nullptr;
     uint8_t* out_mask = nullptr;
     uint64_t out_cap = 0;
+    bool one_block = false, out_one_block = false;  // tags and cnt (out_cov and out_mask) lie in the allocation of the keys
     uint64_t n_keys = 0, n_solid = 0, digest = 0, pushes = 0;
     uint64_t skipped_pushes = 0;  // pushes of records the record filter kept out of the table
     bool filtered = false;        // the accumulator holds only keys that may become solid
