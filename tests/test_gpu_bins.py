@@ -340,3 +340,23 @@ def test_a_sample_that_tells_too_little(k, keep, acc_filter):
         assert c.timing("bins_aggregate")[1] == (1 if keep and acc_filter else 2) and c.timing("pass2")[1] == 0
     finally:
         c.close()
+
+
+@pytest.mark.parametrize("k,kb,filtered", [(21, 64, True), (55, 128, True), (21, 64, False)])
+def test_small_builds_filter_as_larger_ones(k, kb, filtered):
+    """Below the sample's size too, a build whose distinct keys exceed a fifth of its windows keeps
+    out of the accumulator what cannot become solid."""
+    seqs = uneven_reads(k, 400_000 if filtered else 8_000, 3_000, 200, (), 0.002)
+    c = api.Context(0)
+    try:
+        compare_gate_only(c, bank_of(seqs), k, kb, 16, None, 16)
+        compare_build(c, bank_of(seqs), k, kb, 16, None, 16)
+        info = []
+        for acc_filter in (1, 0):
+            c.set_tuning(acc_filter=acc_filter)
+            t = api.build_cdbg_ext(bank_of(seqs), k, None, 100_000, ctx=c, counter_bits=16, cms_log2_width=16)
+            info.append((t.filtered(), *t.info()[:2], t.pushes()))
+        assert info[0][0] == filtered and not info[1][0] and info[0][2:] == info[1][2:]
+        assert (info[0][1] < info[1][1]) == filtered
+    finally:
+        c.close()
