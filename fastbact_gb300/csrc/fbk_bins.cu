@@ -268,7 +268,7 @@ __global__ void __launch_bounds__(256) k_bin_scan(const unsigned long long* __re
         p += x[j];
         if (i0 + j == n - 1) pre[n] = p;
         const uint32_t windows = (uint32_t)x[j];
-        if (big && windows > 1u << 13) {  // rare
+        if (big && windows > 1u << 13) {  // rare (HEAVY_FROM)
             for (int c = 0; c < 3; ++c)
                 if (windows > 1u << (13 + 2 * c)) atomicAdd(&big[c], (unsigned long long)windows);
         }
@@ -405,6 +405,7 @@ struct HeavyPiece {
     uint32_t sub, parts;  // sub-bins [sub, sub + parts)
 };
 constexpr uint32_t HEAVY_PIECE = 1024;  // runs
+constexpr uint32_t HEAVY_FROM = 1u << 13;  // not less: k_bin_scan counts the windows of bins above it
 // counts: pieces, sub-bins.
 __global__ void k_heavy_pieces(const unsigned long long* __restrict__ pre, uint32_t n, uint32_t target, uint32_t from,
                                HeavyPiece* __restrict__ pieces, uint32_t cap, uint32_t* __restrict__ counts) {
@@ -534,6 +535,7 @@ constexpr uint32_t AGG_SMEM = 113000;  // two blocks an SM (228 KB, 1 KB reserve
 constexpr uint32_t AGG_NARROW_MAX = 65535;  // windows of a group whose u16 counts cannot overflow
 constexpr uint32_t AGG_QUEUE = 64 * 8;      // bytes of a warp's queue
 constexpr uint32_t AGG_LATER = 16384;       // windows a block can put off, at most
+constexpr uint32_t SAMPLE_WINDOWS = 4096;   // windows of a sampled bin whose keys are all counted
 constexpr uint32_t AGG_TURNS = 1u << 16;    // a turn is repeated only when another lane has entered a key
 constexpr uint32_t NO_PLACE = 0xFFFFFFFFu;  // AGG_FIRST; the bank holds fewer than 2^32 - 1 bases
 constexpr uint32_t POS_TWICE = 0xFFFFFFFFu; // place + 1 of the key's first window otherwise, 0: no key
@@ -723,6 +725,8 @@ __global__ void __launch_bounds__(AGG_THREADS, 2) k_bin_agg(AggArgs A) {
             if constexpr (COUNT) sh_add_if(on && !(w.rc ? has_l : has_r), elack + 4 * entry, 1);
         };
         uint64_t lo = 0, width = 1ULL << 32;  // the part of the hash range being counted
+        // of a sampled bin a part of the keys that fits, each for as many as there are parts
+        if (SAMPLE && windows > SAMPLE_WINDOWS) width >>= 32 - __clz((windows - 1) / SAMPLE_WINDOWS);
         const uint64_t* src = runs;           // the group's runs, or the windows put off
         uint32_t n_src = n_runs;
         uint64_t* later = A.later + (uint64_t)blockIdx.x * 2 * A.later_cap;
@@ -942,6 +946,7 @@ __global__ void __launch_bounds__(AGG_THREADS, 2) k_bin_agg(AggArgs A) {
                 goto again;
             }
             const uint32_t n_entries = min(s_entries, cap), n_later = s_later;
+            const unsigned long long weight = SAMPLE ? (1ULL << 32) / width : 1;
             // What becomes of entry i: 1 seen once, 2 low row, 3 row; its counts in e.
             auto counts = [&](uint32_t i, uint32_t (&e)[8]) {
                 const uint4 a = sh_ld128(ecnt + ((4 * i) << cl));
@@ -981,7 +986,7 @@ __global__ void __launch_bounds__(AGG_THREADS, 2) k_bin_agg(AggArgs A) {
                 counts(i, e);
                 const uint32_t a = e[0] + e[1] + e[2] + e[3], b = e[4] + e[5] + e[6] + e[7];
                 if (a < 2 && b < 2 && pos != POS_TWICE && !((a | b) && (s_alone[i >> 5] >> (i & 31) & 1u))) {
-                    ++tot_single;
+                    tot_single += weight;
                     if (!SAMPLE) atomicOr(&A.single[(pos - 1) >> 5], 1u << ((pos - 1) & 31));
                     continue;
                 }
@@ -1001,8 +1006,8 @@ __global__ void __launch_bounds__(AGG_THREADS, 2) k_bin_agg(AggArgs A) {
                 codes |= (low ? 2u : 3u) << turn;
             }
             if constexpr (SAMPLE) {
-                tot_multi += n_row + n_low;
-                tot_kept += n_row;
+                tot_multi += (n_row + n_low) * weight;
+                tot_kept += n_row * weight;
                 block_sync();
             } else if constexpr (!FIRST) {
                 // rows and low rows are counted, reserved once, then written
@@ -1058,7 +1063,7 @@ __global__ void __launch_bounds__(AGG_THREADS, 2) k_bin_agg(AggArgs A) {
             } else {
                 src = runs;
                 n_src = n_runs;
-                lo += width;
+                lo = SAMPLE ? 1ULL << 32 : lo + width;
             }
         }
     }
@@ -1579,8 +1584,7 @@ fbk_status bin_runs(fbk_ctx* ctx, Scratch& B, BinRuns& R, const BankDev& bv, uin
             sample->n_groups = std::min<uint32_t>(F, 1024);
             sample->stride = F / sample->n_groups;
             sample->start = R.pre;
-            // (a heavy bin is no sample of the others, and its keys would be taken in parts)
-            sample->heavy_from = (uint32_t)std::min<uint64_t>(AGG_NARROW_MAX, std::max<uint64_t>(8192, 8 * windows / F));
+            sample->heavy_from = 1u << 18;  // (1 ms of a block's time)
             TIMED(ctx, R.est ? "est_sample" : "bins_sample", agg_launch_nk<AGG_SAMPLE>((int)((k + 31) / 32), stream, *sample));
         }
         CK(ctx, cudaMemcpyAsync(h, R.counters, 8 * BC_N, cudaMemcpyDeviceToHost, stream));
@@ -1602,21 +1606,26 @@ fbk_status bin_runs(fbk_ctx* ctx, Scratch& B, BinRuns& R, const BankDev& bv, uin
     return FBK_OK;
 }
 
-// Windows of a group of bins whose keys about fill 0.7 of the entries.
+// Windows of a group of bins whose keys about fill 0.7 of the entries; no more than 20,000, as
+// very deep banks (a key in many of the windows that are in flight is entered many times) need
+// more room than that: 30 kb at 2000x, k = 21, with up to 60,000 2.3 ms, so 1.5 (12,000 1.5, 8000
+// 1.5; 5 Mbp at 100x 10.8, 10.8, 11.1, 11.5).
 uint64_t group_windows(uint32_t entries, uint64_t n_windows, uint64_t distinct) {
     const uint64_t t = (uint64_t)(0.7 * (double)entries * (double)std::max<uint64_t>(n_windows, 1) / (double)std::max<uint64_t>(distinct, 1));
-    return std::max<uint64_t>(512, std::min<uint64_t>(t, 60000));
+    return std::max<uint64_t>(512, std::min<uint64_t>(t, 20000));
 }
 
 // The heavy bins' windows by sub-bin, for groups of `target` windows; A then takes them first and
 // passes their bins over.  h: the counters on the host.  Where there is no memory for it, A
 // keeps the bins as they are.
-fbk_status split_heavy(fbk_ctx* ctx, Scratch& B, const BinRuns& R, const unsigned long long* h, uint64_t target, AggArgs& A) {
+fbk_status split_heavy(fbk_ctx* ctx, Scratch& B, const BinRuns& R, const unsigned long long* h, uint64_t target, uint64_t at_least,
+                       AggArgs& A) {
     A.n_heavy = 0;
     A.heavy_from = 0xFFFFFFFFu;
     // a group of ordinary bins stays below three targets (k_bin_groups)
-    const uint32_t from = (uint32_t)std::max<uint64_t>(3 * target, 1u << 13);
-    const uint64_t windows = h[BC_BIG + (from >= 1u << 17 ? 2 : from >= 1u << 15 ? 1 : 0)];  // no fewer than they have
+    const uint32_t from = (uint32_t)std::max<uint64_t>(3 * target, at_least);
+    // the windows in bins above 2^13, 2^15 or 2^17: no fewer than the heavy bins', as `from` is no less
+    const uint64_t windows = h[BC_BIG + (from >= 1u << 17 ? 2 : from >= 1u << 15 ? 1 : 0)];
     if (!windows) return FBK_OK;
     const cudaStream_t stream = ctx->stream;
     const uint32_t cap = (uint32_t)(windows / HEAVY_PIECE + windows / from + 1), n_sub = (uint32_t)(windows / target + windows / from + 1);
@@ -1720,14 +1729,13 @@ fbk_status bins_build(fbk_ctx* ctx, const fbk_bank* b, const fbk_build_params* p
         kept = est(BC_KEPT);
         filter = may_filter && acc_filter_on(ctx->acc_filter, nw, distinct, n_windows);
     }
-    // groups that about fill 0.7 of the entries, with few enough windows for 16-bit counts
     const uint64_t target =
         sampled ? group_windows(cms ? count_entries(nk, false) : agg_entries(nk, false), n_windows, distinct) : small;
     const uint32_t n_groups = (uint32_t)(n_windows / target + 1);
     unsigned long long* start = (unsigned long long*)B.get(8ULL * (n_groups + 1));
     if (!start) return set_err(ctx, FBK_ERR_OOM, "minimizer bins: groups");
     A.runs = runs;
-    rs = split_heavy(ctx, B, R, h, target, A);
+    rs = split_heavy(ctx, B, R, h, target, HEAVY_FROM, A);
     if (rs) return rs;
     fbk_table* tb = new fbk_table();
     tb->ctx = ctx;
@@ -1924,7 +1932,7 @@ fbk_status bins_first(fbk_ctx* ctx, const fbk_bank* b, uint64_t n_reads, uint64_
     A.firsts = (FirstKey*)B.get(A.cap_rows * sizeof(FirstKey));
     if (!start || !A.firsts) return FBK_OK;
     A.start = start;
-    st = split_heavy(ctx, B, R, h, target, A);
+    st = split_heavy(ctx, B, R, h, target, HEAVY_FROM, A);
     if (st) return st;
     TIMED(ctx, "est_groups", (k_bin_groups<<<std::min<unsigned>(1024, (R.F + 256) / 256), 256, 0, stream>>>(R.pre, R.F, (uint32_t)target,
                                                                                                           A.n_groups, start),

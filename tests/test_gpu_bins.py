@@ -360,3 +360,19 @@ def test_small_builds_filter_as_larger_ones(k, kb, filtered):
         assert (info[0][1] < info[1][1]) == filtered
     finally:
         c.close()
+
+
+@pytest.mark.parametrize("k", [21, 77])
+@pytest.mark.parametrize("genome_len,acc_filter", [(3_000, 0), (20_000, 1), (700, 2)])
+def test_deep_banks(k, genome_len, acc_filter):
+    """Depths of hundreds to ten thousand: every bin that holds anything holds many windows, few of
+    them distinct, and is sampled by a part of its keys."""
+    seqs = uneven_reads(k, genome_len, 60_000, 130 + k // 2, (), 0.004)
+    c = api.Context(0)
+    try:
+        c.set_tuning(acc_filter=acc_filter)
+        c.set_timing(True)
+        compare_gate_only(c, bank_of(seqs), k, api.key_bits_for_k(k), 16, None, 18)
+        assert c.timing("bins_sample")[1] == 1 and c.timing("bins_aggregate")[1] == 1 and c.timing("pass2")[1] == 0
+    finally:
+        c.close()
