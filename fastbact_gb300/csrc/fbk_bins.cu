@@ -1511,10 +1511,10 @@ bool bins_applicable(const fbk_ctx* ctx, const fbk_bank* b, const fbk_build_para
 
 // Up to this many windows no sample is taken: rows are allocated for every window.
 constexpr uint64_t BINS_SAMPLE_FROM = 4u << 20;
-// Windows of a group then: as many groups as blocks are resident, of 512 to 6000 windows.  (6000
+// Windows of a group then: as many groups as blocks are resident, of 512 to 3000 windows.  (6000
 // for all: 100 reads of distinct k-mers, k = 55, 0.29 ms, 0.20 so, 0.35 over records; 3000 reads
-// of 3 Mbp, k = 77, 0.36, 0.21 and 0.32.)
-uint64_t small_group(uint64_t windows, int sms) { return std::max<uint64_t>(512, std::min<uint64_t>(6000, windows / (2 * (uint64_t)sms))); }
+// of 3 Mbp, k = 77, 0.36, 0.21 and 0.32; 35,000 of them 0.70, 0.51 and 0.58.)
+uint64_t small_group(uint64_t windows, int sms) { return std::max<uint64_t>(512, std::min<uint64_t>(3000, windows / (2 * (uint64_t)sms))); }
 
 namespace {
 
@@ -1735,7 +1735,7 @@ fbk_status bins_build(fbk_ctx* ctx, const fbk_bank* b, const fbk_build_params* p
     unsigned long long* start = (unsigned long long*)B.get(8ULL * (n_groups + 1));
     if (!start) return set_err(ctx, FBK_ERR_OOM, "minimizer bins: groups");
     A.runs = runs;
-    rs = split_heavy(ctx, B, R, h, target, HEAVY_FROM, A);
+    rs = split_heavy(ctx, B, R, h, target, sampled ? HEAVY_FROM : 2 * HEAVY_FROM, A);
     if (rs) return rs;
     fbk_table* tb = new fbk_table();
     tb->ctx = ctx;
