@@ -1722,6 +1722,15 @@ fbk_status bins_build(fbk_ctx* ctx, const fbk_bank* b, const fbk_build_params* p
     uint64_t distinct = n_windows, multi = n_windows, kept = n_windows;  // upper bounds without a sample
     bool filter = may_filter && (ctx->acc_filter == 2 || nw == 4);
     if (sampled && h[BC_WINDOWS]) {
+        // Where most k-mers are new a key of three words and more costs here, entered, sketched
+        // and asked for once, what it costs over records or more.  Records / here by the share of
+        // distinct windows, 2 and 20 Mbp, 0.1-5% errors: k = 127 0.50 1.25, 0.61 1.10, 0.73 0.95,
+        // 0.83 0.87, 0.92 0.74, 1.0 0.61-0.69; k = 101 0.64 1.07, 0.74 1.02, 0.83 0.94-1.01, 0.93
+        // 0.76-0.82; k = 91 0.69 1.14, 0.79 1.01-1.14, 0.87 0.96, 0.91 0.81, 1.0 0.67-1.09.  (What is
+        // done by here is a tenth to a quarter of the build over records.)
+        const double share = (double)h[BC_DISTINCT] / (double)h[BC_WINDOWS];
+        *declined = nk >= 3 && share > (k > 96 ? 0.75 : 0.85);
+        if (*declined) return FBK_OK;
         const double scale = (double)n_windows / (double)h[BC_WINDOWS];
         auto est = [&](int c) { return std::min<uint64_t>(n_windows, (uint64_t)(1.1 * scale * (double)h[c]) + 65536); };
         distinct = est(BC_DISTINCT);

@@ -376,3 +376,16 @@ def test_deep_banks(k, genome_len, acc_filter):
         assert c.timing("bins_sample")[1] == 1 and c.timing("bins_aggregate")[1] == 1 and c.timing("pass2")[1] == 0
     finally:
         c.close()
+
+
+@pytest.mark.parametrize("k,rate,keep,binned", [(77, 0.06, False, False), (127, 0.04, True, False), (77, 0.002, False, True), (33, 0.15, False, True)])
+def test_banks_of_mostly_new_keys(k, rate, keep, binned):
+    """Wide keys of which most occur once go over the record buckets once a sample says so."""
+    seqs = uneven_reads(k, 600_000, 34_000, 130 + k, (), rate)
+    c = api.Context(0)
+    try:
+        c.set_timing(True)
+        (compare_build if keep else compare_gate_only)(c, bank_of(seqs), k, api.key_bits_for_k(k), 16, None, 20)
+        assert c.timing("bins_sample")[1] == 1 and (c.timing("bins_aggregate")[1] > 0) == binned and (c.timing("pass2")[1] > 0) != binned
+    finally:
+        c.close()
