@@ -339,7 +339,7 @@ def run_ours(args, rank, world, local):
         t = api.build_cdbg_ext(dbank, k, None, ge.genome_size, ctx=ctx, counter_bits=cb, cms_log2_width=LOG2W)
         t.release()
         ctx.sync()
-        per_k[str(k)] = {f: round(ctx.timing(f)[0], 3) for f in ("bins_runs", "bins_scatter", "bins_sample", "bins_aggregate",
+        per_k[str(k)] = {f: round(ctx.timing(f)[0], 3) for f in ("bins_runs", "bins_scatter", "bins_sample", "bins_heavy", "bins_aggregate",
                                                                   "bins_sketch", "bins_singles", "bins_gate", "pass1", "pass2_emit",
                                                                   "pass2_count", "pass2_upsert", "convert", "table_init")
                          if ctx.timing(f)[0] > 0}
@@ -363,7 +363,7 @@ def run_ours(args, rank, world, local):
                            "bitmap from the counts; same tables as the ladder gate"}
 
     # ---- roofline of the dominant pass --------------------------------------------
-    # Algorithmic bytes per pass (per k-mer occurrence): pass 1 = packed input +
+    # Algorithmic bytes per pass over occurrences (per k-mer occurrence): pass 1 = packed input +
     # 4 counters read and written (8 c_b); pass 2 = packed input + 4 counters read
     # (4 c_b) + 2 x (entry read + written) per transition push, entry = key + cov (2)
     # + 8 edge counters (16); c_b = 2 bytes (u16 sketch).
@@ -381,7 +381,9 @@ def run_ours(args, rank, world, local):
         "pass1": sum(bank_bytes + kmers_pass[k][0] * 8 * c_b for k in KS),
         "pass2": sum(bank_bytes + kmers_pass[k][1] * 4 * c_b + pushes[k] * 2 * (key_bytes[k] + 2 + 16) for k in KS),
     }
-    alg["bins"] = alg["pass1"] + alg["pass2"]
+    # Over minimizer bins the counters and entries stay in shared memory: what is left is the packed
+    # input once and the converted rows (key, cov, mask); instruction issue bounds that form.
+    alg["bins"] = sum(bank_bytes + r[2] * (key_bytes[r[0]] + 3) for r in res)
     dom = max(fam_ms, key=fam_ms.get)
     per_pass_ms = fam_ms[dom] / (args.steps * len(KS))
     per_pass_bytes = alg[dom] / len(KS)
@@ -501,17 +503,19 @@ def run_ours(args, rank, world, local):
                                              "k_singles, k_bin_gate)",
                                      "pass2": "pass 2 (record emit k_emit_roll / k_emit_flat + k_count_records + "
                                               "k_upsert / k_upsert_all)"})[dom],
-                         "bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
+                         "bound": "instruction issue" if dom == "bins" else "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                          "frac": achieved / peak, "peak_source": peak_src, "traffic": traffic,
                          "traffic_source": traffic_src,
                          "alg_bytes_per_pass": per_pass_bytes, "ms_per_pass": per_pass_ms,
-                         "note": "per pass = one k of one step; achieved = algorithmic bytes / event-timed kernel time"},
+                         "note": "per pass = one k of one step; achieved = algorithmic bytes / event-timed kernel time"
+                                 + ("; the bytes are the packed input and the converted rows, and the kernels' issue slots, not "
+                                    "the memory, bound them (profiles/k_bin_isolate5M_25x.md)" if dom == "bins" else "")},
             # the edge-counter atomics of the record buckets' upserts (one per transition push)
             # over the upsert time, where that form ran
             "l2_atomics": {"kind": "edge-counter atomics of pass 2 (one per transition push)",
                            "ops_per_step": sum(pushes.values()),
-                           "per_s": sum(pushes.values()) * args.steps / (kernel_ms["pass2_upsert"][0] / 1e3)
-                           if kernel_ms["pass2_upsert"][0] > 0 else None},
+                           "per_s": sum(pushes.values()) * args.steps / (kernel_ms["pass2_upsert"][0] / 1e3)}
+            if kernel_ms["pass2_upsert"][0] > 0 else None,
             "gpu_launches": launches,
             "clocks": clk,
             "e2e": e2e,
