@@ -422,6 +422,8 @@ __global__ void k_heavy_pieces(const unsigned long long* __restrict__ pre, uint3
 
 // Counts the windows of the pieces by sub-bin (PUT: moves them there), a block per piece, a warp
 // per 32 runs, a lane per window.  Windows of one sub-bin that meet in a warp share an atomic.
+// Bound by latency and issue: 5 Mbp of GC 0.15 at 25x, k = 21, 0.27 ms to count and 0.36 to move,
+// half of the issue slots, L2 12 and 23%, DRAM 4 and 12%.
 template <int NK, bool PUT>
 __global__ void __launch_bounds__(256) k_heavy_split(const uint64_t* __restrict__ data, const uint64_t* __restrict__ runs,
                                                      const HeavyPiece* __restrict__ pieces, const uint32_t* __restrict__ counts, uint32_t cap,
